@@ -344,7 +344,7 @@ void render_device(SceneHandle& h, const tpt_render_config& c, double* acc, doub
         ck(cudaEventCreate(&ev.e[0]), "event");
         ck(cudaEventCreate(&ev.e[1]), "event");
         cudaEventRecord(ev.e[0], h.stream);
-        cudaError_t e = launch_plain(h.plain, p, acc, acc_w, acc_sq, h.d_counters, h.d_flags, h.stream);
+        cudaError_t e = launch_plain(h.plain, p, acc, acc_w, acc_sq, h.d_counters, h.d_flags, h.sm_count, h.stream);
         cudaEventRecord(ev.e[1], h.stream);
         unsigned long long cnt[4] = {0, 0, 0, 0};
         int flags = 0;
@@ -779,6 +779,14 @@ int tpt_scene_create(const tpt_scene_desc* desc, void** out_scene) {
         W.lights64 = P.lights;
         W.inst64 = P.instances;
         W.spheres64 = P.spheres;
+        P.nodes32 = W.nodes;
+        P.meshes32 = W.meshes;
+        P.spheres32 = W.spheres;
+        P.top_root = W.top_root;
+        std::vector<int2> links;
+        link_plain(pi, fi, links, P.top_pad);
+        P.links = h->upload(links);
+        P.n_tris = (int)links.size();
         ck(cudaStreamSynchronize(h->stream), "scene upload");
         for (HostScene::Mesh& m : hs.meshes) m.bvh = HostBvh{};
         h->hs = std::move(hs);

@@ -31,7 +31,8 @@ struct alignas(16) TriF64 {
 };
 static_assert(sizeof(TriF64) == 80, "TriF64 is 80 B");
 
-struct MeshF64 { int32_t node_offset, n_nodes, tri_offset, n_tris; };
+// deep = 1: the tree may need more than the reference walk's 64 stack entries.
+struct MeshF64 { int32_t node_offset, n_nodes, tri_offset, n_tris, deep; };
 
 // Transform (src/transform.rs:11-21) + Instance (src/world.rs:39-46).
 struct InstanceF64 {

@@ -414,7 +414,7 @@ void flatten_plain_materials(const HostScene& hs, std::vector<MaterialF64>& mats
 void flatten_plain(const HostScene& hs, PlainImage& img) {
     for (const HostScene::Mesh& m : hs.meshes) {
         MeshF64 me{(int32_t)img.nodes.size(), (int32_t)(m.bvh.left_right.size() / 2), (int32_t)img.tris.size(),
-                   (int32_t)m.mat.size()};
+                   (int32_t)m.mat.size(), m.bvh.max_depth > 63 ? 1 : 0};
         const size_t nn = m.bvh.left_right.size() / 2;
         for (size_t i = 0; i < nn; ++i) {
             NodeF64 n{};
@@ -767,6 +767,35 @@ void flatten_fp32(const HostScene& hs, Fp32Image& img) {
         }
         img.env_row_cdf[h] = 1.0f;
     }
+}
+
+void link_plain(const PlainImage& plain, const Fp32Image& fp, std::vector<int2>& links, float& top_pad) {
+    const size_t n = plain.tris.size();
+    links.resize(n);
+    std::vector<int32_t> leaf(n, 0), place(n);
+    for (size_t m = 0; m < plain.meshes.size(); ++m) {  // both images hold the meshes one after another
+        const MeshF64& me = plain.meshes[m];
+        for (int32_t i = me.node_offset; i < me.node_offset + me.n_nodes; ++i) {
+            const NodeF64& nd = plain.nodes[(size_t)i];
+            if (nd.left != -1 || nd.right != -1) continue;
+            for (uint32_t k = nd.start; k < nd.start + nd.count; ++k) leaf[(size_t)me.tri_offset + k] = i;
+        }
+        const size_t t0 = (size_t)me.tri_offset, t1 = t0 + (size_t)me.n_tris;
+        for (size_t k = t0; k < t1; ++k) place[t0 + (size_t)plain.tris[k].orig] = (int32_t)k;
+        for (size_t k = t0; k < t1; ++k) {
+            int32_t orig;
+            std::memcpy(&orig, &fp.tris[k].e1.w, 4);
+            const int32_t at = place[t0 + (size_t)orig];
+            links[k] = make_int2(at, leaf[(size_t)at]);
+        }
+    }
+    float mag = 0.0f;
+    for (size_t i = (size_t)fp.top_node_begin; i < fp.nodes.size(); ++i) {
+        const BvhNode2& b = fp.nodes[i];
+        for (float v : {b.lx.x, b.lx.y, b.lx.z, b.lx.w, b.rx.x, b.rx.y, b.rx.z, b.rx.w, b.zz.x, b.zz.y, b.zz.z, b.zz.w})
+            mag = std::max(mag, std::fabs(v));
+    }
+    top_pad = mag * 0x1p-20f;
 }
 
 namespace {

@@ -134,6 +134,12 @@ struct Fp32Image {       // FP32 layout for the wavefront kernels
 };
 void flatten_fp32(const HostScene& hs, Fp32Image& img);
 
+// What the plain f64 kernel needs to walk the FP32 image's trees: per
+// triangle in their leaf order, its index in plain.tris and the node of
+// plain.nodes whose leaf range holds it; and the padding of the top-level
+// boxes, 2^-20 of the largest coordinate in them.
+void link_plain(const PlainImage& plain, const Fp32Image& fp, std::vector<int2>& links, float& top_pad);
+
 // Several scenes in one set of device arrays for batch renders: the FP32
 // images and the f64 light/instance/sphere tables of each scene appended,
 // every index rebased (BVH node and leaf references, material ids, mesh

@@ -1,12 +1,20 @@
-// Plain f64 form of the path integrator: one thread per pixel runs the
-// pixel's samples in order, continuing the reference's per-pixel RNG stream
-// (src/render.rs:141-158) through radiance() (src/integrator.rs:53-135) with
-// the reference's f64 arithmetic.  This translation unit is compiled with
+// Plain f64 form of the path integrator: each pixel's samples run in order on
+// one lane, continuing the reference's per-pixel RNG stream (src/render.rs:
+// 141-158) through radiance() (src/integrator.rs:53-135) with the
+// reference's f64 arithmetic.  This translation unit is compiled with
 // -fmad=false so a*b+c rounds twice, as in the reference; f64 division and
 // sqrt are IEEE-rounded on the GPU.  Transcendentals come from CUDA's libm,
 // whose last-bit results can differ from glibc's, so a pixel's stream can
 // diverge from the reference's after such a difference flips a branch.
+//
+// What World::hit returns is defined by the f64 tests of its triangles and
+// spheres; which boxes are looked at on the way is not.  So rays walk the
+// FP32 forms' trees with FP32 box tests that err on the side of visiting
+// (world_trace), and only the primitives that are left run the reference's
+// f64 arithmetic.
 #include "plain_f64.cuh"
+
+#include <algorithm>
 
 namespace tpt {
 namespace plain {
@@ -44,13 +52,6 @@ __device__ __forceinline__ size_t as_usize(double f) { return f > 0.0 ? (size_t)
 struct Ray { V o, d; double time; };
 struct Hit { double t; V p, n; int mat; };
 
-struct Ctx {
-    const PlainScene* S;
-    uint32_t shadow_rays;
-    uint32_t closest_rays;
-    int* flags;
-};
-
 // ---- src/geometry.rs ------------------------------------------------------
 __device__ bool box_hit(const double* bmin, const double* bmax, const Ray& r, V inv, double tmin, double tmax,
                         double* t_enter) {  // Aabb::hit_inv / hit_range_inv (:117-165)
@@ -67,69 +68,65 @@ __device__ bool box_hit(const double* bmin, const double* bmax, const Ray& r, V 
     return true;
 }
 
-__device__ bool tri_hit(const TriF64& tr, const Ray& r, double tmin, double tmax, Hit& h) {  // :236-273
-    const double t = r.time;
-    V v0 = ld(tr.v0) * (1.0 - t) + ld(tr.v0) * t;  // vertices_at (:212-218), static
-    V v1 = ld(tr.v1) * (1.0 - t) + ld(tr.v1) * t;
-    V v2 = ld(tr.v2) * (1.0 - t) + ld(tr.v2) * t;
-    V e1 = v1 - v0, e2 = v2 - v0;
-    V pvec = cross(r.d, e2);
+// Triangle::hit (:236-273): the distance, and the edges its normal comes from.
+__device__ __forceinline__ bool tri_test(const TriF64& tr, V o, V d, double time, double tmin, double tmax, double& th,
+                                         V& e1, V& e2) {
+    V v0 = ld(tr.v0) * (1.0 - time) + ld(tr.v0) * time;  // vertices_at (:212-218), static
+    V v1 = ld(tr.v1) * (1.0 - time) + ld(tr.v1) * time;
+    V v2 = ld(tr.v2) * (1.0 - time) + ld(tr.v2) * time;
+    e1 = v1 - v0;
+    e2 = v2 - v0;
+    V pvec = cross(d, e2);
     double det = dot(e1, pvec);
     if (fabs(det) < 1e-10) return false;
     double inv_det = 1.0 / det;
-    V tvec = r.o - v0;
+    V tvec = o - v0;
     double u = dot(tvec, pvec) * inv_det;
     if (u < 0.0 || u > 1.0) return false;
     V qvec = cross(tvec, e1);
-    double v = dot(r.d, qvec) * inv_det;
+    double v = dot(d, qvec) * inv_det;
     if (v < 0.0 || u + v > 1.0) return false;
-    double th = dot(e2, qvec) * inv_det;
-    if (th < tmin || th > tmax) return false;
-    h.t = th;
-    h.p = r.o + r.d * th;
-    h.n = norm(cross(e1, e2));
-    h.mat = tr.mat;
-    return true;
+    th = dot(e2, qvec) * inv_det;
+    return !(th < tmin || th > tmax);
 }
 
-__device__ bool sphere_hit(const SphereF64& s, const Ray& r, double tmin, double tmax, Hit& h) {  // :174-195
-    V c = ld(s.c);
+// Sphere::hit (:174-195): the distance.
+__device__ __forceinline__ bool sphere_test(V c, double rad, const Ray& r, double tmin, double tmax, double& t) {
     V oc = r.o - c;
     double a = dot(r.d, r.d);
     double b = dot(oc, r.d);
-    double cc = dot(oc, oc) - s.r * s.r;
+    double cc = dot(oc, oc) - rad * rad;
     double d = b * b - a * cc;
     if (d <= 0.0) return false;
     double sd = sqrt(d);
-    double t = (-b - sd) / a;
+    t = (-b - sd) / a;
     if (t < tmin || t > tmax) {
         t = (-b + sd) / a;
         if (t < tmin || t > tmax) return false;
     }
-    h.t = t;
-    h.p = r.o + r.d * t;
-    h.n = (h.p - c) / s.r;
-    h.mat = s.mat;
     return true;
 }
 
 // ---- src/bvh.rs:248-351 ---------------------------------------------------
-__device__ bool bvh_hit(Ctx& cx, const MeshF64& m, const Ray& r, double tmin, double tmax, Hit& best) {
-    if (m.n_nodes == 0) return false;
-    const NodeF64* nodes = cx.S->nodes + m.node_offset;
-    const TriF64* tris = cx.S->tris + m.tri_offset;
+// Bvh::hit as the reference walks it: its own tree, box by box in f64.  Kept
+// for what depends on the order of that walk (mesh_done below) and for trees
+// deeper than its stack.  Returns the triangle (index in S.tris), -1 = none.
+__device__ __noinline__ int bvh_hit(const NodeF64* nodes, const TriF64* tris, int* flags, V o, V d, double time,
+                                    double tmin, double tmax, double* t_hit) {
+    const Ray r{o, d, time};
     V inv = mk(1.0 / r.d.x, 1.0 / r.d.y, 1.0 / r.d.z);
     int stack[kStack];
     int sp = 0;
     stack[sp++] = 0;
-    bool found = false;
+    int best = -1;
     while (sp > 0) {
         const NodeF64& n = nodes[stack[--sp]];
         if (!box_hit(n.bmin, n.bmax, r, inv, tmin, tmax, nullptr)) continue;
         if (n.left == -1 && n.right == -1) {
             for (uint32_t k = n.start; k < n.start + n.count; ++k) {
-                Hit h;
-                if (tri_hit(tris[k], r, tmin, tmax, h)) { tmax = h.t; best = h; found = true; }
+                double th;
+                V e1, e2;
+                if (tri_test(tris[k], o, d, time, tmin, tmax, th, e1, e2)) { tmax = th; best = (int)k; }
             }
             continue;
         }
@@ -155,10 +152,11 @@ __device__ bool bvh_hit(Ctx& cx, const MeshF64& m, const Ray& r, double tmin, do
         }
         for (int k = 0; k < np; ++k) {
             if (sp < kStack) stack[sp++] = push[k];
-            else raise_flag(cx.flags, TPT_FLAG_STACK_OVERFLOW);
+            else raise_flag(flags, TPT_FLAG_STACK_OVERFLOW);
         }
     }
-    return found;
+    *t_hit = tmax;
+    return best;
 }
 
 __device__ V xf_point(const InstanceF64& x, V p) {          // apply_point (transform.rs:75-77)
@@ -171,32 +169,206 @@ __device__ V mat_vec(const double* a, V p) {
               a[6] * p.x + a[7] * p.y + a[8] * p.z);
 }
 
-// World::hit (src/world.rs:81-121)
-__device__ bool world_hit(Ctx& cx, const Ray& r, double tmin, double tmax, Hit& best) {
-    const PlainScene& S = *cx.S;
-    double closest = tmax;
-    bool found = false;
-    for (int i = 0; i < S.n_instances; ++i) {
-        const InstanceF64& inst = S.instances[i];
-        const MeshF64& mesh = S.meshes[inst.mesh_id];
-        Ray ro{mat_vec(inst.a_inv, r.o - ld(inst.t)), norm(mat_vec(inst.a_inv, r.d)), r.time};
-        Hit h;
-        if (bvh_hit(cx, mesh, ro, tmin, 1e30, h)) {
-            V p_world = xf_point(inst, h.p);
-            V n_world = norm(mat_vec(inst.nmat, h.n));
-            double t_world = dot(p_world - r.o, r.d);
-            if (t_world > tmin && t_world < closest) {
-                closest = t_world;
-                best = Hit{t_world, p_world, n_world, inst.mat_override >= 0 ? inst.mat_override : h.mat};
-                found = true;
+// ---- World::hit (src/world.rs:81-121) ---------------------------------------
+// The FP32 view of a ray for the box tests.  A slab distance (b - o) / d is
+// formed as b * idir - o * idir; against the f64 value its error is at most
+// a few ulps of the distance itself (the rounding of d, of its reciprocal
+// and of the sum) plus the rounding of o and of o * idir, below |o| * 2^-22
+// in world units.  The second part, and `pad` (world units), widen the box:
+// the near planes' offset is lowered and the far planes' raised by that
+// much; the first is covered by kSlack on the far distance.
+constexpr float kSlack = 1.0f + 1e-6f;
+struct Ray32 {
+    float3 idir, near_off, far_off;
+};
+__device__ __forceinline__ float safe_rcp(float d) {
+    return 1.0f / (fabsf(d) > 1e-20f ? d : copysignf(1e-20f, d));
+}
+__device__ __forceinline__ void set_axis(double o, double d, float pad, float& idir, float& lo, float& hi) {
+    const float of = (float)o;
+    idir = safe_rcp((float)d);
+    const float c = of * idir, m = (fabsf(of) * 2.4e-7f + pad) * fabsf(idir);
+    lo = -c - m;
+    hi = -c + m;
+}
+__device__ __forceinline__ Ray32 ray32(V o, V d, float pad) {
+    Ray32 r;
+    set_axis(o.x, d.x, pad, r.idir.x, r.near_off.x, r.far_off.x);
+    set_axis(o.y, d.y, pad, r.idir.y, r.near_off.y, r.far_off.y);
+    set_axis(o.z, d.z, pad, r.idir.z, r.near_off.z, r.far_off.z);
+    return r;
+}
+// Entry distance of the widened box; *hit = false only when no f64 test in
+// the box can succeed below tmax (a NaN keeps the box).
+__device__ __forceinline__ float box32(const Ray32& r, float x0, float x1, float y0, float y1, float z0, float z1,
+                                       float tmax, bool* hit) {
+    const bool sx = r.idir.x < 0.0f, sy = r.idir.y < 0.0f, sz = r.idir.z < 0.0f;
+    const float nx = __fmaf_rn(sx ? x1 : x0, r.idir.x, r.near_off.x), fx = __fmaf_rn(sx ? x0 : x1, r.idir.x, r.far_off.x);
+    const float ny = __fmaf_rn(sy ? y1 : y0, r.idir.y, r.near_off.y), fy = __fmaf_rn(sy ? y0 : y1, r.idir.y, r.far_off.y);
+    const float nz = __fmaf_rn(sz ? z1 : z0, r.idir.z, r.near_off.z), fz = __fmaf_rn(sz ? z0 : z1, r.idir.z, r.far_off.z);
+    const float n = fmaxf(fmaxf(nx, ny), fmaxf(nz, 0.0f));
+    const float f = fminf(fminf(fx, fy), fminf(fz, tmax)) * kSlack;
+    *hit = !(n > f);
+    return n;
+}
+
+// The closest hit so far in the world.
+struct Best {
+    double t;        // world distance (the ray's tmax until something is hit)
+    double th;       // instances: distance in the mesh's space
+    int inst, prim;  // instance and triangle, or -1 and the sphere; prim -1 = nothing
+};
+
+// True when the walk of instance `inst` ends in the closest hit: its mesh
+// hit taken to the world and compared as world.rs:92-108 does.
+__device__ __forceinline__ bool mesh_done(const PlainScene& S, const Ray& r, V o, V d, int inst, int tri, double th,
+                                          Best& best) {
+    if (tri < 0) return false;
+    const V p = xf_point(S.instances[inst], o + d * th);
+    const double t_world = dot(p - r.o, r.d);
+    // the reference tests instances in index order with a strict comparison
+    // and spheres after them: of equal distances the lowest instance stays
+    const bool closer = t_world < best.t || (t_world == best.t && best.inst > inst);
+    if (!(t_world > kEps && closer)) return false;
+    best = Best{t_world, th, inst, tri};
+    return true;
+}
+
+constexpr int kLeaveMesh = ~0;  // stack entry: back to world space (no leaf of a tree has the code 0 / 0)
+
+// World::hit over the top-level tree (spheres and instances) and the mesh
+// trees of the FP32 forms.  Bound by the latency of dependent node loads in
+// divergent lanes; against the reference's own tree and its linear sphere
+// and instance loops in f64 it visits the same primitives' tests with an
+// eighth of the f64 work (rates at k_paths below).
+//
+// Why the result is the reference's, whatever tree is walked:
+//  * A primitive's f64 test decides alone whether and where it is hit; the
+//    closest one wins.  Equal distances follow the reference's loop order:
+//    instances by index, spheres after them, the last sphere.
+//  * Bvh::hit reaches a triangle only through its leaf's box.  The f64 box
+//    test is monotonic, so a leaf that passes has ancestors that pass; the
+//    leaf's own test (box_hit on `leaf`) is therefore the whole condition,
+//    and it is run for each triangle that is hit.
+//  * What remains depends on the order of the reference's walk: two
+//    triangles of one mesh hit at the same distance, or a leaf box entered
+//    no earlier than the hit (the box might have been culled by an earlier
+//    hit).  Then the mesh is walked again by bvh_hit.
+__device__ __forceinline__ bool world_trace(const PlainScene& S, const Ray& r, double tmax, bool any, Best& best,
+                                            int* stack, int* flags) {
+    best = Best{tmax, 0.0, -1, -1};
+    Ray32 q = ray32(r.o, r.d, S.top_pad);
+    float far = __double2float_ru(tmax);
+    V o = r.o, d = r.d;  // the ray in the entered mesh's space
+    int inst = -1, tri = -1;
+    bool redo = false;
+    double th = 1e30;
+    int ref = S.top_root, sp = 0;
+    for (;;) {
+        while (ref >= 0) {
+            const float4* np = reinterpret_cast<const float4*>(S.nodes32 + ref);
+            const float4 lx = __ldg(np), rx = __ldg(np + 1), zz = __ldg(np + 2);
+            const int2 rf = __ldg(reinterpret_cast<const int2*>(np + 3));
+            bool hl, hr;
+            const float ln = box32(q, lx.x, lx.y, lx.z, lx.w, zz.x, zz.y, far, &hl);
+            const float rn = box32(q, rx.x, rx.y, rx.z, rx.w, zz.z, zz.w, far, &hr);
+            if (hl && hr) {
+                const bool right = rn < ln;
+                if (sp < kStack) stack[sp++] = right ? rf.x : rf.y;
+                else raise_flag(flags, TPT_FLAG_STACK_OVERFLOW);
+                ref = right ? rf.y : rf.x;
+            } else if (hl || hr) {
+                ref = hl ? rf.x : rf.y;
+            } else {
+                ref = sp > 0 ? stack[--sp] : TPT_REF_NONE;
             }
         }
+        if (ref == TPT_REF_NONE) return best.prim >= 0;
+        const uint32_t code = (uint32_t)(~ref), first = code >> 3, count = code & 7u;
+        if (ref == kLeaveMesh) {
+            if (redo) {
+                const MeshF64 m = S.meshes[S.instances[inst].mesh_id];
+                tri = bvh_hit(S.nodes + m.node_offset, S.tris + m.tri_offset, flags, o, d, r.time, kEps, 1e30, &th);
+                if (tri >= 0) tri += m.tri_offset;
+            }
+            if (mesh_done(S, r, o, d, inst, tri, th, best) && any) return true;
+            inst = -1;
+            q = ray32(r.o, r.d, S.top_pad);
+            far = __double2float_ru(best.t);
+        } else if (count == 7u) {  // enter an instance's mesh
+            const InstanceF64& I = S.instances[first];
+            const int root = S.meshes32[I.mesh_id].root_ref;
+            if (root != TPT_REF_NONE) {
+                const V du = mat_vec(I.a_inv, r.d);
+                o = mat_vec(I.a_inv, r.o - ld(I.t));
+                d = norm(du);
+                inst = (int)first;
+                tri = -1;
+                th = 1e30;
+                redo = S.meshes[I.mesh_id].deep != 0;
+                q = ray32(o, d, 0.0f);
+                // hits past the closest one so far are not needed; one world
+                // unit is |A^-1 d| units here
+                const double reach = best.t * len(du) * (1.0 + 1e-6);
+                far = reach < 1e30 ? __double2float_ru(reach) : 1e30f;
+                if (sp < kStack) stack[sp++] = kLeaveMesh;
+                else raise_flag(flags, TPT_FLAG_STACK_OVERFLOW);
+                if (!redo) {
+                    ref = root;
+                    continue;
+                }
+            }
+        } else if (inst >= 0) {
+#pragma unroll 1
+            for (uint32_t k = first; k < first + count; ++k) {
+                const int2 link = __ldg(S.links + k);
+                double t;
+                V e1, e2;
+                if (!tri_test(S.tris[link.x], o, d, r.time, kEps, th, t, e1, e2)) continue;
+                const NodeF64& leaf = S.nodes[link.y];
+                const V inv = mk(1.0 / d.x, 1.0 / d.y, 1.0 / d.z);
+                double enter;
+                if (!box_hit(leaf.bmin, leaf.bmax, Ray{o, d, r.time}, inv, kEps, 1e30, &enter)) continue;
+                redo = redo || !(enter < t) || (tri >= 0 && t == th);
+                th = t;
+                tri = link.x;
+                far = fminf(far, __double2float_ru(t));
+            }
+        } else {
+#pragma unroll 1
+            for (uint32_t k = first; k < first + count; ++k) {
+                const int id = __ldg(&S.spheres32[k].orig);
+                const SphereF64& s = S.spheres[id];
+                double t;
+                if (!sphere_test(ld(s.c), s.r, r, kEps, best.t, t)) continue;
+                // of equal distances the sphere tested last by the
+                // reference's loop, and spheres over instances
+                if (t == best.t && best.inst < 0 && best.prim > id) continue;
+                best = Best{t, 0.0, -1, id};
+                if (any) return true;
+                far = __double2float_ru(t);
+            }
+        }
+        ref = sp > 0 ? stack[--sp] : TPT_REF_NONE;
     }
-    for (int i = 0; i < S.n_spheres; ++i) {
-        Hit h;
-        if (sphere_hit(S.spheres[i], r, tmin, closest, h)) { closest = h.t; best = h; found = true; }
+}
+
+// The closest hit's point, normal and material (geometry.rs:174-195, :236-273,
+// world.rs:92-108).
+__device__ __forceinline__ Hit hit_of(const PlainScene& S, const Ray& r, const Best& b) {
+    if (b.inst < 0) {
+        const SphereF64& s = S.spheres[b.prim];
+        const V p = r.o + r.d * b.t;
+        return Hit{b.t, p, (p - ld(s.c)) / s.r, s.mat};
     }
-    return found;
+    const InstanceF64& I = S.instances[b.inst];
+    const V o = mat_vec(I.a_inv, r.o - ld(I.t)), d = norm(mat_vec(I.a_inv, r.d));
+    const TriF64& tr = S.tris[b.prim];
+    const V v0 = ld(tr.v0) * (1.0 - r.time) + ld(tr.v0) * r.time;
+    const V e1 = (ld(tr.v1) * (1.0 - r.time) + ld(tr.v1) * r.time) - v0;
+    const V e2 = (ld(tr.v2) * (1.0 - r.time) + ld(tr.v2) * r.time) - v0;
+    return Hit{b.t, xf_point(I, o + d * b.th), norm(mat_vec(I.nmat, norm(cross(e1, e2)))),
+               I.mat_override >= 0 ? I.mat_override : tr.mat};
 }
 
 // ---- src/material.rs -------------------------------------------------------
@@ -380,83 +552,86 @@ __device__ void mat_eval(const MaterialF64& m, V wo, V wi, V n, V& f, double& pd
 }
 
 // ---- src/env.rs ------------------------------------------------------------
-__device__ V env_lookup(const PlainScene& S, V dir) {                        // :92-121
+// EnvMap::lookup (:92-121) and, when asked for, the density of the same
+// direction (:156-182; both take the same u, v).
+__device__ __forceinline__ V env_at(const PlainScene& S, V dir, bool want_pdf, double& pdf) {
     V d = norm(dir);
     double theta = acos(clampd(d.y, -1.0, 1.0));
     double phi = atan2(d.z, d.x);
     if (phi < 0.0) phi += kTau;
     double u = phi / kTau, v = theta / kPi;
-    const size_t W = (size_t)S.env_w, H = (size_t)S.env_h;
+    const int W = S.env_w, H = S.env_h;
     double x = u * (double)W;
     double y = v * ((double)H - 1.0);
-    size_t x0 = as_usize(floor(x)) % W;
-    size_t x1 = (x0 + 1) % W;
-    size_t y0 = as_usize(floor(clampd(y, 0.0, (double)(H - 1))));
-    size_t y1 = y0 + 1 < H - 1 ? y0 + 1 : H - 1;
+    int x0 = (int)floor(x);           // 0 <= u <= 1 (a NaN converts to 0), so x0 % W needs one step
+    if (x0 >= W) x0 -= W;
+    const int x1 = x0 + 1 < W ? x0 + 1 : 0;
+    const int y0 = (int)floor(clampd(y, 0.0, (double)(H - 1)));
+    const int y1 = y0 + 1 < H - 1 ? y0 + 1 : H - 1;
     double fx = x - floor(x), fy = y - floor(y);
     const double* D = S.env_data;
-    V c00 = ld(D + 3 * (y0 * W + x0)), c10 = ld(D + 3 * (y0 * W + x1));
-    V c01 = ld(D + 3 * (y1 * W + x0)), c11 = ld(D + 3 * (y1 * W + x1));
+    const size_t r0 = (size_t)y0 * W, r1 = (size_t)y1 * W;
+    V c00 = ld(D + 3 * (r0 + x0)), c10 = ld(D + 3 * (r0 + x1));
+    V c01 = ld(D + 3 * (r1 + x0)), c11 = ld(D + 3 * (r1 + x1));
     V c0 = c00 * (1.0 - fx) + c10 * fx;
     V c1 = c01 * (1.0 - fx) + c11 * fx;
+    if (want_pdf) {
+        pdf = 1.0 / (4.0 * kPi);
+        if (S.env_total > 0.0) {
+            double fxw = floor(u * (double)W), fyh = floor(v * (double)H);
+            fxw = fxw < 0.0 ? 0.0 : (fxw > (double)(W - 1) ? (double)(W - 1) : fxw);
+            fyh = fyh < 0.0 ? 0.0 : (fyh > (double)(H - 1) ? (double)(H - 1) : fyh);
+            const int px = (int)fxw, py = (int)fyh;
+            double th0 = kPi * (double)py / (double)H, th1 = kPi * (double)(py + 1) / (double)H;
+            double st = fmax(sin(theta), 1e-6);
+            double rw = fmax(cos(th0) - cos(th1), 0.0);
+            double l = fmax(lum(ld(D + 3 * ((size_t)py * W + px))), 0.0);
+            double wgt = l * rw;
+            pdf = 0.0;
+            if (wgt > 0.0) {
+                double pdf_uv = (wgt / S.env_total) * (double)W * (double)H;
+                pdf = pdf_uv / (2.0 * kPi * kPi * st);
+            }
+        }
+    }
     return c0 * (1.0 - fy) + c1 * fy;
-}
-__device__ double env_pdf(const PlainScene& S, V dir) {                      // :156-182
-    if (S.env_total <= 0.0) return 1.0 / (4.0 * kPi);
-    V d = norm(dir);
-    double theta = acos(clampd(d.y, -1.0, 1.0));
-    double phi = atan2(d.z, d.x);
-    if (phi < 0.0) phi += kTau;
-    double u = phi / kTau, v = theta / kPi;
-    const size_t W = (size_t)S.env_w, H = (size_t)S.env_h;
-    double fxw = floor(u * (double)W), fyh = floor(v * (double)H);
-    fxw = fxw < 0.0 ? 0.0 : (fxw > (double)(W - 1) ? (double)(W - 1) : fxw);
-    fyh = fyh < 0.0 ? 0.0 : (fyh > (double)(H - 1) ? (double)(H - 1) : fyh);
-    size_t x = as_usize(fxw), y = as_usize(fyh);
-    double th0 = kPi * (double)y / (double)H, th1 = kPi * (double)(y + 1) / (double)H;
-    double st = fmax(sin(theta), 1e-6);
-    double rw = fmax(cos(th0) - cos(th1), 0.0);
-    double l = fmax(lum(ld(S.env_data + 3 * (y * W + x))), 0.0);
-    double wgt = l * rw;
-    if (wgt <= 0.0) return 0.0;
-    double pdf_uv = (wgt / S.env_total) * (double)W * (double)H;
-    return pdf_uv / (2.0 * kPi * kPi * st);
 }
 __device__ size_t cdf_search(const double* cdf, size_t n, double x) {      // env.rs:185-197, world.rs:324-336
     size_t lo = 0, hi = n == 0 ? 0 : n - 1;
+#pragma unroll 1
     while (lo + 1 < hi) {
         size_t mid = (lo + hi) / 2;
         if (cdf[mid] <= x) lo = mid; else hi = mid;
     }
     return lo;
 }
-__device__ void env_uniform(const PlainScene& S, uint64_t& rng, V& dir, V& rad, double& pdf) {  // :200-210
+// EnvMap::sample_dir (:124-152): the direction.  False when it was drawn
+// uniformly (:200-210), whose density is 1 / 4 pi.
+__device__ bool env_sample_dir(const PlainScene& S, uint64_t& rng, V& dir) {
+    const size_t W = (size_t)S.env_w, H = (size_t)S.env_h;
+    if (S.env_total > 0.0) {
+        double r0 = pcg_f64(rng) * S.env_total;
+        size_t y = cdf_search(S.env_row_cdf, H + 1, r0);
+        if (y > H - 1) y = H - 1;
+        double row_sum = fmax(S.env_row_cdf[y + 1] - S.env_row_cdf[y], 0.0);
+        if (row_sum > 0.0) {
+            double r1 = pcg_f64(rng) * row_sum;
+            size_t x = cdf_search(S.env_col_cdf + y * (W + 1), W + 1, r1);
+            if (x > W - 1) x = W - 1;
+            double u = ((double)x + pcg_f64(rng)) / (double)W;
+            double v = ((double)y + pcg_f64(rng)) / (double)H;
+            double theta = kPi * v, phi = kTau * u;
+            double st = sin(theta);
+            dir = mk(cos(phi) * st, cos(theta), sin(phi) * st);
+            return true;
+        }
+    }
     double u = pcg_f64(rng), v = pcg_f64(rng);
     double z = 1.0 - 2.0 * u;
     double r = sqrt(fmax(1.0 - z * z, 0.0));
     double phi = kTau * v;
     dir = mk(r * cos(phi), z, r * sin(phi));
-    rad = env_lookup(S, dir);
-    pdf = 1.0 / (4.0 * kPi);
-}
-__device__ void env_sample_dir(const PlainScene& S, uint64_t& rng, V& dir, V& rad, double& pdf) {  // :124-152
-    if (S.env_total <= 0.0) { env_uniform(S, rng, dir, rad, pdf); return; }
-    const size_t W = (size_t)S.env_w, H = (size_t)S.env_h;
-    double r0 = pcg_f64(rng) * S.env_total;
-    size_t y = cdf_search(S.env_row_cdf, H + 1, r0);
-    if (y > H - 1) y = H - 1;
-    double row_sum = fmax(S.env_row_cdf[y + 1] - S.env_row_cdf[y], 0.0);
-    if (row_sum <= 0.0) { env_uniform(S, rng, dir, rad, pdf); return; }
-    double r1 = pcg_f64(rng) * row_sum;
-    size_t x = cdf_search(S.env_col_cdf + y * (W + 1), W + 1, r1);
-    if (x > W - 1) x = W - 1;
-    double u = ((double)x + pcg_f64(rng)) / (double)W;
-    double v = ((double)y + pcg_f64(rng)) / (double)H;
-    double theta = kPi * v, phi = kTau * u;
-    double st = sin(theta);
-    dir = mk(cos(phi) * st, cos(theta), sin(phi) * st);
-    rad = env_lookup(S, dir);
-    pdf = env_pdf(S, dir);
+    return false;
 }
 
 // ---- src/world.rs:171-272 --------------------------------------------------
@@ -514,91 +689,6 @@ __device__ __forceinline__ double mis(double a, double b) {
     return (a2 + b2 > 0.0) ? a2 / (a2 + b2) : 0.0;
 }
 
-__device__ V radiance(Ctx& cx, Ray ray, uint64_t& rng, int max_bounces, int rr_start) {  // :53-135
-    const PlainScene& S = *cx.S;
-    const bool has_env = S.env_kind == TPT_ENV_MAP;
-    V acc = mk(0, 0, 0), beta = mk(1, 1, 1);
-    double last_pdf = 0.0;
-    bool last_nd = false;
-    for (int bounce = 0; bounce < max_bounces; ++bounce) {
-        Hit hit;
-        cx.closest_rays++;
-        if (!world_hit(cx, ray, kEps, kTMax, hit)) {
-            V bg;
-            if (has_env) {
-                bg = env_lookup(S, ray.d);
-            } else {
-                double t = 0.5 * (ray.d.y + 1.0);  // sky (:25-28)
-                bg = (1.0 - t) * mk(0.9, 0.95, 1.0) + t * mk(0.6, 0.75, 1.0);
-            }
-            V contrib = had(beta, bg);
-            if (has_env && last_nd) contrib = contrib * mis(last_pdf, env_pdf(S, ray.d));
-            acc = acc + clamp_lum(contrib, 50.0);
-            break;
-        }
-        if (bounce >= rr_start) {
-            double p = fmax(fmin(fmax(fmax(beta.x, beta.y), beta.z), 0.95), 0.05);
-            if (pcg_f64(rng) > p) break;
-            beta = beta / p;
-        }
-        const MaterialF64& mat = S.mats[hit.mat];
-        if (mat.kind == TPT_MAT_DIFFUSE_LIGHT) {
-            acc = acc + clamp_lum(had(beta, ld(mat.c)), 50.0);
-            break;
-        }
-        V n = dot(hit.n, ray.d) < 0.0 ? hit.n : -hit.n;
-        if (mat.kind != TPT_MAT_METAL && mat.kind != TPT_MAT_DIELECTRIC) {
-            if (has_env) {  // nee_environment (:148-172)
-                V wi, li;
-                double pe;
-                env_sample_dir(S, rng, wi, li, pe);
-                double c = fmax(dot(n, wi), 0.0);
-                if (c > 0.0 && pe > 0.0) {
-                    Ray sh{hit.p + kEps * wi, wi, ray.time};
-                    Hit tmp;
-                    cx.shadow_rays++;
-                    if (!world_hit(cx, sh, kEps, kTMax, tmp)) {
-                        V f;
-                        double pb;
-                        mat_eval(mat, norm(-ray.d), wi, n, f, pb);
-                        acc = acc + had(had(beta, f), li) * (c * mis(pe, pb) / pe);
-                    }
-                }
-            }
-            V lp, ln, le;
-            double lpdf;
-            if (sample_light(S, rng, ray.time, hit.p, lp, ln, le, lpdf)) {  // nee_area_light (:178-213)
-                V tl = lp - hit.p;
-                double d2 = dot(tl, tl);
-                double dist = sqrt(d2);
-                if (dist > 1e-6) {
-                    V wi = tl / dist;
-                    double c = fmax(dot(n, wi), 0.0);
-                    if (c > 0.0) {
-                        Ray sh{hit.p + kEps * wi, wi, ray.time};
-                        double tm = fmax(dist - kEps, kEps);
-                        Hit tmp;
-                        cx.shadow_rays++;
-                        if (!world_hit(cx, sh, kEps, tm, tmp)) {
-                            V f;
-                            double pb;
-                            mat_eval(mat, norm(-ray.d), wi, n, f, pb);
-                            if (lpdf > 0.0) acc = acc + had(had(beta, f), le) * (c * mis(lpdf, pb) / lpdf);
-                        }
-                    }
-                }
-            }
-        }
-        Bsdf s;
-        if (!mat_sample(mat, ray, hit, rng, s)) break;
-        last_pdf = s.pdf;
-        last_nd = !s.delta;
-        beta = had(beta, s.w);
-        ray = s.ray;
-    }
-    return acc;
-}
-
 __device__ Ray camera_ray(const CameraF64& c, double sx, double sy, uint64_t& rng) {  // ray.rs:91-108
     V u = ld(c.u), v = ld(c.v), w = ld(c.w), o = ld(c.o);
     V dir_base = norm(((-w) + (sx * c.half_w) * u) + (sy * c.half_h) * v);
@@ -607,6 +697,7 @@ __device__ Ray camera_ray(const CameraF64& c, double sx, double sy, uint64_t& rn
         double dx = 0.0, dy = 0.0;
         // sample_unit_disk (:112-120); the acceptance rate is pi/4, so the
         // 256-try bound is never reached in practice ((1-pi/4)^256 ~ 1e-171).
+#pragma unroll 1
         for (int k = 0; k < 256; ++k) {
             dx = 2.0 * pcg_f64(rng) - 1.0;
             dy = 2.0 * pcg_f64(rng) - 1.0;
@@ -621,36 +712,167 @@ __device__ Ray camera_ray(const CameraF64& c, double sx, double sy, uint64_t& rn
     return Ray{origin, dir, time};
 }
 
-// One thread per pixel; blocks tile the image 16x8.
-__global__ void __launch_bounds__(128) k_render(PlainScene S, PlainParams P, double* __restrict__ acc,
-                                                double* __restrict__ acc_w, double* __restrict__ acc_sq,
-                                                unsigned long long* __restrict__ counters, int* flags) {
-    const int x = blockIdx.x * 16 + (threadIdx.x & 15);
-    const int fy = blockIdx.y * 8 + (threadIdx.x >> 4);  // film row
-    const int y = P.row_begin + fy * P.row_step;          // image row
-    Ctx cx{&S, 0u, 0u, flags};
-    uint32_t nsamp = 0;
-    if (x < P.width && fy < P.n_rows) {
-        uint64_t rng = pixel_seed((uint32_t)x, (uint32_t)y, P.seed);
-        const double inv_w = 1.0 / (double)P.width, inv_h = 1.0 / (double)P.height;
-        V c = mk(0, 0, 0), c2 = mk(0, 0, 0);
-        int max_spp = P.spp > 1 ? P.spp : 1;
-        int min_spp = P.adaptive_min_spp > 1 ? P.adaptive_min_spp : 1;
-        if (min_spp > max_spp) min_spp = max_spp;
-        double mean = 0.0, m2 = 0.0;
-        int n = 0;
-        for (int s = 0; s < P.spp; ++s) {
-            double jx = pcg_f64(rng);
-            double jy = pcg_f64(rng);
-            double sx = ((double)x + jx) * inv_w * 2.0 - 1.0;
-            double sy = 1.0 - ((double)y + jy) * inv_h * 2.0;
-            Ray r = camera_ray(S.cam, sx, sy, rng);
-            V smp = radiance(cx, r, rng, P.max_bounces, P.rr_start);
-            c = c + smp;
-            c2 = c2 + had(smp, smp);
+// What a path waits for before its next bounce.
+constexpr int kJobEnv = 1, kJobArea = 2, kJobClosest = 4;
+
+// Every lane runs one pixel's samples, bounce by bounce; a lane whose pixel is
+// finished takes the next one.  A round of the block is: shade what the last
+// closest-hit rays met (radiance(), src/integrator.rs:53-135, one bounce),
+// finish samples and start new ones, then trace -- first the NEE shadow rays
+// of the bounce, then its next ray -- until no lane of the warp waits for a
+// ray.  The contributions of the shadow rays are formed before the trace and
+// added after it, in the reference's order, so a round has one copy of the
+// walk and one of the shading code.
+//
+// Bound by instruction fetch, then by the latency of each pixel's chain of
+// bounces (its samples share one stream): the f64 code is some 190 KB, a warp
+// alone waits for nearly every line of it ("no instruction" 18 of 23 cycles
+// per issue), and no SM has work for more than a few warps at 65,536 pixels.
+// Barriers between the stages keep the block's warps on the same lines.
+// Measured on one B200, sphere scene 256x256 x 64 spp / mesh scene (327,680
+// triangles, 200 spheres, env map) 480x270 x 32 spp, ms: one thread per pixel
+// over the reference's tree and linear loops 43.7 / 115; this kernel without
+// barriers 21.0 / 17.3; with them 8.5 / 16.2 in blocks of 256, one per SM,
+// and 11.8 / 13.8 in blocks of 128, two per SM.  At 128 registers (512 lanes
+// per SM) 10.6 / 18.4.  `lanes` lanes of each warp take pixels.
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_constant__ PlainScene S,
+                                                     const __grid_constant__ PlainParams P, double* __restrict__ acc,
+                                                     double* __restrict__ acc_w, double* __restrict__ acc_sq,
+                                                     unsigned long long* __restrict__ counters, int* flags,
+                                                     unsigned lanes) {
+    const unsigned lane = threadIdx.x & 31u;
+    const bool has_env = S.env_kind == TPT_ENV_MAP;
+    const double inv_w = 1.0 / (double)P.width, inv_h = 1.0 / (double)P.height;
+    const int max_spp = P.spp > 1 ? P.spp : 1;
+    const int min_spp = min(P.adaptive_min_spp > 1 ? P.adaptive_min_spp : 1, max_spp);
+    // pixels are handed out by 8 x 4 tiles, a warp's worth each
+    const unsigned tiles_x = (unsigned)(P.width + 7) / 8u, n_ids = tiles_x * ((unsigned)(P.n_rows + 3) / 4u) * 32u;
+    int stack[kStack];
+    unsigned long long n_samples = 0, n_closest = 0, n_shadow = 0;
+    // the pixel
+    int x = -1, row = 0, n = 0;
+    uint64_t rng = 0;
+    V c = mk(0, 0, 0), c2 = mk(0, 0, 0);
+    double mean = 0.0, m2 = 0.0;
+    bool exhausted = lane >= lanes;
+    // the path
+    Ray ray{};
+    V L = mk(0, 0, 0), beta = mk(1, 1, 1);
+    double last_pdf = 0.0;
+    int bounce = 0, jobs = 0;
+    bool last_nd = false, ended = false, found = false;
+    Best best{};
+    // shadow rays: direction, contribution when nothing is in the way
+    V sh_p = mk(0, 0, 0), env_wi = mk(0, 0, 0), env_c = mk(0, 0, 0), area_wi = mk(0, 0, 0), area_c = mk(0, 0, 0);
+    double area_t = 0.0;
+    for (;;) {
+        __syncthreads();
+        const bool shade = x >= 0 && !ended;
+        V dir = ray.d, nrm = mk(0, 0, 0);
+        bool surface = false, want_pdf = last_nd;
+        Hit hit{};
+        int kind = -1;
+        if (shade && found) {
+            hit = hit_of(S, ray, best);
+            if (bounce >= P.rr_start) {
+                double p = fmax(fmin(fmax(fmax(beta.x, beta.y), beta.z), 0.95), 0.05);
+                if (pcg_f64(rng) > p) ended = true;
+                else beta = beta / p;
+            }
+            if (!ended) {
+                kind = S.mats[hit.mat].kind;
+                if (kind == TPT_MAT_DIFFUSE_LIGHT) {
+                    L = L + clamp_lum(had(beta, ld(S.mats[hit.mat].c)), 50.0);
+                    ended = true;
+                } else {
+                    surface = true;
+                    nrm = dot(hit.n, ray.d) < 0.0 ? hit.n : -hit.n;
+                    sh_p = hit.p;
+                }
+            }
+        }
+        const bool nee = surface && kind != TPT_MAT_METAL && kind != TPT_MAT_DIELECTRIC;
+        __syncthreads();
+        if (nee && has_env) want_pdf = env_sample_dir(S, rng, dir);
+        V bg = mk(0, 0, 0);
+        double pe = 1.0 / (4.0 * kPi);
+        __syncthreads();
+        if (has_env && shade && (!found || nee)) bg = env_at(S, dir, want_pdf, pe);
+        __syncthreads();
+        if (shade && !found) {  // miss
+            if (!has_env) {
+                double t = 0.5 * (ray.d.y + 1.0);  // sky (:25-28)
+                bg = (1.0 - t) * mk(0.9, 0.95, 1.0) + t * mk(0.6, 0.75, 1.0);
+            }
+            V contrib = had(beta, bg);
+            if (has_env && last_nd) contrib = contrib * mis(last_pdf, pe);
+            L = L + clamp_lum(contrib, 50.0);
+            ended = true;
+        }
+        bool area = false;
+        double ca = 0.0, lpdf = 1.0;
+        V le = mk(0, 0, 0);
+        if (nee) {
+            V lp, ln;
+            if (sample_light(S, rng, ray.time, hit.p, lp, ln, le, lpdf)) {  // nee_area_light (:178-213)
+                V tl = lp - hit.p;
+                double d2 = dot(tl, tl);
+                double dist = sqrt(d2);
+                if (dist > 1e-6) {
+                    area_wi = tl / dist;
+                    ca = fmax(dot(nrm, area_wi), 0.0);
+                    area = ca > 0.0;
+                    area_t = fmax(dist - kEps, kEps);
+                }
+            }
+        }
+        __syncthreads();
+        if (nee) {
+            // nee_environment (:148-172), then nee_area_light: one BSDF
+            // evaluation each.  A contribution of exactly zero adds nothing,
+            // whatever its shadow ray meets.
+            const MaterialF64& mat = S.mats[hit.mat];
+            const V wo = norm(-ray.d);
+            const double ce = has_env ? fmax(dot(nrm, dir), 0.0) : 0.0;
+#pragma unroll 1
+            for (int k = 0; k < 2; ++k) {
+                if (!(k == 0 ? ce > 0.0 && pe > 0.0 : area)) continue;
+                const V wi = k == 0 ? dir : area_wi, li = k == 0 ? bg : le;
+                const double cs = k == 0 ? ce : ca, pl = k == 0 ? pe : lpdf;
+                ++n_shadow;
+                V f;
+                double pb;
+                mat_eval(mat, wo, wi, nrm, f, pb);
+                const V contrib = had(had(beta, f), li) * (cs * mis(pl, pb) / pl);
+                if (contrib.x == 0.0 && contrib.y == 0.0 && contrib.z == 0.0) continue;
+                if (k == 0) { env_wi = wi; env_c = contrib; jobs |= kJobEnv; }
+                else { area_c = contrib; jobs |= kJobArea; }
+            }
+        }
+        __syncthreads();
+        if (surface) {
+            Bsdf s;
+            if (!mat_sample(S.mats[hit.mat], ray, hit, rng, s)) {
+                ended = true;
+            } else {
+                last_pdf = s.pdf;
+                last_nd = !s.delta;
+                beta = had(beta, s.w);
+                ray = s.ray;
+                if (++bounce >= P.max_bounces) ended = true;
+                else jobs |= kJobClosest;
+            }
+        }
+        __syncthreads();
+        bool start = false;
+        if (x >= 0 && ended && jobs == 0) {  // the sample is complete (src/render.rs:158-191)
+            c = c + L;
+            c2 = c2 + had(L, L);
             n += 1;
+            bool stop = n >= P.spp;
             if (P.adaptive) {  // render.rs:160-176
-                double l = lum(smp);
+                double l = lum(L);
                 double delta = l - mean;
                 mean += delta / (double)n;
                 double delta2 = l - mean;
@@ -658,36 +880,115 @@ __global__ void __launch_bounds__(128) k_render(PlainScene S, PlainParams P, dou
                 if (n >= min_spp) {
                     double var = n > 1 ? m2 / (double)(n - 1) : __longlong_as_double(0x7ff0000000000000ll);
                     double den = fmax(fabs(mean), 1e-4);
-                    if (sqrt(var) / den < P.adaptive_threshold) break;
+                    if (sqrt(var) / den < P.adaptive_threshold) stop = true;
+                }
+            }
+            if (stop) {
+                const size_t gi = (size_t)row * (size_t)P.width + (size_t)x;
+                acc[3 * gi] = c.x; acc[3 * gi + 1] = c.y; acc[3 * gi + 2] = c.z;
+                acc_w[gi] = (double)n;
+                if (acc_sq) { acc_sq[3 * gi] = c2.x; acc_sq[3 * gi + 1] = c2.y; acc_sq[3 * gi + 2] = c2.z; }
+                n_samples += (unsigned long long)n;
+                x = -1;
+            }
+            start = !stop;
+        }
+        const bool want = x < 0 && !exhausted;
+        const unsigned wm = __ballot_sync(0xffffffffu, want);
+        if (wm) {
+            unsigned base = 0;
+            const int leader = __ffs(wm) - 1;
+            if ((int)lane == leader) base = (unsigned)atomicAdd(&counters[3], (unsigned long long)__popc(wm));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (want) {
+                const unsigned id = base + __popc(wm & ((1u << lane) - 1u));
+                const unsigned tile = id >> 5, ty = tile / tiles_x;
+                const int px = (int)((tile - ty * tiles_x) * 8u + (id & 7u)), py = (int)(ty * 4u + ((id >> 3) & 3u));
+                exhausted = id >= n_ids;
+                if (!exhausted && px < P.width && py < P.n_rows) {
+                    x = px;
+                    row = py;
+                    n = 0;
+                    c = c2 = mk(0, 0, 0);
+                    mean = m2 = 0.0;
+                    rng = pixel_seed((uint32_t)x, (uint32_t)(P.row_begin + row * P.row_step), P.seed);
+                    start = true;
                 }
             }
         }
-        const size_t gi = (size_t)fy * (size_t)P.width + (size_t)x;
-        acc[3 * gi] = c.x; acc[3 * gi + 1] = c.y; acc[3 * gi + 2] = c.z;
-        acc_w[gi] = (double)n;
-        if (acc_sq) { acc_sq[3 * gi] = c2.x; acc_sq[3 * gi + 1] = c2.y; acc_sq[3 * gi + 2] = c2.z; }
-        nsamp = (uint32_t)n;
+        if (start) {  // src/render.rs:151-158
+            const int y = P.row_begin + row * P.row_step;
+            double jx = pcg_f64(rng);
+            double jy = pcg_f64(rng);
+            double sx = ((double)x + jx) * inv_w * 2.0 - 1.0;
+            double sy = 1.0 - ((double)y + jy) * inv_h * 2.0;
+            ray = camera_ray(S.cam, sx, sy, rng);
+            L = mk(0, 0, 0);
+            beta = mk(1, 1, 1);
+            last_pdf = 0.0;
+            last_nd = false;
+            bounce = 0;
+            ended = P.max_bounces <= 0;
+            if (!ended) jobs = kJobClosest;
+        }
+        if (!__syncthreads_or(x >= 0 || !exhausted)) break;
+        while (__any_sync(0xffffffffu, jobs != 0)) {
+            if (jobs != 0) {
+                const int job = jobs & -jobs;
+                Ray r = ray;
+                double tmax = kTMax;
+                if (job != kJobClosest) {
+                    const V wi = job == kJobEnv ? env_wi : area_wi;
+                    r = Ray{sh_p + kEps * wi, wi, ray.time};
+                    if (job == kJobArea) tmax = area_t;
+                }
+                Best b;
+                const bool h = world_trace(S, r, tmax, job != kJobClosest, b, stack, flags);
+                if (job == kJobClosest) {
+                    best = b;
+                    found = h;
+                    ++n_closest;
+                } else if (!h) {
+                    L = L + (job == kJobEnv ? env_c : area_c);
+                }
+                jobs ^= job;
+            }
+        }
     }
-    // Warp-reduce the ray/path counters, one atomic per warp.
-    unsigned long long cr = cx.closest_rays, sr = cx.shadow_rays, np = nsamp;
     for (int off = 16; off > 0; off >>= 1) {
-        cr += __shfl_down_sync(0xffffffffu, cr, off);
-        sr += __shfl_down_sync(0xffffffffu, sr, off);
-        np += __shfl_down_sync(0xffffffffu, np, off);
+        n_samples += __shfl_down_sync(0xffffffffu, n_samples, off);
+        n_closest += __shfl_down_sync(0xffffffffu, n_closest, off);
+        n_shadow += __shfl_down_sync(0xffffffffu, n_shadow, off);
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&counters[0], np);
-        atomicAdd(&counters[1], cr);
-        atomicAdd(&counters[2], sr);
+    if (lane == 0) {
+        atomicAdd(&counters[0], n_samples);
+        atomicAdd(&counters[1], n_closest);
+        atomicAdd(&counters[2], n_shadow);
     }
 }
 
 }  // namespace plain
 
 cudaError_t launch_plain(const PlainScene& S, const PlainParams& P, double* acc, double* acc_w, double* acc_sq,
-                         unsigned long long* counters, int* flags, cudaStream_t stream) {
-    dim3 grid((unsigned)((P.width + 15) / 16), (unsigned)((P.n_rows + 7) / 8));
-    plain::k_render<<<grid, 128, 0, stream>>>(S, P, acc, acc_w, acc_sq, counters, flags);
+                         unsigned long long* counters, int* flags, int sm_count, cudaStream_t stream) {
+    // Short walks: one block of 256 per SM, whose warps share the most fetched
+    // lines.  Past about a thousand triangles the warps' walks differ so much
+    // in length that waiting for the slowest of 8 costs more than fetching for
+    // 4, and two blocks of 128 are better (480x270 x 32 spp with 200 spheres
+    // and 1,280 / 20,480 / 327,680 triangles, ms: 9.6 / 11.9 / 15.9 in blocks
+    // of 256, 9.2 / 10.7 / 14.0 in blocks of 128; sphere scene 8.5 / 11.7).
+    const int block = S.n_tris < 1024 ? 256 : 128;
+    // 256 lanes per SM hold a pixel each.  A film of fewer pixels spreads them
+    // over the warps: a warp of a few lanes diverges less, and it is each
+    // pixel's own chain of bounces that the render waits for (48x30 x 64 spp:
+    // 7.5 ms in full warps, 4.6 spread).
+    const long long pixels = (long long)((P.width + 7) / 8) * ((P.n_rows + 3) / 4) * 32;  // in whole 8 x 4 tiles
+    const long long warps = (long long)sm_count * 8;
+    const unsigned lanes = (unsigned)std::min<long long>(32, std::max<long long>(1, (pixels + warps - 1) / warps));
+    const long long per_block = (long long)lanes * (block / 32);
+    const unsigned grid = (unsigned)std::min<long long>((pixels + per_block - 1) / per_block, warps * 32 / block);
+    if (block == 256) plain::k_paths<256><<<grid, 256, 0, stream>>>(S, P, acc, acc_w, acc_sq, counters, flags, lanes);
+    else plain::k_paths<128><<<grid, 128, 0, stream>>>(S, P, acc, acc_w, acc_sq, counters, flags, lanes);
     return cudaGetLastError();
 }
 

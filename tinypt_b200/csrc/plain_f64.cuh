@@ -1,7 +1,8 @@
-// Device view of the f64 scene image and the plain kernel's launch: one
-// thread per pixel runs the reference's render worker (src/render.rs:129-205)
-// and radiance() (src/integrator.rs:53-135) in f64 over the reference's own
-// node, triangle, sphere and instance layouts.
+// Device view of the f64 scene image and the plain kernel's launch: one lane
+// per pixel runs the reference's render worker (src/render.rs:129-205) and
+// radiance() (src/integrator.rs:53-135) in f64 over the reference's own
+// node, triangle, sphere and instance layouts, found through the FP32 forms'
+// trees.
 #pragma once
 
 #include "device_common.cuh"
@@ -28,6 +29,15 @@ struct PlainScene {
     const double* env_col_cdf;
     double env_total;
     CameraF64 cam;
+    // The FP32 forms' trees (WfScene's arrays) and, per triangle in their
+    // leaf order, its place in `tris` (x) and its leaf in `nodes` (y).
+    const BvhNode2* nodes32;
+    const MeshF32* meshes32;
+    const SphereF32* spheres32;
+    const int2* links;
+    int n_tris;
+    int top_root;
+    float top_pad;             // widens the top-level boxes: far above the f64 error of a sphere test
 };
 
 struct PlainParams {
@@ -38,8 +48,9 @@ struct PlainParams {
     int row_begin, row_step, n_rows;  // film row k is image row row_begin + k * row_step
 };
 
-// counters[0] = samples, [1] = closest-hit rays, [2] = shadow rays.
+// counters[0] = samples, [1] = closest-hit rays, [2] = shadow rays, [3] =
+// pixels handed out; all zero on entry.
 cudaError_t launch_plain(const PlainScene& S, const PlainParams& P, double* acc, double* acc_w, double* acc_sq,
-                         unsigned long long* counters, int* flags, cudaStream_t stream);
+                         unsigned long long* counters, int* flags, int sm_count, cudaStream_t stream);
 
 }  // namespace tpt
