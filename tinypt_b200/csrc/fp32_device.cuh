@@ -488,30 +488,45 @@ __device__ __forceinline__ void dir_uv(float3 d, float& u, float& v, float& thet
     u = phi / kTau;
     v = theta / kPi;
 }
-static __device__ float3 env_lookup(const WfScene& S, float3 d) {
+// The radiance of direction d (bilinear) and, when pdf is given, the density
+// env_sample_dir draws it with (nearest texel): both take the same u, v.
+__device__ __forceinline__ float3 env_at(const WfScene& S, float3 d, float* pdf) {
     float u, v, theta;
     dir_uv(d, u, v, theta);
     const int W = S.env_w, H = S.env_h;
     const float x = u * (float)W, y = v * ((float)H - 1.0f);
     const float fxf = floorf(x);
-    int x0 = (int)fxf % W;
-    if (x0 < 0) x0 = 0;
-    const int x1 = (x0 + 1) % W;
-    int y0 = (int)floorf(fminf(fmaxf(y, 0.0f), (float)(H - 1)));
+    int x0 = (int)fxf;                 // 0 <= u <= 1 (a NaN converts to 0): x0 modulo W takes one step
+    if (x0 >= W) x0 -= W;
+    const int x1 = x0 + 1 < W ? x0 + 1 : 0;
+    const int y0 = (int)floorf(fminf(fmaxf(y, 0.0f), (float)(H - 1)));
     const int y1 = min(y0 + 1, H - 1);
     const float fx = x - fxf, fy = y - floorf(y);
+    if (pdf) {
+        *pdf = 1.0f / (4.0f * kPi);
+        if (S.env_has_cdf) {
+            const int px = (int)fminf(fmaxf(fxf, 0.0f), (float)(W - 1));
+            const int py = (int)fminf(fmaxf(floorf(v * (float)H), 0.0f), (float)(H - 1));
+            const float pdf_uv = __ldg(&S.env_tex[py * W + px].w);
+            *pdf = pdf_uv <= 0.0f ? 0.0f : pdf_uv / (2.0f * kPi * kPi * fmaxf(sinf(theta), 1e-6f));
+        }
+    }
     const float3 c00 = f3(__ldg(S.env_tex + y0 * W + x0)), c10 = f3(__ldg(S.env_tex + y0 * W + x1));
     const float3 c01 = f3(__ldg(S.env_tex + y1 * W + x0)), c11 = f3(__ldg(S.env_tex + y1 * W + x1));
     const float3 c0 = c00 * (1.0f - fx) + c10 * fx;
     const float3 c1 = c01 * (1.0f - fx) + c11 * fx;
     return c0 * (1.0f - fy) + c1 * fy;
 }
-// What a ray that leaves the scene sees (src/integrator.rs:71-83): the env
-// map, or without one the sky gradient (:25-28).
-__device__ __forceinline__ float3 background(const WfScene& S, float3 rd) {
-    if (S.env_kind == TPT_ENV_MAP) return env_lookup(S, rd);
+static __device__ float3 env_lookup(const WfScene& S, float3 d) { return env_at(S, d, nullptr); }
+// The sky gradient a scene without an env map shows (src/integrator.rs:25-28).
+__device__ __forceinline__ float3 sky(float3 rd) {
     const float t = 0.5f * (rd.y + 1.0f);
     return f3(0.9f, 0.95f, 1.0f) * (1.0f - t) + f3(0.6f, 0.75f, 1.0f) * t;
+}
+// What a ray that leaves the scene sees (src/integrator.rs:71-83): the env
+// map, or without one the sky.
+__device__ __forceinline__ float3 background(const WfScene& S, float3 rd) {
+    return S.env_kind == TPT_ENV_MAP ? env_lookup(S, rd) : sky(rd);
 }
 static __device__ float env_pdf(const WfScene& S, float3 d) {
     if (!S.env_has_cdf) return 1.0f / (4.0f * kPi);
@@ -533,32 +548,37 @@ __device__ __forceinline__ int cdf_search(const float* __restrict__ cdf, int n, 
     }
     return lo;
 }
-static __device__ void env_uniform(const WfScene& S, uint64_t& rng, float3& dir, float3& rad, float& pdf) {
+// The direction of an env-map sample (src/env.rs:124-152); false when it was
+// drawn uniformly (:200-210), with density 1 / 4 pi.
+__device__ __forceinline__ bool env_sample_to(const WfScene& S, uint64_t& rng, float3& dir) {
+    if (S.env_has_cdf) {
+        const int W = S.env_w, H = S.env_h;
+        const float r0 = pcg_f32(rng);
+        const int y = min(cdf_search(S.env_row, H + 1, r0), H - 1);
+        if (!(__ldg(S.env_row + y + 1) - __ldg(S.env_row + y) <= 0.0f)) {
+            const float r1 = pcg_f32(rng);
+            const int x = min(cdf_search(S.env_col + (size_t)y * (W + 1), W + 1, r1), W - 1);
+            const float u = ((float)x + pcg_f32(rng)) / (float)W;
+            const float v = ((float)y + pcg_f32(rng)) / (float)H;
+            float st, ct, sp, cp;
+            sincosf(kPi * v, &st, &ct);
+            sincosf(kTau * u, &sp, &cp);
+            dir = f3(cp * st, ct, sp * st);
+            return true;
+        }
+    }
     const float u = pcg_f32(rng), v = pcg_f32(rng);
     const float z = 1.0f - 2.0f * u;
     const float r = sqrtf(fmaxf(1.0f - z * z, 0.0f));
     float s, c;
     __sincosf(kTau * v, &s, &c);
     dir = f3(r * c, z, r * s);
-    rad = env_lookup(S, dir);
-    pdf = 1.0f / (4.0f * kPi);
+    return false;
 }
 static __device__ void env_sample_dir(const WfScene& S, uint64_t& rng, float3& dir, float3& rad, float& pdf) {
-    if (!S.env_has_cdf) { env_uniform(S, rng, dir, rad, pdf); return; }
-    const int W = S.env_w, H = S.env_h;
-    const float r0 = pcg_f32(rng);
-    const int y = min(cdf_search(S.env_row, H + 1, r0), H - 1);
-    if (__ldg(S.env_row + y + 1) - __ldg(S.env_row + y) <= 0.0f) { env_uniform(S, rng, dir, rad, pdf); return; }
-    const float r1 = pcg_f32(rng);
-    const int x = min(cdf_search(S.env_col + (size_t)y * (W + 1), W + 1, r1), W - 1);
-    const float u = ((float)x + pcg_f32(rng)) / (float)W;
-    const float v = ((float)y + pcg_f32(rng)) / (float)H;
-    float st, ct, sp, cp;
-    sincosf(kPi * v, &st, &ct);
-    sincosf(kTau * u, &sp, &cp);
-    dir = f3(cp * st, ct, sp * st);
-    rad = env_lookup(S, dir);
-    pdf = env_pdf(S, dir);
+    const bool by_cdf = env_sample_to(S, rng, dir);
+    pdf = 1.0f / (4.0f * kPi);
+    rad = env_at(S, dir, by_cdf ? &pdf : nullptr);
 }
 
 // World::sample_light (src/world.rs:171-209) with the reference's CDF quirk:

@@ -150,9 +150,28 @@ __device__ __forceinline__ void start_task(const WfScene& S0, const WfParams& P0
     sts(&st.ray_d[slot], make_float4(d.x, d.y, d.z, ifloat(-1)));
     sts(&st.beta[slot], make_float4(1.0f, 1.0f, 1.0f, 0.0f));
     sts(&st.rad[slot], make_float4(0.0f, 0.0f, 0.0f, time));
-    sts(&st.sacc[slot], make_double4(0.0, 0.0, 0.0, 0.0));
-    if (st.ssq) st.ssq[slot] = make_double4(0.0, 0.0, 0.0, 0.0);
     if (st.welford) st.welford[slot] = make_double2(0.0, 0.0);
+}
+
+// A sample's radiance joins its task's f64 sums (a: radiance and count, q:
+// squares), which start at zero with the task's first sample and go to the
+// slot's record while samples are left (`keep`): a one-sample task (most
+// renders that do not fill the pool) never touches the record.
+__device__ __forceinline__ void add_sample(const WfState& st, int slot, float3 L, bool first, bool keep, double4& a,
+                                           double4& q) {
+    a = q = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (!first) {
+        a = lds(&st.sacc[slot]);
+        if (st.ssq) q = lds(&st.ssq[slot]);
+    }
+    a.x += (double)L.x; a.y += (double)L.y; a.z += (double)L.z; a.w += 1.0;
+    if (st.ssq) {
+        q.x += (double)L.x * (double)L.x; q.y += (double)L.y * (double)L.y; q.z += (double)L.z * (double)L.z;
+    }
+    if (keep) {
+        sts(&st.sacc[slot], a);
+        if (st.ssq) sts(&st.ssq[slot], q);
+    }
 }
 
 template <bool BATCH>
@@ -238,14 +257,8 @@ __device__ __forceinline__ bool camera_miss_next(const WfScene& S0, const WfPara
         sts(&st.rsamp[(size_t)tp.j * P.round_len + (tp.sample_start - P.sample_base) + m.x],
             make_float4(L.x, L.y, L.z, 0.0f));
     } else {
-        double4 a = lds(&st.sacc[slot]);
-        a.x += (double)L.x; a.y += (double)L.y; a.z += (double)L.z; a.w += 1.0;
-        sts(&st.sacc[slot], a);
-        if (st.ssq) {
-            double4 q = lds(&st.ssq[slot]);
-            q.x += (double)L.x * (double)L.x; q.y += (double)L.y * (double)L.y; q.z += (double)L.z * (double)L.z;
-            sts(&st.ssq[slot], q);
-        }
+        double4 a, q;
+        add_sample(st, slot, L, m.x == 0, true, a, q);
     }
     m.x += 1;
     const int pixel = tp.pixel;
@@ -363,27 +376,11 @@ __device__ __forceinline__ float3 take_pending(const WfState& st, int slot, int&
 // written and the path state reset (returns true); otherwise the task's sums
 // go to the film (one task per pixel) or to the task's partial sums, and
 // need_task is set so the slot takes a new task.
-__device__ __forceinline__ bool finish_sample(const WfScene& S, const WfParams& P, const WfState& st, int slot,
-                                              int4& m, int& fl, float3& L, float3& beta, float& last_pdf,
-                                              float& ptime, uint64_t& rng, bool& need_task, const Film& F,
-                                              long long base) {
+// finish_sums does all of that but the camera ray; tp is the task's place.
+__device__ __forceinline__ bool finish_sums(const WfParams& P, const WfState& st, int slot, int4& m, float3 L,
+                                            bool& need_task, const Film& F, const TaskPos& tp) {
     const long long task = (long long)m.w;       // batch-wide task id
-    const long long lt = task - base;            // within its job
-    const TaskPos tp = task_pos(P, lt);
-    double4 a = make_double4(0.0, 0.0, 0.0, 0.0);
-    if (st.rsamp) {  // adaptive round: the sample itself, for the in-order stopping rule
-        sts(&st.rsamp[(size_t)tp.j * P.round_len + (tp.sample_start - P.sample_base) + m.x],
-            make_float4(L.x, L.y, L.z, 0.0f));
-    } else {
-        a = lds(&st.sacc[slot]);
-        a.x += (double)L.x; a.y += (double)L.y; a.z += (double)L.z; a.w += 1.0;
-        sts(&st.sacc[slot], a);
-        if (st.ssq) {
-            double4 q = st.ssq[slot];
-            q.x += (double)L.x * (double)L.x; q.y += (double)L.y * (double)L.y; q.z += (double)L.z * (double)L.z;
-            st.ssq[slot] = q;
-        }
-    }
+    const bool first = m.x == 0;
     m.x += 1;
     const int task_len = tp.len;
     bool stop = m.x >= task_len;
@@ -400,32 +397,37 @@ __device__ __forceinline__ bool finish_sample(const WfScene& S, const WfParams& 
             if (sqrt(var) / fmax(fabs(wv.x), 1e-4) < P.adaptive_threshold) stop = true;
         }
     }
-    const int pixel = tp.pixel;
-    if (stop && st.rsamp) {  // adaptive round: k_round_merge adds the samples
-        need_task = true;
-        return false;
+    need_task = stop;
+    if (st.rsamp) {  // adaptive round: the sample itself, for the in-order stopping rule (k_round_merge adds it)
+        sts(&st.rsamp[(size_t)tp.j * P.round_len + (tp.sample_start - P.sample_base) + m.x - 1],
+            make_float4(L.x, L.y, L.z, 0.0f));
+        return !stop;
     }
+    double4 a, q;
+    add_sample(st, slot, L, first, !stop, a, q);
     if (stop) {
         if (P.n_chunks == 1) {  // one task per pixel: straight into the film
-            const size_t px = (size_t)pixel;
+            const size_t px = (size_t)tp.pixel;
             F.acc[3 * px] = a.x; F.acc[3 * px + 1] = a.y; F.acc[3 * px + 2] = a.z;
             F.acc_w[px] = a.w;
-            if (F.acc_sq) {
-                const double4 q = st.ssq[slot];
-                F.acc_sq[3 * px] = q.x; F.acc_sq[3 * px + 1] = q.y; F.acc_sq[3 * px + 2] = q.z;
-            }
+            if (F.acc_sq) { F.acc_sq[3 * px] = q.x; F.acc_sq[3 * px + 1] = q.y; F.acc_sq[3 * px + 2] = q.z; }
         } else {  // per-task sums, merged in task order by k_merge
             st.part[task - P.task_first] = a;
-            if (st.part_sq) st.part_sq[task - P.task_first] = st.ssq[slot];
+            if (st.part_sq) st.part_sq[task - P.task_first] = q;
         }
-        need_task = true;
-        return false;
     }
+    return !stop;
+}
+__device__ __forceinline__ bool finish_sample(const WfScene& S, const WfParams& P, const WfState& st, int slot,
+                                              int4& m, int& fl, float3& L, float3& beta, float& last_pdf,
+                                              float& ptime, uint64_t& rng, bool& need_task, const Film& F,
+                                              long long base) {
+    const TaskPos tp = task_pos(P, (long long)m.w - base);
+    if (!finish_sums(P, st, slot, m, L, need_task, F, tp)) return false;
     float3 o, d;
-    const int row = (int)fdiv(P.w_div, (uint32_t)pixel);
-    camera_ray(S.cam, pixel - row * P.width, P.row_begin + row * P.row_step, 1.0f / (float)P.width,
-               1.0f / (float)P.height, rng, o, d,
-               ptime);
+    const int row = (int)fdiv(P.w_div, (uint32_t)tp.pixel);
+    camera_ray(S.cam, tp.pixel - row * P.width, P.row_begin + row * P.row_step, 1.0f / (float)P.width,
+               1.0f / (float)P.height, rng, o, d, ptime);
     sts(&st.ray_o[slot], make_float4(o.x, o.y, o.z, ifloat(-1)));
     sts(&st.ray_d[slot], make_float4(d.x, d.y, d.z, ifloat(-1)));
     beta = f3(1.0f, 1.0f, 1.0f);
@@ -437,21 +439,26 @@ __device__ __forceinline__ bool finish_sample(const WfScene& S, const WfParams& 
 }
 
 // Slots whose task finished take the next tasks from the pool (one atomic
-// per warp).  Must be called by all lanes of a converged warp.
-template <bool BATCH>
-__device__ __forceinline__ bool take_next_task(const WfScene& S, const WfParams& P, const WfState& st, int slot,
-                                               bool need_task) {
+// per warp); -1 = none left, or not wanted.  Must be called by all lanes of
+// a converged warp.
+__device__ __forceinline__ long long next_task(const WfParams& P, const WfState& st, bool need_task) {
     const unsigned want = __ballot_sync(0xffffffffu, need_task);
-    if (!want) return false;
+    if (!want) return -1;
     const int leader = __ffs(want) - 1;
     long long t0 = 0;
     if ((int)lane_id() == leader)
         t0 = (long long)atomicAdd((unsigned long long*)&st.ctr->next_task, (unsigned long long)__popc(want));
     t0 = __shfl_sync(0xffffffffu, t0, leader);
-    if (!need_task) return false;
+    if (!need_task) return -1;
     const long long t = t0 + __popc(want & ((1u << lane_id()) - 1u));
-    if (t >= fetch_end(P)) return false;
-    start_task<BATCH>(S, P, st, slot, task_of_fetch(P, t));
+    return t < fetch_end(P) ? task_of_fetch(P, t) : -1;
+}
+template <bool BATCH>
+__device__ __forceinline__ bool take_next_task(const WfScene& S, const WfParams& P, const WfState& st, int slot,
+                                               bool need_task) {
+    const long long task = next_task(P, st, need_task);
+    if (task < 0) return false;
+    start_task<BATCH>(S, P, st, slot, task);
     return true;
 }
 
@@ -563,260 +570,386 @@ __global__ void __launch_bounds__(128) k_shade_pre(WfScene S, WfParams P, WfStat
 // One bounce of radiance() (src/integrator.rs:67-132) per queued path, all
 // material kinds in one kernel (the default; it keeps each path's state in
 // registers through the whole bounce).
-// CTAS: resident blocks per SM the kernel is compiled for (its register
-// budget).  More warps hide the latency of the path-state loads; fewer
-// registers spill the heavier BSDF paths.  Measured on one B200 (4 vs 8):
-// the 1080p mesh+env frame runs 9% faster at 8, the adaptive Cornell frame
-// (long GGX/dielectric paths in the noisy pixels) 6% faster at 4, the batch
-// workload 8% faster at 4.
+//
+// Bound by the latency of the path-state loads and, before this shape, by
+// instruction fetch: 80 to 100 KB of straight code, of which a warp on its own
+// waited for every line (7 to 13 "no instruction" cycles per issue), at 14 of
+// 32 lanes.  So a block of 256 first orders its slots by what their rays met
+// (miss or material kind), its warps go through the stages together (1.2 "no
+// instruction" cycles left), each stage appears once -- one evaluation of the
+// env map for misses and NEE samples, one camera ray for the next sample and
+// the next task -- and the records of its next slots are prefetched.
+// Measured on one B200, ms: sphere scene 256x256 x 64 spp 2.82 -> 2.33, built-in
+// scene 853x479 x 17 spp 2.92 -> 2.32, mesh scene 960x540 x 64 spp 9.92 ->
+// 9.08, the 1080p frame 147 -> 140.  Stages without the ordering, blocks of
+// 128: 2.46 / 2.50 / 9.63 / 139; blocks of 512: 2.29 / 2.34 / 9.25 / 143.
+constexpr int kShadeBlock = 256;
 // One visit of the shading kernel to a live slot (the per-slot body of
 // k_shade, shared with k_tail): the bounce of radiance() (src/integrator.rs:
 // 67-132) for the slot's closest hit, its NEE shadow records, the sample's
-// completion when nothing is pending.  Returns what the caller's queues and
-// task fetch need.
+// completion when nothing is pending, the next camera ray.  Returns what the
+// caller's queues need.
 struct ShadeOut {
-    bool cont, term, need_task, finished_here;
+    bool cont, term, finished_here;
     int sh_env, sh_area;
 };
-template <bool BATCH>
-__device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams& P0, const WfState& st, int slot) {
-    bool cont = false, term = false, need_task = false, finished_here = false;
+// STAGED (k_shade): every thread of the block calls it, `active` or not, the
+// block's warps wait for one another between the stages, and a slot whose
+// task is done takes the next task from the pool.  Otherwise (k_tail) a
+// thread calls it alone, and a slot whose task is done is finished.
+template <bool BATCH, bool STAGED>
+__device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams& P0, const WfState& st, int slot,
+                                               bool active) {
+    auto stage = [] {
+        if constexpr (STAGED) __syncthreads();
+    };
+    bool finished_here = false, done = false, surface = false;
     int sh_env = 0, sh_area = 0;
     WfScene S = S0;
     WfParams P = P0;
     Film F = film_of(st);
     long long tbase = 0;
-    if constexpr (BATCH) apply_job(P0.jobs[st.job[slot]], S, P, F, tbase);
-    const bool has_env = S.env_kind == TPT_ENV_MAP;
-    const float4 o4 = lds(&st.ray_o[slot]), d4 = lds(&st.ray_d[slot]);
-    const float3 ro = f3(o4), rd = f3(d4);
-    const float4 h4 = lds(&st.hit[slot]);
-    const int prim = fbits(h4.y), inst = fbits(h4.z);
-    const float4 b4 = lds(&st.beta[slot]);
-    float3 beta = f3(b4);
-    float last_pdf = b4.w;
-    const float4 r4 = lds(&st.rad[slot]);
-    float3 L = f3(r4);
-    float ptime = r4.w;
-    int4 m;
-    uint64_t rng;
-    load_path(st, slot, m, rng);
-    int fl = m.z;
-    L = take_pending(st, slot, fl, L);
-    bool done = m.y >= P.max_bounces;  // max_bounces = 0: radiance() returns 0
-    if (!done && prim < 0) {  // miss (:71-83)
-        float3 contrib = beta * background(S, rd);
-        if (has_env && (fl & F_LAST_ND)) contrib = contrib * mis(last_pdf, env_pdf(S, rd));
+    float3 ro = f3(0, 0, 0), rd = f3(0, 0, 0), beta = f3(0, 0, 0), L = f3(0, 0, 0), hp = f3(0, 0, 0), ng = f3(0, 0, 0);
+    float last_pdf = 0.0f, ptime = 0.0f, t_hit = 0.0f;
+    int prim = -1, inst = -1, fl = 0, mid = 0, kind = 0;
+    int4 m = make_int4(0, 0, 0, 0);
+    uint64_t rng = 0;
+    bool has_env = false;
+    if (active) {
+        if constexpr (BATCH) apply_job(P0.jobs[st.job[slot]], S, P, F, tbase);
+        has_env = S.env_kind == TPT_ENV_MAP;
+        const float4 o4 = lds(&st.ray_o[slot]), d4 = lds(&st.ray_d[slot]);
+        ro = f3(o4);
+        rd = f3(d4);
+        const float4 h4 = lds(&st.hit[slot]);
+        t_hit = h4.x;
+        prim = fbits(h4.y);
+        inst = fbits(h4.z);
+        const float4 b4 = lds(&st.beta[slot]);
+        beta = f3(b4);
+        last_pdf = b4.w;
+        const float4 r4 = lds(&st.rad[slot]);
+        L = f3(r4);
+        ptime = r4.w;
+        load_path(st, slot, m, rng);
+        fl = m.z;
+        L = take_pending(st, slot, fl, L);
+        done = m.y >= P.max_bounces;  // max_bounces = 0: radiance() returns 0
+    }
+    const bool miss = active && !done && prim < 0;
+    if (active && !done && !miss) {
+        if (m.y >= P.rr_start) {  // Russian roulette (:89-95)
+            const float p = fmaxf(fminf(max3(beta), 0.95f), 0.05f);
+            if (pcg_f32(rng) > p) done = true;
+            else beta = beta / p;
+        }
+        if (!done) {
+            hp = ro + rd * t_hit;
+            if (inst < 0) {
+                const SphereF32 sp = S.spheres[prim];
+                ng = (hp - f3(sp.cr)) / sp.cr.w;
+                mid = sp.mat;
+            } else {
+                const TriF32* tp = S.tris + (prim - S.n_spheres);
+                const float4 v0 = __ldg(&tp->v0), e1 = __ldg(&tp->e1), e2 = __ldg(&tp->e2);
+                const float3 no = cross(f3(e1), f3(e2));
+                const InstanceF32* I = S.inst + inst;
+                const float4 n0 = __ldg(&I->nrm[0]), n1 = __ldg(&I->nrm[1]), n2 = __ldg(&I->nrm[2]);
+                ng = normalize(f3(n0.x * no.x + n0.y * no.y + n0.z * no.z, n1.x * no.x + n1.y * no.y + n1.z * no.z,
+                                  n2.x * no.x + n2.y * no.y + n2.z * no.z));
+                const int ov = fbits(__ldg(&I->wbox_max.w));
+                mid = ov >= 0 ? ov : fbits(v0.w);
+            }
+            kind = S.mats[mid].kind;
+            if (kind == TPT_MAT_DIFFUSE_LIGHT) {  // emitter (:100-104)
+                L = L + clamp_lum(beta * f3(S.mats[mid].c), 50.0f);
+                done = true;
+            } else {
+                surface = true;
+            }
+        }
+    }
+    const bool nee = surface && kind != TPT_MAT_METAL && kind != TPT_MAT_DIELECTRIC;
+    const bool entering = dot(ng, rd) < 0.0f;
+    const float3 n = entering ? ng : -ng;
+    const float3 wo = -rd;
+    stage();
+    // the env map in the ray's direction (a miss) or the NEE sample's
+    float3 wi = rd, li = f3(0, 0, 0);
+    float pe = 1.0f / (4.0f * kPi);
+    bool want_pdf = (fl & F_LAST_ND) != 0;
+    if (nee && has_env) want_pdf = env_sample_to(S, rng, wi);
+    stage();
+    if (has_env && (miss || nee)) {
+        float pdf = pe;
+        li = env_at(S, wi, &pdf);
+        if (want_pdf) pe = pdf;
+    }
+    stage();
+    if (miss) {  // (:71-83)
+        if (!has_env) li = sky(rd);
+        float3 contrib = beta * li;
+        if (has_env && (fl & F_LAST_ND)) contrib = contrib * mis(last_pdf, pe);
         L = L + clamp_lum(contrib, 50.0f);
         done = true;
     }
-    if (!done && m.y >= P.rr_start) {  // Russian roulette (:89-95)
-        const float p = fmaxf(fminf(max3(beta), 0.95f), 0.05f);
-        if (pcg_f32(rng) > p) done = true;
-        else beta = beta / p;
-    }
-    if (!done) {
-        const float3 hp = ro + rd * h4.x;
-        float3 ng;
-        int mid;
-        if (inst < 0) {
-            const SphereF32 sp = S.spheres[prim];
-            ng = (hp - f3(sp.cr)) / sp.cr.w;
-            mid = sp.mat;
-        } else {
-            const TriF32* tp = S.tris + (prim - S.n_spheres);
-            const float4 v0 = __ldg(&tp->v0), e1 = __ldg(&tp->e1), e2 = __ldg(&tp->e2);
-            const float3 no = cross(f3(e1), f3(e2));
-            const InstanceF32* I = S.inst + inst;
-            const float4 n0 = __ldg(&I->nrm[0]), n1 = __ldg(&I->nrm[1]), n2 = __ldg(&I->nrm[2]);
-            ng = normalize(f3(n0.x * no.x + n0.y * no.y + n0.z * no.z, n1.x * no.x + n1.y * no.y + n1.z * no.z,
-                              n2.x * no.x + n2.y * no.y + n2.z * no.z));
-            const int ov = fbits(__ldg(&I->wbox_max.w));
-            mid = ov >= 0 ? ov : fbits(v0.w);
+    if (nee && has_env) {  // nee_environment (:148-172)
+        const float c = fmaxf(dot(n, wi), 0.0f);
+        if (c > 0.0f && pe > 0.0f) {
+            float3 f;
+            float pb;
+            mat_eval(S.mats[mid], wo, wi, n, f, pb);
+            const float3 contrib = beta * f * li * (c * mis(pe, pb) / pe);
+            if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) {
+                const float3 so = hp + wi * kEps;
+                sts(&st.sh_o[2 * slot], make_float4(so.x, so.y, so.z, kTMax));
+                sts(&st.sh_d[2 * slot], make_float4(wi.x, wi.y, wi.z, ifloat(prim)));
+                sts(&st.sh_c[2 * slot], make_float4(contrib.x, contrib.y, contrib.z, ifloat(inst)));
+                sh_env = 1;
+                fl |= F_PEND_ENV;
+            }
         }
-        const MaterialF32 mt = S.mats[mid];
-        const float3 mc = f3(mt.c);
-        if (mt.kind == TPT_MAT_DIFFUSE_LIGHT) {  // emitter (:100-104)
-            L = L + clamp_lum(beta * mc, 50.0f);
-            done = true;
-        } else {
-            const bool entering = dot(ng, rd) < 0.0f;
-            const float3 n = entering ? ng : -ng;
-            const float3 wo = -rd;
-            if (mt.kind != TPT_MAT_METAL && mt.kind != TPT_MAT_DIELECTRIC) {
-                if (has_env) {  // nee_environment (:148-172)
-                    float3 wi, li;
-                    float pe;
-                    env_sample_dir(S, rng, wi, li, pe);
-                    const float c = fmaxf(dot(n, wi), 0.0f);
-                    if (c > 0.0f && pe > 0.0f) {
-                        float3 f;
-                        float pb;
-                        mat_eval(mt, wo, wi, n, f, pb);
-                        const float3 contrib = beta * f * li * (c * mis(pe, pb) / pe);
-                        if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) {
-                            const float3 so = hp + wi * kEps;
-                            sts(&st.sh_o[2 * slot], make_float4(so.x, so.y, so.z, kTMax));
-                            sts(&st.sh_d[2 * slot], make_float4(wi.x, wi.y, wi.z, ifloat(prim)));
-                            sts(&st.sh_c[2 * slot], make_float4(contrib.x, contrib.y, contrib.z, ifloat(inst)));
-                            sh_env = 1;
-                            fl |= F_PEND_ENV;
-                        }
-                    }
-                }
-                float3 lp, le;
-                float lpdf;
-                int lidx;
-                double lud, lvd;
-                if (sample_light(S, rng, hp, lp, le, lpdf, lidx, lud, lvd)) {  // nee_area_light (:178-213)
-                    const float3 tl = lp - hp;
-                    const float dist = length(tl);
-                    if (dist > 1e-6f) {
-                        const float3 wi = tl / dist;
-                        const float c = fmaxf(dot(n, wi), 0.0f);
-                        if (c > 0.0f && !ref_light_self_occluded(S.lights64, S.spheres64, S.inst64, lidx, ro, rd, h4.x, lud, lvd, (double)ptime)) {
-                            float3 f;
-                            float pb;
-                            mat_eval(mt, wo, wi, n, f, pb);
-                            const float3 contrib = beta * f * le * (c * mis(lpdf, pb) / lpdf);
-                            if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) {
-                                const float3 so = hp + wi * kEps;
-                                // stops 1e-4 short of the light: the light itself is
-                                // handled by ref_light_self_occluded
-                                sts(&st.sh_o[2 * slot + 1], make_float4(so.x, so.y, so.z, fmaxf(dist - 2.0f * kEps, kEps)));
-                                sts(&st.sh_d[2 * slot + 1], make_float4(wi.x, wi.y, wi.z, ifloat(prim)));
-                                sts(&st.sh_c[2 * slot + 1], make_float4(contrib.x, contrib.y, contrib.z, ifloat(inst)));
-                                sh_area = 1;
-                                fl |= F_PEND_AREA;
-                            }
-                        }
+    }
+    stage();
+    if (nee) {
+        float3 lp, le;
+        float lpdf;
+        int lidx;
+        double lud, lvd;
+        if (sample_light(S, rng, hp, lp, le, lpdf, lidx, lud, lvd)) {  // nee_area_light (:178-213)
+            const float3 tl = lp - hp;
+            const float dist = length(tl);
+            if (dist > 1e-6f) {
+                const float3 wl = tl / dist;
+                const float c = fmaxf(dot(n, wl), 0.0f);
+                if (c > 0.0f && !ref_light_self_occluded(S.lights64, S.spheres64, S.inst64, lidx, ro, rd, t_hit, lud, lvd, (double)ptime)) {
+                    float3 f;
+                    float pb;
+                    mat_eval(S.mats[mid], wo, wl, n, f, pb);
+                    const float3 contrib = beta * f * le * (c * mis(lpdf, pb) / lpdf);
+                    if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) {
+                        const float3 so = hp + wl * kEps;
+                        // stops 1e-4 short of the light: the light itself is
+                        // handled by ref_light_self_occluded
+                        sts(&st.sh_o[2 * slot + 1], make_float4(so.x, so.y, so.z, fmaxf(dist - 2.0f * kEps, kEps)));
+                        sts(&st.sh_d[2 * slot + 1], make_float4(wl.x, wl.y, wl.z, ifloat(prim)));
+                        sts(&st.sh_c[2 * slot + 1], make_float4(contrib.x, contrib.y, contrib.z, ifloat(inst)));
+                        sh_area = 1;
+                        fl |= F_PEND_AREA;
                     }
                 }
             }
-            // Material::sample (src/material.rs:76-201)
-            float3 nd = f3(0, 0, 0), w = f3(0, 0, 0), no = hp;
-            float pdf = 0.0f;
-            bool delta = false, ok = true, self_ok = true;
-            switch (mt.kind) {
-                case TPT_MAT_LAMBERT:
-                    nd = cos_hemi(n, rng);
-                    w = mc;
-                    pdf = fmaxf(dot(n, nd), 0.0f) / kPi;
-                    break;
-                case TPT_MAT_METAL:
-                    nd = rd - n * (2.0f * dot(rd, n));
-                    w = mc;
-                    delta = true;
-                    break;
-                case TPT_MAT_DIELECTRIC: {
-                    const float ior = mt.c.w;
-                    const float eta = entering ? 1.0f / ior : ior;
-                    const float ci = fmaxf(dot(wo, n), 0.0f);
-                    const float fq = (ior - 1.0f) / (ior + 1.0f);
-                    const float f0 = fq * fq;
-                    const float fr = f0 + (1.0f - f0) * pow5(1.0f - ci);
-                    float3 bt = f3(1, 1, 1);
-                    if (!entering) {
-                        const float dist = fmaxf(h4.x, 0.0f);
-                        bt = f3(__expf(-mc.x * dist), __expf(-mc.y * dist), __expf(-mc.z * dist));
-                    }
-                    const float cosi = fminf(fmaxf(dot(wo, n), -1.0f), 1.0f);
-                    const float sin2t = eta * eta * (1.0f - cosi * cosi);
-                    const bool has_refr = !(sin2t >= 1.0f);
-                    const bool refl = !has_refr || pcg_f32(rng) < fr;
-                    if (refl) {
-                        nd = rd - n * (2.0f * dot(rd, n));
-                        bt = bt * (fr / fmaxf(fr, 1e-6f));
-                    } else {
-                        nd = rd * eta + n * (eta * cosi - sqrtf(1.0f - sin2t));
-                        bt = bt * ((1.0f - fr) / fmaxf(1.0f - fr, 1e-6f)) * (eta * eta);
-                    }
-                    w = bt;
-                    delta = true;
-                    break;
-                }
-                case TPT_MAT_GGX: {
-                    GgxSample gs;
-                    if (!ggx_sample(rd, n, mt, rng, gs)) { ok = false; break; }
-                    nd = gs.nd;
-                    w = gs.w;
-                    pdf = gs.pdf;
-                    break;
-                }
-                case TPT_MAT_SUBSURFACE: {
+        }
+    }
+    stage();
+    if (surface) {  // Material::sample (src/material.rs:76-201)
+        const MaterialF32 mt = S.mats[mid];
+        const float3 mc = f3(mt.c);
+        float3 nd = f3(0, 0, 0), w = f3(0, 0, 0), no = hp;
+        float pdf = 0.0f;
+        bool delta = false, ok = true, self_ok = true;
+        switch (kind) {
+            case TPT_MAT_LAMBERT:
+            case TPT_MAT_SUBSURFACE: {
+                const bool sub = kind == TPT_MAT_SUBSURFACE;
+                w = mc;
+                if (sub) {
                     const float sc = fmaxf(mt.c.w, 1e-4f);
                     const float u = fmaxf(pcg_f32(rng), 1e-12f);
                     const float dist = -__logf(u) * sc;
-                    nd = cos_hemi(ng, rng);  // unoriented normal (material.rs:187-188)
                     w = mc * __expf(-dist / sc);
                     no = hp - ng * dist;
-                    pdf = fmaxf(dot(n, nd), 0.0f) / kPi;
                     self_ok = false;     // origin moved off the surface
-                    break;
                 }
-                default:
-                    ok = false;
+                nd = cos_hemi(sub ? ng : n, rng);  // subsurface: unoriented normal (material.rs:187-188)
+                pdf = fmaxf(dot(n, nd), 0.0f) / kPi;
+                break;
             }
-            if (!ok) {
-                done = true;
-            } else {
-                beta = beta * w;
-                last_pdf = pdf;
-                fl = delta ? (fl & ~F_LAST_ND) : (fl | F_LAST_ND);
-                const float3 o2 = no + nd * kEps;
-                sts(&st.ray_o[slot], make_float4(o2.x, o2.y, o2.z, ifloat(self_ok ? prim : -1)));
-                sts(&st.ray_d[slot], make_float4(nd.x, nd.y, nd.z, ifloat(self_ok ? inst : -1)));
-                m.y += 1;
-                if (m.y >= P.max_bounces) done = true;  // bounce loop bound (:67)
+            case TPT_MAT_METAL:
+                nd = rd - n * (2.0f * dot(rd, n));
+                w = mc;
+                delta = true;
+                break;
+            case TPT_MAT_DIELECTRIC: {
+                const float ior = mt.c.w;
+                const float eta = entering ? 1.0f / ior : ior;
+                const float ci = fmaxf(dot(wo, n), 0.0f);
+                const float fq = (ior - 1.0f) / (ior + 1.0f);
+                const float f0 = fq * fq;
+                const float fr = f0 + (1.0f - f0) * pow5(1.0f - ci);
+                float3 bt = f3(1, 1, 1);
+                if (!entering) {
+                    const float dist = fmaxf(t_hit, 0.0f);
+                    bt = f3(__expf(-mc.x * dist), __expf(-mc.y * dist), __expf(-mc.z * dist));
+                }
+                const float cosi = fminf(fmaxf(dot(wo, n), -1.0f), 1.0f);
+                const float sin2t = eta * eta * (1.0f - cosi * cosi);
+                const bool has_refr = !(sin2t >= 1.0f);
+                const bool refl = !has_refr || pcg_f32(rng) < fr;
+                if (refl) {
+                    nd = rd - n * (2.0f * dot(rd, n));
+                    bt = bt * (fr / fmaxf(fr, 1e-6f));
+                } else {
+                    nd = rd * eta + n * (eta * cosi - sqrtf(1.0f - sin2t));
+                    bt = bt * ((1.0f - fr) / fmaxf(1.0f - fr, 1e-6f)) * (eta * eta);
+                }
+                w = bt;
+                delta = true;
+                break;
             }
+            case TPT_MAT_GGX: {
+                GgxSample gs;
+                if (!ggx_sample(rd, n, mt, rng, gs)) { ok = false; break; }
+                nd = gs.nd;
+                w = gs.w;
+                pdf = gs.pdf;
+                break;
+            }
+            default:
+                ok = false;
+        }
+        if (!ok) {
+            done = true;
+        } else {
+            beta = beta * w;
+            last_pdf = pdf;
+            fl = delta ? (fl & ~F_LAST_ND) : (fl | F_LAST_ND);
+            const float3 o2 = no + nd * kEps;
+            sts(&st.ray_o[slot], make_float4(o2.x, o2.y, o2.z, ifloat(self_ok ? prim : -1)));
+            sts(&st.ray_d[slot], make_float4(nd.x, nd.y, nd.z, ifloat(self_ok ? inst : -1)));
+            m.y += 1;
+            if (m.y >= P.max_bounces) done = true;  // bounce loop bound (:67)
         }
     }
-    if (done && !sh_env && !sh_area) {
+    stage();
+    bool cont = active && !done, need_task = false, camera = false;
+    const bool term = active && done && (sh_env || sh_area);
+    TaskPos tp{};
+    if (active && done && !term) {
         // Nothing pending: finish the sample here instead of in k_regen.
-        cont = finish_sample(S, P, st, slot, m, fl, L, beta, last_pdf, ptime, rng, need_task, F, tbase);
+        tp = task_pos(P, (long long)m.w - tbase);
+        camera = finish_sums(P, st, slot, m, L, need_task, F, tp);
         finished_here = true;
-    } else {
-        cont = !done;
-        term = done;
     }
-    sts(&st.beta[slot], make_float4(beta.x, beta.y, beta.z, last_pdf));
-    sts(&st.rad[slot], make_float4(L.x, L.y, L.z, ptime));
-    m.z = fl;
-    store_path(st, slot, m, rng);
-    return ShadeOut{cont, term, need_task, finished_here, sh_env, sh_area};
+    if constexpr (STAGED) {
+        const long long task = next_task(P0, st, need_task);
+        if (task >= 0) {
+            if constexpr (BATCH) {
+                const int j = find_job(P0, task);
+                st.job[slot] = j;
+                apply_job(P0.jobs[j], S, P, F, tbase);
+            }
+            tp = task_pos(P, task - tbase);
+            m = make_int4(0, 0, 0, (int)task);
+            if (st.welford) st.welford[slot] = make_double2(0.0, 0.0);
+            camera = true;
+            need_task = false;
+        }
+    }
+    if (camera) {
+        const int row = (int)fdiv(P.w_div, (uint32_t)tp.pixel);
+        const int x = tp.pixel - row * P.width, y = P.row_begin + row * P.row_step;
+        if (m.x == 0) rng = task_seed((uint32_t)x, (uint32_t)y, (uint32_t)tp.sample_start, P.seed);  // a new task
+        float3 o, d;
+        camera_ray(S.cam, x, y, 1.0f / (float)P.width, 1.0f / (float)P.height, rng, o, d, ptime);
+        sts(&st.ray_o[slot], make_float4(o.x, o.y, o.z, ifloat(-1)));
+        sts(&st.ray_d[slot], make_float4(d.x, d.y, d.z, ifloat(-1)));
+        beta = f3(1.0f, 1.0f, 1.0f);
+        last_pdf = 0.0f;
+        L = f3(0, 0, 0);
+        m.y = 0;
+        fl = 0;
+        cont = true;
+    }
+    if (active && !need_task) {
+        sts(&st.beta[slot], make_float4(beta.x, beta.y, beta.z, last_pdf));
+        sts(&st.rad[slot], make_float4(L.x, L.y, L.z, ptime));
+        m.z = fl;
+        store_path(st, slot, m, rng);
+    }
+    return ShadeOut{cont, term, finished_here, sh_env, sh_area};
 }
 
+// What the shading stages do with a live slot: 0 = its ray left the scene, 1 +
+// the material kind it hit.
+__device__ __forceinline__ int shade_class(const WfScene& S, const WfState& st, int slot) {
+    const float4 h4 = __ldg(&st.hit[slot]);
+    const int prim = fbits(h4.y), inst = fbits(h4.z);
+    if (prim < 0) return 0;
+    int mid;
+    if (inst < 0) {
+        mid = __ldg(&S.spheres[prim].mat);
+    } else {
+        const int ov = fbits(__ldg(&S.inst[inst].wbox_max.w));
+        mid = ov >= 0 ? ov : fbits(__ldg(&S.tris[prim - S.n_spheres].v0.w));
+    }
+    return 1 + __ldg(&S.mats[mid].kind);
+}
+// The block's slots ordered by class, stable: thread t gets the t-th.  cls:
+// the thread's own class (7 = no slot).
+__device__ __forceinline__ int sort_by_class(int slot, int cls, int (*counts)[8], int* order) {
+    const int w = threadIdx.x >> 5;
+    int rank = 0;
+    for (int k = 0; k < 8; ++k) {
+        const unsigned m = __ballot_sync(0xffffffffu, cls == k);
+        if (cls == k) rank = __popc(m & ((1u << lane_id()) - 1u));
+        if (lane_id() == (unsigned)k) counts[w][k] = __popc(m);
+    }
+    __syncthreads();
+    // exclusive prefix over (class, warp), one warp
+    constexpr int W = kShadeBlock / 32;
+    if (w == 0) {
+        int run = 0;
+        for (int k = 0; k < 8; ++k) {
+            int v = lane_id() < (unsigned)W ? counts[lane_id()][k] : 0, x = v;
+            for (int off = 1; off < W; off <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, off);
+                if ((int)lane_id() >= off) x += y;
+            }
+            if (lane_id() < (unsigned)W) counts[lane_id()][k] = run + x - v;
+            run += __shfl_sync(0xffffffffu, x, W - 1);
+        }
+    }
+    __syncthreads();
+    order[counts[w][cls] + rank] = cls == 7 ? -1 : slot;
+    __syncthreads();
+    return order[threadIdx.x];
+}
+
+// CTAS: blocks of 128 threads' worth of registers per SM (4, 6 or 8).
 template <bool BATCH, int CTAS>
-__global__ void __launch_bounds__(128, CTAS) k_shade(WfScene S0, WfParams P0, WfState st, int cur) {
-    // At 6+ blocks per SM the kernel spills: ptxas may put the spills in
-    // shared memory (13 KB per block) instead of local memory, which at
-    // 1024 threads per SM does not fit in L1 (1080p frame: +1.0% paths/s).
+__global__ void __launch_bounds__(kShadeBlock, CTAS * 128 / kShadeBlock) k_shade(WfScene S0, WfParams P0, WfState st,
+                                                                                int cur) {
+    // At 6+ blocks of 128 per SM the kernel spills: ptxas may put the spills
+    // in shared memory instead of local memory, which at 1024 threads per SM
+    // does not fit in L1 (1080p frame: +1.0% paths/s).
     if constexpr (CTAS >= 6) asm volatile(".pragma \"enable_smem_spilling\";");
+    __shared__ int counts[kShadeBlock / 32][8], order[kShadeBlock];
     const int live = st.ctr->n_ext[cur];  // the slots the closest-hit kernel traced
     const bool use_q = P0.ordered_queue || use_ext_queue(live, P0.n_slots, P0.queue_div);
     const int n = use_q ? live : P0.n_slots;
     const int* __restrict__ qe = st.q_ext[cur];
     const int nxt = cur ^ 1;
     const int stride = gridDim.x * blockDim.x;
-    for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
-        const int i = base + (int)lane_id();
-        const bool active = i < n && (use_q || st.act[i]);
-        bool cont = false, term = false, need_task = false, finished_here = false;
-        int slot = 0;
-        int sh_env = 0, sh_area = 0;
-        if (active) {
-            slot = use_q ? qe[i] : i;
-            const ShadeOut r = shade_slot<BATCH>(S0, P0, st, slot);
-            cont = r.cont; term = r.term; need_task = r.need_task; finished_here = r.finished_here;
-            sh_env = r.sh_env; sh_area = r.sh_area;
+    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+        const int i = base + (int)threadIdx.x;
+        bool active = i < n && (use_q || st.act[i]);
+        int slot = active ? (use_q ? qe[i] : i) : 0;
+        slot = sort_by_class(slot, active ? shade_class(S0, st, slot) : 7, counts, order);
+        active = slot >= 0;
+        if (use_q && i + stride < n) {  // the records of the block's next slots, on their way to L2
+            const int next = __ldg(qe + i + stride);
+            auto fetch = [](const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); };
+            fetch(st.ray_o + next); fetch(st.ray_d + next); fetch(st.hit + next);
+            fetch(st.beta + next); fetch(st.rad + next); fetch(st.path + next);
         }
-        if (take_next_task<BATCH>(S0, P0, st, slot, need_task)) cont = true;
-        if (active) st.act[slot] = cont ? 1 : 0;
-        if (!P0.ordered_queue) warp_push(st.q_ext[nxt], &st.ctr->n_ext[nxt], cont, slot);
-        warp_push(st.q_term, &st.ctr->n_term, term, slot);
-        warp_count(&st.ctr->n_done_in_shade, finished_here);
-        warp_push(st.q_sh, &st.ctr->n_sh, sh_env != 0, 2 * slot);
-        warp_push(st.q_sh, &st.ctr->n_sh, sh_area != 0, 2 * slot + 1);
+        const ShadeOut r = shade_slot<BATCH, true>(S0, P0, st, slot, active);
+        if (active) st.act[slot] = r.cont ? 1 : 0;
+        if (!P0.ordered_queue) warp_push(st.q_ext[nxt], &st.ctr->n_ext[nxt], r.cont, slot);
+        warp_push(st.q_term, &st.ctr->n_term, r.term, slot);
+        warp_count(&st.ctr->n_done_in_shade, r.finished_here);
+        warp_push(st.q_sh, &st.ctr->n_sh, r.sh_env != 0, 2 * slot);
+        warp_push(st.q_sh, &st.ctr->n_sh, r.sh_area != 0, 2 * slot + 1);
     }
 }
 
@@ -1378,7 +1511,7 @@ __global__ void __launch_bounds__(128) k_tail(WfScene S, WfParams P, WfState st)
             sts(&st.hit[slot], make_float4(T.hit_prim >= 0 ? T.tmax : kTMax, ifloat(T.hit_prim), ifloat(T.hit_inst),
                                            0.0f));
             ++rays_c;
-            const ShadeOut r = shade_slot<BATCH>(S, P, st, slot);
+            const ShadeOut r = shade_slot<BATCH, false>(S, P, st, slot, true);
             if (r.finished_here) ++samples;
             for (int k = 0; k < 2; ++k) {
                 if (!(k == 0 ? r.sh_env : r.sh_area)) continue;
@@ -1872,14 +2005,14 @@ struct Grids { int extend, shade, shadow, regen, surface[5], shade_all, shade_al
 // (each returns at once when its queue is empty).
 void launch_shade(const Grids& g, cudaStream_t s, const WfScene& S, const WfParams& P, const WfState& st, int cur) {
     if (P.jobs) {  // batch renders: fused shading only
-        if (P.shade_ctas == 8) wf::k_shade<true, 8><<<g.shade_batch8, 128, 0, s>>>(S, P, st, cur);
-        else wf::k_shade<true, 4><<<g.shade_batch, 128, 0, s>>>(S, P, st, cur);
+        if (P.shade_ctas == 8) wf::k_shade<true, 8><<<g.shade_batch8, wf::kShadeBlock, 0, s>>>(S, P, st, cur);
+        else wf::k_shade<true, 4><<<g.shade_batch, wf::kShadeBlock, 0, s>>>(S, P, st, cur);
         return;
     }
     if (!P.shade_sort) {
-        if (P.shade_ctas == 4) wf::k_shade<false, 4><<<g.shade_all4, 128, 0, s>>>(S, P, st, cur);
-        else if (P.shade_ctas == 6) wf::k_shade<false, 6><<<g.shade_all6, 128, 0, s>>>(S, P, st, cur);
-        else wf::k_shade<false, 8><<<g.shade_all, 128, 0, s>>>(S, P, st, cur);
+        if (P.shade_ctas == 4) wf::k_shade<false, 4><<<g.shade_all4, wf::kShadeBlock, 0, s>>>(S, P, st, cur);
+        else if (P.shade_ctas == 6) wf::k_shade<false, 6><<<g.shade_all6, wf::kShadeBlock, 0, s>>>(S, P, st, cur);
+        else wf::k_shade<false, 8><<<g.shade_all, wf::kShadeBlock, 0, s>>>(S, P, st, cur);
         return;
     }
     wf::k_shade_pre<<<g.shade, 128, 0, s>>>(S, P, st, cur);
@@ -1913,9 +2046,9 @@ void launch_regen(int grid, cudaStream_t s, const WfScene& S, const WfParams& P,
 }
 
 template <class K>
-int grid_for(K kernel, int sm_count) {
+int grid_for(K kernel, int sm_count, int block = 128) {
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, block, 0);
     return sm_count * (occ > 0 ? occ : 1);
 }
 
@@ -1924,11 +2057,11 @@ Grids pick_grids(int sm_count) {
     g.extend = grid_for(wf::k_trace<false, false, true, false>, sm_count);
     g.shadow = grid_for(wf::k_trace<true, false, true, false>, sm_count);
     g.shade = grid_for(wf::k_shade_pre, sm_count);
-    g.shade_all = grid_for(wf::k_shade<false, 8>, sm_count);
-    g.shade_all4 = grid_for(wf::k_shade<false, 4>, sm_count);
-    g.shade_all6 = grid_for(wf::k_shade<false, 6>, sm_count);
-    g.shade_batch = grid_for(wf::k_shade<true, 4>, sm_count);
-    g.shade_batch8 = grid_for(wf::k_shade<true, 8>, sm_count);
+    g.shade_all = grid_for(wf::k_shade<false, 8>, sm_count, wf::kShadeBlock);
+    g.shade_all4 = grid_for(wf::k_shade<false, 4>, sm_count, wf::kShadeBlock);
+    g.shade_all6 = grid_for(wf::k_shade<false, 6>, sm_count, wf::kShadeBlock);
+    g.shade_batch = grid_for(wf::k_shade<true, 4>, sm_count, wf::kShadeBlock);
+    g.shade_batch8 = grid_for(wf::k_shade<true, 8>, sm_count, wf::kShadeBlock);
     g.surface[0] = grid_for(wf::k_shade_surface<TPT_MAT_LAMBERT>, sm_count);
     g.surface[1] = grid_for(wf::k_shade_surface<TPT_MAT_METAL>, sm_count);
     g.surface[2] = grid_for(wf::k_shade_surface<TPT_MAT_DIELECTRIC>, sm_count);
