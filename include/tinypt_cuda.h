@@ -164,7 +164,8 @@ typedef struct tpt_stats {
     uint64_t paths;             /* camera samples finished (sum of acc_w)      */
     uint64_t rays_closest;      /* closest-hit traces: camera + extension      */
     uint64_t rays_shadow;       /* occlusion traces (NEE shadow rays)          */
-    uint64_t iterations;        /* wavefront iterations (0 for PLAIN_F64)      */
+    uint64_t iterations;        /* wavefront iterations (0 for PLAIN_F64 and for
+                                   small renders, which run in one kernel)   */
     int32_t  device_flags;      /* TPT_FLAG_* raised by kernels                */
     int32_t  profile;           /* in: 1 = per-stage timing + traversal counts
                                    (wavefront only; slower, for profiling)   */
@@ -250,17 +251,16 @@ int tpt_render_device(void* scene, const tpt_render_config* config,
  * TPT_MODE_WAVEFRONT_FP32 (config->mode is ignored) into the caller's DEVICE
  * buffers d_acc (width*height*3 f64) and d_acc_w (width*height f64).
  *
- * Scratch (path state, queues, counters) lives in one file-scope device array
- * of 5,128,704 bytes (about 5.1 MB) that every GPU loading the library holds
- * until exit; films larger than 16384 pixels are rejected with
- * TPT_ERR_INVALID.  The call
+ * Scratch is one file-scope device variable (the counters, under 1 KB) that
+ * every GPU loading the library holds until exit; films larger than 16384
+ * pixels are rejected with TPT_ERR_INVALID.  The call
  * makes no cudaMalloc/cudaFree and creates no graph, event or stream.
- * The first call on a device looks up the array's device address (once per
+ * The first call on a device looks up the variable's device address (once per
  * device); make that first call before any stream capture.  Under CUDA's
  * lazy module loading (the default) that first call may also be when the
- * array is placed in device memory, so make it before the caller's own
- * allocator takes the GPU's free memory.  All calls share
- * the array: calls that overlap on the GPU race and must be serialised by
+ * library's kernels are placed in device memory, so make it before the
+ * caller's own allocator takes the GPU's free memory.  All calls share
+ * the counters: calls that overlap on the GPU race and must be serialised by
  * the caller.  stats may be NULL; its profile field is ignored. */
 int tpt_render_device_noalloc(void* scene, const tpt_render_config* config, double* d_acc, double* d_acc_w,
                               tpt_stats* stats);

@@ -158,7 +158,7 @@ __device__ __noinline__ bool adj_step(const WfScene& S, const AdjParams& P, AdjP
     Tracer T;
     TraceCount cnt;
     tracer_start(S, T, p.o, p.d, kTMax, p.self_prim, p.self_inst);
-    tracer_run<false, false>(S, T, stack, kEps, 1 << 30, flags, cnt);
+    tracer_run<false>(S, T, stack, kEps, 1 << 30, flags, cnt, false);
     const int prim = T.hit_prim, inst = T.hit_inst;
     const float th = T.tmax;
     if (prim < 0) {  // miss (:71-83)
@@ -227,7 +227,7 @@ __device__ __noinline__ bool adj_step(const WfScene& S, const AdjParams& P, AdjP
                 const float3 contrib = p.beta * f * li * (c * mis(pe, pb) / pe);
                 if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) {
                     tracer_start(S, T, hp + wi * kEps, wi, kTMax, prim, inst);
-                    tracer_run<true, false>(S, T, stack, kEps, 1 << 30, flags, cnt);
+                    tracer_run<false>(S, T, stack, kEps, 1 << 30, flags, cnt, true);
                     if (T.hit_prim < 0) {
                         const float3 a = delta * contrib;
                         if (p.grad) {
@@ -258,7 +258,7 @@ __device__ __noinline__ bool adj_step(const WfScene& S, const AdjParams& P, AdjP
                     const float3 contrib = p.beta * f * le * (c * mis(lpdf, pb) / lpdf);
                     if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) {
                         tracer_start(S, T, hp + wi * kEps, wi, fmaxf(dist - 2.0f * kEps, kEps), prim, inst);
-                        tracer_run<true, false>(S, T, stack, kEps, 1 << 30, flags, cnt);
+                        tracer_run<false>(S, T, stack, kEps, 1 << 30, flags, cnt, true);
                         if (T.hit_prim < 0) {
                             const float3 a = delta * contrib;
                             if (p.grad) {

@@ -284,7 +284,7 @@ void fill_wf_params(const tpt_render_config& c, WfParams& p, bool noalloc) {
     p.ext_queue = 1;
     p.queue_div = queue_div_setting();
     p.ordered_queue = env_int("TPT_QUEUE_ORDER", 1) != 0;
-    // the drain's last live slots run to the end in k_tail; unset: -1, the
+    // the drain's last live slots run to the end in k_paths; unset: -1, the
     // default (262,144, at most a sixteenth of the pool)
     p.tail_live = noalloc ? 0 : std::max(-1, env_int("TPT_TAIL_SLOTS", -1));
     // one-task adaptive renders run the stopping rule after every sample in

@@ -238,10 +238,10 @@ __device__ __forceinline__ void tracer_pop(Tracer& T, const Stack& stack) {
 }
 
 // Runs up to `chunk` leaf visits of one ray.  Returns true when the ray is
-// finished: stack exhausted, or (ANY) an occluder found.
-template <bool ANY, bool COUNT, class Stack>
+// finished: stack exhausted, or (any) an occluder found.
+template <bool COUNT, class Stack>
 __device__ __forceinline__ bool tracer_run(const WfScene& S, Tracer& T, const Stack& stack, float tmin, int chunk, int* flags,
-                                           TraceCount& cnt) {
+                                           TraceCount& cnt, bool any) {
     for (int it = 0; it < chunk; ++it) {
         const float3 ood = f3(T.o.x * T.idir.x, T.o.y * T.idir.y, T.o.z * T.idir.z);
         while (T.ref >= 0) {
@@ -335,7 +335,7 @@ __device__ __forceinline__ bool tracer_run(const WfScene& S, Tracer& T, const St
                     T.tmax = t;
                     T.hit_prim = S.n_spheres + (int)k;
                     T.hit_inst = T.inst;
-                    if (ANY) { stop = true; break; }
+                    if (any) { stop = true; break; }
                 }
             }
         } else {  // spheres (world space)
@@ -348,7 +348,7 @@ __device__ __forceinline__ bool tracer_run(const WfScene& S, Tracer& T, const St
                     T.tmax = t;
                     T.hit_prim = (int)k;
                     T.hit_inst = -1;
-                    if (ANY) { stop = true; break; }
+                    if (any) { stop = true; break; }
                 }
             }
         }

@@ -150,27 +150,39 @@ __device__ __forceinline__ void start_task(const WfScene& S0, const WfParams& P0
     sts(&st.ray_d[slot], make_float4(d.x, d.y, d.z, ifloat(-1)));
     sts(&st.beta[slot], make_float4(1.0f, 1.0f, 1.0f, 0.0f));
     sts(&st.rad[slot], make_float4(0.0f, 0.0f, 0.0f, time));
-    if (st.welford) st.welford[slot] = make_double2(0.0, 0.0);
 }
 
-// A sample's radiance joins its task's f64 sums (a: radiance and count, q:
-// squares), which start at zero with the task's first sample and go to the
-// slot's record while samples are left (`keep`): a one-sample task (most
-// renders that do not fill the pool) never touches the record.
-__device__ __forceinline__ void add_sample(const WfState& st, int slot, float3 L, bool first, bool keep, double4& a,
-                                           double4& q) {
-    a = q = make_double4(0.0, 0.0, 0.0, 0.0);
-    if (!first) {
-        a = lds(&st.sacc[slot]);
-        if (st.ssq) q = lds(&st.ssq[slot]);
+// A task's f64 sums: radiance and count, squares (when wanted), and the
+// Welford mean and m2 of one-task adaptive sampling.  They start at zero with
+// the task's first sample and go to the slot's records while samples are
+// left, so a one-sample task (most renders that do not fill the pool) never
+// touches those.
+struct Sums {
+    double4 a, q;
+    double2 w;
+};
+__device__ __forceinline__ Sums zero_sums() {
+    return Sums{make_double4(0.0, 0.0, 0.0, 0.0), make_double4(0.0, 0.0, 0.0, 0.0), make_double2(0.0, 0.0)};
+}
+__device__ __forceinline__ Sums load_sums(const WfState& st, int slot, bool first) {
+    Sums s = zero_sums();
+    if (!first && !st.rsamp) {
+        s.a = lds(&st.sacc[slot]);
+        if (st.ssq) s.q = lds(&st.ssq[slot]);
+        if (st.welford) s.w = st.welford[slot];
     }
-    a.x += (double)L.x; a.y += (double)L.y; a.z += (double)L.z; a.w += 1.0;
-    if (st.ssq) {
-        q.x += (double)L.x * (double)L.x; q.y += (double)L.y * (double)L.y; q.z += (double)L.z * (double)L.z;
-    }
-    if (keep) {
-        sts(&st.sacc[slot], a);
-        if (st.ssq) sts(&st.ssq[slot], q);
+    return s;
+}
+__device__ __forceinline__ void store_sums(const WfState& st, int slot, const Sums& s) {
+    if (st.rsamp) return;
+    sts(&st.sacc[slot], s.a);
+    if (st.ssq) sts(&st.ssq[slot], s.q);
+    if (st.welford) st.welford[slot] = s.w;
+}
+__device__ __forceinline__ void add_sample(Sums& s, float3 L, bool squares) {
+    s.a.x += (double)L.x; s.a.y += (double)L.y; s.a.z += (double)L.z; s.a.w += 1.0;
+    if (squares) {
+        s.q.x += (double)L.x * (double)L.x; s.q.y += (double)L.y * (double)L.y; s.q.z += (double)L.z * (double)L.z;
     }
 }
 
@@ -257,8 +269,9 @@ __device__ __forceinline__ bool camera_miss_next(const WfScene& S0, const WfPara
         sts(&st.rsamp[(size_t)tp.j * P.round_len + (tp.sample_start - P.sample_base) + m.x],
             make_float4(L.x, L.y, L.z, 0.0f));
     } else {
-        double4 a, q;
-        add_sample(st, slot, L, m.x == 0, true, a, q);
+        Sums sums = load_sums(st, slot, m.x == 0);
+        add_sample(sums, L, st.ssq != nullptr);
+        store_sums(st, slot, sums);
     }
     m.x += 1;
     const int pixel = tp.pixel;
@@ -331,7 +344,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace(WfScene S, WfParams P, Wf
         // A window of inactive slots leaves every lane empty but the cursor
         // short of n: the warp keeps fetching until all lanes are exhausted.
         if (!__any_sync(0xffffffffu, item >= 0 || !exhausted)) break;
-        if (item >= 0 && tracer_run<ANY, COUNT>(S, T, stack, kEps, chunk, flags, cnt)) {
+        if (item >= 0 && tracer_run<COUNT>(S, T, stack, kEps, chunk, flags, cnt, ANY)) {
             if (ANY) {
                 reinterpret_cast<float*>(st.sh_c + item)[3] = T.hit_prim >= 0 ? 0.0f : 1.0f;
             } else {
@@ -376,25 +389,23 @@ __device__ __forceinline__ float3 take_pending(const WfState& st, int slot, int&
 // written and the path state reset (returns true); otherwise the task's sums
 // go to the film (one task per pixel) or to the task's partial sums, and
 // need_task is set so the slot takes a new task.
-// finish_sums does all of that but the camera ray; tp is the task's place.
-__device__ __forceinline__ bool finish_sums(const WfParams& P, const WfState& st, int slot, int4& m, float3 L,
-                                            bool& need_task, const Film& F, const TaskPos& tp) {
+// finish_sums does all of that but the camera ray and the slot's records:
+// the sums are the caller's, tp is the task's place.
+__device__ __forceinline__ bool finish_sums(const WfParams& P, const WfState& st, int4& m, float3 L, bool& need_task,
+                                            const Film& F, const TaskPos& tp, Sums& s) {
     const long long task = (long long)m.w;       // batch-wide task id
-    const bool first = m.x == 0;
     m.x += 1;
     const int task_len = tp.len;
     bool stop = m.x >= task_len;
     if (P.adaptive) {  // Welford on luminance (render.rs:160-176)
-        double2 wv = st.welford[slot];
         const double l = 0.2126 * (double)L.x + 0.7152 * (double)L.y + 0.0722 * (double)L.z;
-        const double delta = l - wv.x;
-        wv.x += delta / (double)m.x;
-        wv.y += delta * (l - wv.x);
-        st.welford[slot] = wv;
+        const double delta = l - s.w.x;
+        s.w.x += delta / (double)m.x;
+        s.w.y += delta * (l - s.w.x);
         const int min_spp = min(max(P.adaptive_min_spp, 1), max(task_len, 1));
         if (m.x >= min_spp && m.x > 1) {
-            const double var = wv.y / (double)(m.x - 1);
-            if (sqrt(var) / fmax(fabs(wv.x), 1e-4) < P.adaptive_threshold) stop = true;
+            const double var = s.w.y / (double)(m.x - 1);
+            if (sqrt(var) / fmax(fabs(s.w.x), 1e-4) < P.adaptive_threshold) stop = true;
         }
     }
     need_task = stop;
@@ -403,17 +414,16 @@ __device__ __forceinline__ bool finish_sums(const WfParams& P, const WfState& st
             make_float4(L.x, L.y, L.z, 0.0f));
         return !stop;
     }
-    double4 a, q;
-    add_sample(st, slot, L, first, !stop, a, q);
+    add_sample(s, L, st.acc_sq != nullptr);
     if (stop) {
         if (P.n_chunks == 1) {  // one task per pixel: straight into the film
             const size_t px = (size_t)tp.pixel;
-            F.acc[3 * px] = a.x; F.acc[3 * px + 1] = a.y; F.acc[3 * px + 2] = a.z;
-            F.acc_w[px] = a.w;
-            if (F.acc_sq) { F.acc_sq[3 * px] = q.x; F.acc_sq[3 * px + 1] = q.y; F.acc_sq[3 * px + 2] = q.z; }
+            F.acc[3 * px] = s.a.x; F.acc[3 * px + 1] = s.a.y; F.acc[3 * px + 2] = s.a.z;
+            F.acc_w[px] = s.a.w;
+            if (F.acc_sq) { F.acc_sq[3 * px] = s.q.x; F.acc_sq[3 * px + 1] = s.q.y; F.acc_sq[3 * px + 2] = s.q.z; }
         } else {  // per-task sums, merged in task order by k_merge
-            st.part[task - P.task_first] = a;
-            if (st.part_sq) st.part_sq[task - P.task_first] = q;
+            st.part[task - P.task_first] = s.a;
+            if (st.part_sq) st.part_sq[task - P.task_first] = s.q;
         }
     }
     return !stop;
@@ -423,7 +433,9 @@ __device__ __forceinline__ bool finish_sample(const WfScene& S, const WfParams& 
                                               float& ptime, uint64_t& rng, bool& need_task, const Film& F,
                                               long long base) {
     const TaskPos tp = task_pos(P, (long long)m.w - base);
-    if (!finish_sums(P, st, slot, m, L, need_task, F, tp)) return false;
+    Sums sums = load_sums(st, slot, m.x == 0);
+    if (!finish_sums(P, st, m, L, need_task, F, tp, sums)) return false;
+    store_sums(st, slot, sums);
     float3 o, d;
     const int row = (int)fdiv(P.w_div, (uint32_t)tp.pixel);
     camera_ray(S.cam, tp.pixel - row * P.width, P.row_begin + row * P.row_step, 1.0f / (float)P.width,
@@ -584,67 +596,44 @@ __global__ void __launch_bounds__(128) k_shade_pre(WfScene S, WfParams P, WfStat
 // 9.08, the 1080p frame 147 -> 140.  Stages without the ordering, blocks of
 // 128: 2.46 / 2.50 / 9.63 / 139; blocks of 512: 2.29 / 2.34 / 9.25 / 143.
 constexpr int kShadeBlock = 256;
-// One visit of the shading kernel to a live slot (the per-slot body of
-// k_shade, shared with k_tail): the bounce of radiance() (src/integrator.rs:
-// 67-132) for the slot's closest hit, its NEE shadow records, the sample's
-// completion when nothing is pending, the next camera ray.  Returns what the
-// caller's queues need.
-struct ShadeOut {
-    bool cont, term, finished_here;
-    int sh_env, sh_area;
+// A path between two closest-hit rays, in registers.
+struct PathRegs {
+    float3 o, d;              // the ray traced last; after bounce(): the next one
+    int self_prim, self_inst; // what it starts on
+    float t;                  // what it met
+    int prim, inst;
+    float3 beta, L;
+    float last_pdf, time;
+    int4 m;                   // samples done, bounce, (flags in fl), task
+    int fl;
+    uint64_t rng;
 };
-// STAGED (k_shade): every thread of the block calls it, `active` or not, the
-// block's warps wait for one another between the stages, and a slot whose
-// task is done takes the next task from the pool.  Otherwise (k_tail) a
-// thread calls it alone, and a slot whose task is done is finished.
-template <bool BATCH, bool STAGED>
-__device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams& P0, const WfState& st, int slot,
-                                               bool active) {
+
+// One bounce of radiance() (src/integrator.rs:67-132): what the closest-hit
+// ray met, the NEE samples -- `emit(k, origin, tmax, direction, contribution)`
+// for each shadow ray, 0 = env, 1 = area light -- and the next direction.
+// Returns true when the path ends.  STAGED: every thread of the block calls
+// it, `active` or not, and the block's warps meet between the stages.
+template <bool STAGED, class Emit>
+__device__ __forceinline__ bool bounce(const WfScene& S, const WfParams& P, PathRegs& p, bool active, Emit&& emit) {
     auto stage = [] {
         if constexpr (STAGED) __syncthreads();
     };
-    bool finished_here = false, done = false, surface = false;
-    int sh_env = 0, sh_area = 0;
-    WfScene S = S0;
-    WfParams P = P0;
-    Film F = film_of(st);
-    long long tbase = 0;
-    float3 ro = f3(0, 0, 0), rd = f3(0, 0, 0), beta = f3(0, 0, 0), L = f3(0, 0, 0), hp = f3(0, 0, 0), ng = f3(0, 0, 0);
-    float last_pdf = 0.0f, ptime = 0.0f, t_hit = 0.0f;
-    int prim = -1, inst = -1, fl = 0, mid = 0, kind = 0;
-    int4 m = make_int4(0, 0, 0, 0);
-    uint64_t rng = 0;
-    bool has_env = false;
-    if (active) {
-        if constexpr (BATCH) apply_job(P0.jobs[st.job[slot]], S, P, F, tbase);
-        has_env = S.env_kind == TPT_ENV_MAP;
-        const float4 o4 = lds(&st.ray_o[slot]), d4 = lds(&st.ray_d[slot]);
-        ro = f3(o4);
-        rd = f3(d4);
-        const float4 h4 = lds(&st.hit[slot]);
-        t_hit = h4.x;
-        prim = fbits(h4.y);
-        inst = fbits(h4.z);
-        const float4 b4 = lds(&st.beta[slot]);
-        beta = f3(b4);
-        last_pdf = b4.w;
-        const float4 r4 = lds(&st.rad[slot]);
-        L = f3(r4);
-        ptime = r4.w;
-        load_path(st, slot, m, rng);
-        fl = m.z;
-        L = take_pending(st, slot, fl, L);
-        done = m.y >= P.max_bounces;  // max_bounces = 0: radiance() returns 0
-    }
+    const bool has_env = active && S.env_kind == TPT_ENV_MAP;
+    const float3 rd = p.d;
+    const int prim = p.prim, inst = p.inst;
+    float3 hp = f3(0, 0, 0), ng = f3(0, 0, 0);
+    int mid = 0, kind = 0;
+    bool done = active && p.m.y >= P.max_bounces, surface = false;  // max_bounces = 0: radiance() returns 0
     const bool miss = active && !done && prim < 0;
     if (active && !done && !miss) {
-        if (m.y >= P.rr_start) {  // Russian roulette (:89-95)
-            const float p = fmaxf(fminf(max3(beta), 0.95f), 0.05f);
-            if (pcg_f32(rng) > p) done = true;
-            else beta = beta / p;
+        if (p.m.y >= P.rr_start) {  // Russian roulette (:89-95)
+            const float q = fmaxf(fminf(max3(p.beta), 0.95f), 0.05f);
+            if (pcg_f32(p.rng) > q) done = true;
+            else p.beta = p.beta / q;
         }
         if (!done) {
-            hp = ro + rd * t_hit;
+            hp = p.o + rd * p.t;
             if (inst < 0) {
                 const SphereF32 sp = S.spheres[prim];
                 ng = (hp - f3(sp.cr)) / sp.cr.w;
@@ -662,7 +651,7 @@ __device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams
             }
             kind = S.mats[mid].kind;
             if (kind == TPT_MAT_DIFFUSE_LIGHT) {  // emitter (:100-104)
-                L = L + clamp_lum(beta * f3(S.mats[mid].c), 50.0f);
+                p.L = p.L + clamp_lum(p.beta * f3(S.mats[mid].c), 50.0f);
                 done = true;
             } else {
                 surface = true;
@@ -677,8 +666,8 @@ __device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams
     // the env map in the ray's direction (a miss) or the NEE sample's
     float3 wi = rd, li = f3(0, 0, 0);
     float pe = 1.0f / (4.0f * kPi);
-    bool want_pdf = (fl & F_LAST_ND) != 0;
-    if (nee && has_env) want_pdf = env_sample_to(S, rng, wi);
+    bool want_pdf = (p.fl & F_LAST_ND) != 0;
+    if (nee && has_env) want_pdf = env_sample_to(S, p.rng, wi);
     stage();
     if (has_env && (miss || nee)) {
         float pdf = pe;
@@ -688,9 +677,9 @@ __device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams
     stage();
     if (miss) {  // (:71-83)
         if (!has_env) li = sky(rd);
-        float3 contrib = beta * li;
-        if (has_env && (fl & F_LAST_ND)) contrib = contrib * mis(last_pdf, pe);
-        L = L + clamp_lum(contrib, 50.0f);
+        float3 contrib = p.beta * li;
+        if (has_env && (p.fl & F_LAST_ND)) contrib = contrib * mis(p.last_pdf, pe);
+        p.L = p.L + clamp_lum(contrib, 50.0f);
         done = true;
     }
     if (nee && has_env) {  // nee_environment (:148-172)
@@ -699,15 +688,8 @@ __device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams
             float3 f;
             float pb;
             mat_eval(S.mats[mid], wo, wi, n, f, pb);
-            const float3 contrib = beta * f * li * (c * mis(pe, pb) / pe);
-            if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) {
-                const float3 so = hp + wi * kEps;
-                sts(&st.sh_o[2 * slot], make_float4(so.x, so.y, so.z, kTMax));
-                sts(&st.sh_d[2 * slot], make_float4(wi.x, wi.y, wi.z, ifloat(prim)));
-                sts(&st.sh_c[2 * slot], make_float4(contrib.x, contrib.y, contrib.z, ifloat(inst)));
-                sh_env = 1;
-                fl |= F_PEND_ENV;
-            }
+            const float3 contrib = p.beta * f * li * (c * mis(pe, pb) / pe);
+            if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) emit(0, hp + wi * kEps, kTMax, wi, contrib);
         }
     }
     stage();
@@ -716,27 +698,22 @@ __device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams
         float lpdf;
         int lidx;
         double lud, lvd;
-        if (sample_light(S, rng, hp, lp, le, lpdf, lidx, lud, lvd)) {  // nee_area_light (:178-213)
+        if (sample_light(S, p.rng, hp, lp, le, lpdf, lidx, lud, lvd)) {  // nee_area_light (:178-213)
             const float3 tl = lp - hp;
             const float dist = length(tl);
             if (dist > 1e-6f) {
                 const float3 wl = tl / dist;
                 const float c = fmaxf(dot(n, wl), 0.0f);
-                if (c > 0.0f && !ref_light_self_occluded(S.lights64, S.spheres64, S.inst64, lidx, ro, rd, t_hit, lud, lvd, (double)ptime)) {
+                if (c > 0.0f && !ref_light_self_occluded(S.lights64, S.spheres64, S.inst64, lidx, p.o, rd, p.t, lud, lvd,
+                                                         (double)p.time)) {
                     float3 f;
                     float pb;
                     mat_eval(S.mats[mid], wo, wl, n, f, pb);
-                    const float3 contrib = beta * f * le * (c * mis(lpdf, pb) / lpdf);
-                    if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f) {
-                        const float3 so = hp + wl * kEps;
-                        // stops 1e-4 short of the light: the light itself is
-                        // handled by ref_light_self_occluded
-                        sts(&st.sh_o[2 * slot + 1], make_float4(so.x, so.y, so.z, fmaxf(dist - 2.0f * kEps, kEps)));
-                        sts(&st.sh_d[2 * slot + 1], make_float4(wl.x, wl.y, wl.z, ifloat(prim)));
-                        sts(&st.sh_c[2 * slot + 1], make_float4(contrib.x, contrib.y, contrib.z, ifloat(inst)));
-                        sh_area = 1;
-                        fl |= F_PEND_AREA;
-                    }
+                    const float3 contrib = p.beta * f * le * (c * mis(lpdf, pb) / lpdf);
+                    // stops 1e-4 short of the light: the light itself is
+                    // handled by ref_light_self_occluded
+                    if (contrib.x > 0.0f || contrib.y > 0.0f || contrib.z > 0.0f)
+                        emit(1, hp + wl * kEps, fmaxf(dist - 2.0f * kEps, kEps), wl, contrib);
                 }
             }
         }
@@ -755,13 +732,13 @@ __device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams
                 w = mc;
                 if (sub) {
                     const float sc = fmaxf(mt.c.w, 1e-4f);
-                    const float u = fmaxf(pcg_f32(rng), 1e-12f);
+                    const float u = fmaxf(pcg_f32(p.rng), 1e-12f);
                     const float dist = -__logf(u) * sc;
                     w = mc * __expf(-dist / sc);
                     no = hp - ng * dist;
                     self_ok = false;     // origin moved off the surface
                 }
-                nd = cos_hemi(sub ? ng : n, rng);  // subsurface: unoriented normal (material.rs:187-188)
+                nd = cos_hemi(sub ? ng : n, p.rng);  // subsurface: unoriented normal (material.rs:187-188)
                 pdf = fmaxf(dot(n, nd), 0.0f) / kPi;
                 break;
             }
@@ -779,13 +756,13 @@ __device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams
                 const float fr = f0 + (1.0f - f0) * pow5(1.0f - ci);
                 float3 bt = f3(1, 1, 1);
                 if (!entering) {
-                    const float dist = fmaxf(t_hit, 0.0f);
+                    const float dist = fmaxf(p.t, 0.0f);
                     bt = f3(__expf(-mc.x * dist), __expf(-mc.y * dist), __expf(-mc.z * dist));
                 }
                 const float cosi = fminf(fmaxf(dot(wo, n), -1.0f), 1.0f);
                 const float sin2t = eta * eta * (1.0f - cosi * cosi);
                 const bool has_refr = !(sin2t >= 1.0f);
-                const bool refl = !has_refr || pcg_f32(rng) < fr;
+                const bool refl = !has_refr || pcg_f32(p.rng) < fr;
                 if (refl) {
                     nd = rd - n * (2.0f * dot(rd, n));
                     bt = bt * (fr / fmaxf(fr, 1e-6f));
@@ -799,7 +776,7 @@ __device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams
             }
             case TPT_MAT_GGX: {
                 GgxSample gs;
-                if (!ggx_sample(rd, n, mt, rng, gs)) { ok = false; break; }
+                if (!ggx_sample(rd, n, mt, p.rng, gs)) { ok = false; break; }
                 nd = gs.nd;
                 w = gs.w;
                 pdf = gs.pdf;
@@ -811,63 +788,55 @@ __device__ __forceinline__ ShadeOut shade_slot(const WfScene& S0, const WfParams
         if (!ok) {
             done = true;
         } else {
-            beta = beta * w;
-            last_pdf = pdf;
-            fl = delta ? (fl & ~F_LAST_ND) : (fl | F_LAST_ND);
-            const float3 o2 = no + nd * kEps;
-            sts(&st.ray_o[slot], make_float4(o2.x, o2.y, o2.z, ifloat(self_ok ? prim : -1)));
-            sts(&st.ray_d[slot], make_float4(nd.x, nd.y, nd.z, ifloat(self_ok ? inst : -1)));
-            m.y += 1;
-            if (m.y >= P.max_bounces) done = true;  // bounce loop bound (:67)
+            p.beta = p.beta * w;
+            p.last_pdf = pdf;
+            p.fl = delta ? (p.fl & ~F_LAST_ND) : (p.fl | F_LAST_ND);
+            p.o = no + nd * kEps;
+            p.d = nd;
+            p.self_prim = self_ok ? prim : -1;
+            p.self_inst = self_ok ? inst : -1;
+            p.m.y += 1;
+            if (p.m.y >= P.max_bounces) done = true;  // bounce loop bound (:67)
         }
     }
     stage();
-    bool cont = active && !done, need_task = false, camera = false;
-    const bool term = active && done && (sh_env || sh_area);
-    TaskPos tp{};
-    if (active && done && !term) {
-        // Nothing pending: finish the sample here instead of in k_regen.
-        tp = task_pos(P, (long long)m.w - tbase);
-        camera = finish_sums(P, st, slot, m, L, need_task, F, tp);
-        finished_here = true;
-    }
-    if constexpr (STAGED) {
-        const long long task = next_task(P0, st, need_task);
-        if (task >= 0) {
-            if constexpr (BATCH) {
-                const int j = find_job(P0, task);
-                st.job[slot] = j;
-                apply_job(P0.jobs[j], S, P, F, tbase);
-            }
-            tp = task_pos(P, task - tbase);
-            m = make_int4(0, 0, 0, (int)task);
-            if (st.welford) st.welford[slot] = make_double2(0.0, 0.0);
-            camera = true;
-            need_task = false;
-        }
-    }
-    if (camera) {
-        const int row = (int)fdiv(P.w_div, (uint32_t)tp.pixel);
-        const int x = tp.pixel - row * P.width, y = P.row_begin + row * P.row_step;
-        if (m.x == 0) rng = task_seed((uint32_t)x, (uint32_t)y, (uint32_t)tp.sample_start, P.seed);  // a new task
-        float3 o, d;
-        camera_ray(S.cam, x, y, 1.0f / (float)P.width, 1.0f / (float)P.height, rng, o, d, ptime);
-        sts(&st.ray_o[slot], make_float4(o.x, o.y, o.z, ifloat(-1)));
-        sts(&st.ray_d[slot], make_float4(d.x, d.y, d.z, ifloat(-1)));
-        beta = f3(1.0f, 1.0f, 1.0f);
-        last_pdf = 0.0f;
-        L = f3(0, 0, 0);
-        m.y = 0;
-        fl = 0;
-        cont = true;
-    }
-    if (active && !need_task) {
-        sts(&st.beta[slot], make_float4(beta.x, beta.y, beta.z, last_pdf));
-        sts(&st.rad[slot], make_float4(L.x, L.y, L.z, ptime));
-        m.z = fl;
-        store_path(st, slot, m, rng);
-    }
-    return ShadeOut{cont, term, finished_here, sh_env, sh_area};
+    return done;
+}
+
+// The camera ray of sample m.x of the task at tp (src/render.rs:151-158) and
+// the path state it starts with; the first sample seeds the task's stream.
+__device__ __forceinline__ void start_sample(const WfScene& S, const WfParams& P, const TaskPos& tp, PathRegs& p) {
+    const int row = (int)fdiv(P.w_div, (uint32_t)tp.pixel);
+    const int x = tp.pixel - row * P.width, y = P.row_begin + row * P.row_step;
+    if (p.m.x == 0) p.rng = task_seed((uint32_t)x, (uint32_t)y, (uint32_t)tp.sample_start, P.seed);
+    camera_ray(S.cam, x, y, 1.0f / (float)P.width, 1.0f / (float)P.height, p.rng, p.o, p.d, p.time);
+    p.self_prim = p.self_inst = -1;
+    p.beta = f3(1.0f, 1.0f, 1.0f);
+    p.L = f3(0.0f, 0.0f, 0.0f);
+    p.last_pdf = 0.0f;
+    p.m.y = 0;
+    p.fl = 0;
+}
+
+// A slot's path as the last iteration left it, its pending shadow rays'
+// results included.
+__device__ __forceinline__ PathRegs load_slot(const WfState& st, int slot) {
+    PathRegs p;
+    const float4 o4 = lds(&st.ray_o[slot]), d4 = lds(&st.ray_d[slot]);
+    p.o = f3(o4);
+    p.d = f3(d4);
+    p.self_prim = fbits(o4.w);
+    p.self_inst = fbits(d4.w);
+    const float4 b4 = lds(&st.beta[slot]), r4 = lds(&st.rad[slot]);
+    p.beta = f3(b4);
+    p.last_pdf = b4.w;
+    p.time = r4.w;
+    load_path(st, slot, p.m, p.rng);
+    p.fl = p.m.z;
+    p.L = take_pending(st, slot, p.fl, f3(r4));
+    p.t = kTMax;
+    p.prim = p.inst = -1;
+    return p;
 }
 
 // What the shading stages do with a live slot: 0 = its ray left the scene, 1 +
@@ -943,13 +912,68 @@ __global__ void __launch_bounds__(kShadeBlock, CTAS * 128 / kShadeBlock) k_shade
             fetch(st.ray_o + next); fetch(st.ray_d + next); fetch(st.hit + next);
             fetch(st.beta + next); fetch(st.rad + next); fetch(st.path + next);
         }
-        const ShadeOut r = shade_slot<BATCH, true>(S0, P0, st, slot, active);
-        if (active) st.act[slot] = r.cont ? 1 : 0;
-        if (!P0.ordered_queue) warp_push(st.q_ext[nxt], &st.ctr->n_ext[nxt], r.cont, slot);
-        warp_push(st.q_term, &st.ctr->n_term, r.term, slot);
-        warp_count(&st.ctr->n_done_in_shade, r.finished_here);
-        warp_push(st.q_sh, &st.ctr->n_sh, r.sh_env != 0, 2 * slot);
-        warp_push(st.q_sh, &st.ctr->n_sh, r.sh_area != 0, 2 * slot + 1);
+        WfScene S = S0;
+        WfParams P = P0;
+        Film F = film_of(st);
+        long long tbase = 0;
+        PathRegs p{};
+        if (active) {
+            if constexpr (BATCH) apply_job(P0.jobs[st.job[slot]], S, P, F, tbase);
+            p = load_slot(st, slot);
+            const float4 h4 = lds(&st.hit[slot]);
+            p.t = h4.x;
+            p.prim = fbits(h4.y);
+            p.inst = fbits(h4.z);
+        }
+        int sh[2] = {0, 0};
+        const int prim = p.prim, inst = p.inst;
+        const bool done = bounce<true>(S, P, p, active, [&](int k, float3 so, float tmax, float3 wi, float3 contrib) {
+            sts(&st.sh_o[2 * slot + k], make_float4(so.x, so.y, so.z, tmax));
+            sts(&st.sh_d[2 * slot + k], make_float4(wi.x, wi.y, wi.z, ifloat(prim)));
+            sts(&st.sh_c[2 * slot + k], make_float4(contrib.x, contrib.y, contrib.z, ifloat(inst)));
+            sh[k] = 1;
+        });
+        if (active) p.fl |= (sh[0] ? F_PEND_ENV : 0) | (sh[1] ? F_PEND_AREA : 0);
+        bool cont = active && !done, need_task = false, camera = false;
+        const bool term = active && done && (sh[0] || sh[1]), finished = active && done && !term;
+        TaskPos tp{};
+        if (finished) {  // nothing pending: the sample ends here instead of in k_regen
+            tp = task_pos(P, (long long)p.m.w - tbase);
+            Sums sums = load_sums(st, slot, p.m.x == 0);
+            camera = finish_sums(P, st, p.m, p.L, need_task, F, tp, sums);
+            if (camera) store_sums(st, slot, sums);
+        }
+        const long long task = next_task(P0, st, need_task);
+        if (task >= 0) {
+            if constexpr (BATCH) {
+                const int j = find_job(P0, task);
+                st.job[slot] = j;
+                apply_job(P0.jobs[j], S, P, F, tbase);
+            }
+            tp = task_pos(P, task - tbase);
+            p.m = make_int4(0, 0, 0, (int)task);
+            camera = true;
+        }
+        if (camera) {
+            start_sample(S, P, tp, p);
+            cont = true;
+        }
+        if (cont || term) {
+            if (cont) {
+                sts(&st.ray_o[slot], make_float4(p.o.x, p.o.y, p.o.z, ifloat(p.self_prim)));
+                sts(&st.ray_d[slot], make_float4(p.d.x, p.d.y, p.d.z, ifloat(p.self_inst)));
+                sts(&st.beta[slot], make_float4(p.beta.x, p.beta.y, p.beta.z, p.last_pdf));
+            }
+            sts(&st.rad[slot], make_float4(p.L.x, p.L.y, p.L.z, p.time));
+            p.m.z = p.fl;
+            store_path(st, slot, p.m, p.rng);
+        }
+        if (active) st.act[slot] = cont ? 1 : 0;
+        if (!P0.ordered_queue) warp_push(st.q_ext[nxt], &st.ctr->n_ext[nxt], cont, slot);
+        warp_push(st.q_term, &st.ctr->n_term, term, slot);
+        warp_count(&st.ctr->n_done_in_shade, finished);
+        warp_push(st.q_sh, &st.ctr->n_sh, sh[0] != 0, 2 * slot);
+        warp_push(st.q_sh, &st.ctr->n_sh, sh[1] != 0, 2 * slot + 1);
     }
 }
 
@@ -1143,7 +1167,7 @@ __global__ void __launch_bounds__(128) k_shade_surface(WfScene S, WfParams P, Wf
 
 // Samples that ended with shadow rays pending finish here, after k_shadow
 // has resolved their visibility.
-// The completion kernel's per-slot body (k_regen, shared with k_tail): a
+// The completion kernel's per-slot body (k_regen): a
 // path that ended with shadow rays pending takes their results, then
 // finish_sample.  Returns whether the slot traces on (the task's next
 // camera ray); need_task when its task is done.
@@ -1477,72 +1501,169 @@ __global__ void k_sky_tasks(WfScene S0, WfParams P0, WfState st, const int* __re
     if (lane_id() == 0 && done) atomicAdd(&st.ctr->sky_samples, done);  // beside k_step: its own counter
 }
 
-// The end of a render's bounce loop: when every task has been taken and at
-// most P.tail_live slots are still live, the loop stops and this kernel
-// runs each live slot (the queue the last iteration left, q_ext[0]) to the
-// end of its task, one thread per slot: closest hit, shade_slot, the shadow
-// rays at once, regen_slot when the path ended with shadow rays pending,
-// and on to the task's next sample.  These are the wavefront kernels'
-// per-slot steps in their order, so the film is that of the loop run to
-// the end; the drain's per-iteration launches and compactions go away.
-// Each slot is bounded by P.max_iters visits (TPT_FLAG_ITER_LIMIT).
-template <bool BATCH>
-__global__ void __launch_bounds__(128) k_tail(WfScene S, WfParams P, WfState st) {
-    const int n = st.ctr->n_ext[0];
-    const int* __restrict__ q = st.q_ext[0];
+// Whole paths in one kernel: every lane carries a path in registers from its
+// first camera ray to the end of its task, then takes the next one.  A round
+// of the block is: the bounce of the closest hits, in step (bounce<true>),
+// finished samples and new ones, then the rays -- the bounce's shadow rays
+// and the next closest-hit ray -- until no lane of the warp waits.  The steps
+// and their order are the wavefront kernels', so the film is the same.
+//
+// TASKS: small renders, from the pool's tasks, instead of the bounce loop and
+// its launches (wf_render decides).  `open`, when given, flags the film's
+// pixels (all jobs') whose camera rays leave the scene: their samples are
+// not traced (camera culling, counted in sky_samples).  Otherwise the end of
+// a bounce loop, once every task has been taken: the live slots of the queue
+// the last iteration left, q_ext[0].
+//
+// `lanes` lanes of each warp take work.  A task whose path outlives
+// P.max_iters rounds is dropped (TPT_FLAG_ITER_LIMIT).
+//
+// Bound by the latency of each path's chain of rays at these sizes, and by
+// instruction fetch (the block's warps share it, as in k_shade).  3 blocks per
+// SM: 2 trace larger renders 20% slower, 4 spill 330 B (allocation-free 96x96 x
+// 16 spp 0.80 ms at 3, 0.92 at 4).  As the end of a loop it replaces a kernel
+// of one thread per slot that kept the path in memory: batch of 10 scenes 36.4
+// -> 33.1 ms, adaptive Cornell film 480x270 23.1 -> 22.2 ms.
+constexpr int kPathsBlock = 128;
+template <bool BATCH, bool TASKS, bool SHARED_STACK>
+__global__ void __launch_bounds__(kPathsBlock, 3) k_paths(WfScene S0, WfParams P0, WfState st,
+                                                      const uint8_t* __restrict__ open, unsigned lanes) {
+    __shared__ int sstack[SHARED_STACK ? kSharedStack * kPathsBlock : 1];
+    int lstack[SHARED_STACK ? 1 : kStack];
+    using Stack = typename std::conditional<SHARED_STACK, TStack<kPathsBlock, kSharedStack>, TStack<1, kStack>>::type;
+    const Stack stack{SHARED_STACK ? sstack + threadIdx.x : lstack};
     int* flags = &st.ctr->flags;
-    int lstack[kStack];
-    const TStack<1, kStack> stack{lstack};
-    unsigned long long samples = 0, rays_c = 0, rays_s = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int slot = q[i];
-        const int root = BATCH ? P.jobs[st.job[slot]].top_root : S.top_root;
-        for (long long visit = 0;; ++visit) {
-            if (visit >= P.max_iters) {
-                raise_flag(flags, TPT_FLAG_ITER_LIMIT);
-                break;
-            }
-            Tracer T;
-            TraceCount cnt;
-            const float4 o4 = lds(&st.ray_o[slot]), d4 = lds(&st.ray_d[slot]);
-            tracer_start_at(root, T, f3(o4), f3(d4), kTMax, fbits(o4.w), fbits(d4.w));
-            while (!tracer_run<false, false>(S, T, stack, kEps, 1 << 30, flags, cnt)) {
-            }
-            sts(&st.hit[slot], make_float4(T.hit_prim >= 0 ? T.tmax : kTMax, ifloat(T.hit_prim), ifloat(T.hit_inst),
-                                           0.0f));
-            ++rays_c;
-            const ShadeOut r = shade_slot<BATCH, false>(S, P, st, slot, true);
-            if (r.finished_here) ++samples;
-            for (int k = 0; k < 2; ++k) {
-                if (!(k == 0 ? r.sh_env : r.sh_area)) continue;
-                const int rec = 2 * slot + k;
-                const float4 so = lds(&st.sh_o[rec]), sd = lds(&st.sh_d[rec]);
-                float* vis = reinterpret_cast<float*>(st.sh_c + rec) + 3;
-                tracer_start_at(root, T, f3(so), f3(sd), so.w, fbits(sd.w), fbits(*vis));
-                while (!tracer_run<true, false>(S, T, stack, kEps, 1 << 30, flags, cnt)) {
-                }
-                *vis = T.hit_prim >= 0 ? 0.0f : 1.0f;
-                ++rays_s;
-            }
-            bool cont = r.cont;
-            if (r.term) {
-                bool need_task = false;
-                cont = regen_slot<BATCH>(S, P, st, slot, need_task);
-                ++samples;
-            }
-            if (!cont) break;  // its task is done, and no task is left to take
+    const long long n_items = TASKS ? fetch_end(P0) - P0.task_first : st.ctr->n_ext[0];
+    unsigned long long samples = 0, rays_c = 0, rays_s = 0, sky_samples = 0;
+    constexpr int kEnv = 1, kArea = 2, kClosest = 4;
+    PathRegs p{};
+    Sums sums = zero_sums();
+    float3 sh_o[2] = {}, sh_d[2] = {}, sh_c[2] = {};
+    float sh_t = 0.0f;
+    int sh_prim = -1, sh_inst = -1;
+    int job = 0, jobs = 0;
+    long long visits = 0;
+    bool alive = false, ended = false, sky_task = false, exhausted = lane_id() >= lanes;
+    for (;;) {
+        WfScene S = S0;
+        WfParams P = P0;
+        Film F = film_of(st);
+        long long tbase = 0;
+        // (A lane without a task takes its last job's view, or job 0's: with
+        // the overlay under a condition nvcc 12.9 left P.width at P0's 0.)
+        if constexpr (BATCH) apply_job(P0.jobs[job], S, P, F, tbase);
+        const bool shade = alive && !ended;
+        if (shade) {
+            sh_prim = p.prim;
+            sh_inst = p.inst;
         }
-        st.act[slot] = 0;
+        const bool done = bounce<true>(S, P, p, shade, [&](int k, float3 so, float tmax, float3 wi, float3 contrib) {
+            if (k == 0) { sh_o[0] = so; sh_d[0] = wi; sh_c[0] = contrib; }
+            else { sh_o[1] = so; sh_d[1] = wi; sh_c[1] = contrib; sh_t = tmax; }
+            jobs |= k == 0 ? kEnv : kArea;
+        });
+        if (shade) {
+            if (done) ended = true;
+            else jobs |= kClosest;
+            if (++visits >= P0.max_iters) {
+                raise_flag(flags, TPT_FLAG_ITER_LIMIT);
+                alive = false;
+                jobs = 0;
+            }
+        }
+        bool camera = false;
+        TaskPos tp{};
+        if (alive && ended && jobs == 0) {  // the sample is complete
+            tp = task_pos(P, (long long)p.m.w - tbase);
+            bool task_done = false;
+            camera = finish_sums(P, st, p.m, p.L, task_done, F, tp, sums);
+            if (sky_task) ++sky_samples;
+            else ++samples;
+            alive = !task_done;
+        }
+        const bool want = !alive && !exhausted;
+        const unsigned wm = __ballot_sync(0xffffffffu, want);
+        if (wm) {
+            const int leader = __ffs(wm) - 1;
+            long long base = 0;
+            if ((int)lane_id() == leader)
+                base = (long long)atomicAdd((unsigned long long*)&st.ctr->next_item, (unsigned long long)__popc(wm));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (want) {
+                const long long k = base + __popc(wm & ((1u << lane_id()) - 1u));
+                exhausted = k >= n_items;
+                if (!exhausted) {
+                    alive = true;
+                    visits = 0;
+                    if constexpr (TASKS) {
+                        const long long task = task_of_fetch(P0, P0.task_first + k);
+                        long long pixel0 = 0;
+                        if constexpr (BATCH) {
+                            job = find_job(P0, task);
+                            apply_job(P0.jobs[job], S, P, F, tbase);
+                            pixel0 = P0.jobs[job].pixel_begin;
+                        }
+                        tp = task_pos(P, task - tbase);
+                        p.m = make_int4(0, 0, 0, (int)task);
+                        sums = zero_sums();
+                        sky_task = open && open[pixel0 + tp.pixel];
+                        camera = true;
+                    } else {
+                        const int slot = st.q_ext[0][k];
+                        if constexpr (BATCH) job = st.job[slot];
+                        p = load_slot(st, slot);
+                        sums = load_sums(st, slot, p.m.x == 0);
+                        ended = false;
+                        jobs = kClosest;
+                    }
+                }
+            }
+        }
+        if (camera) {
+            start_sample(S, P, tp, p);
+            p.t = kTMax;
+            p.prim = p.inst = -1;
+            ended = false;
+            if (!sky_task) jobs = kClosest;
+        }
+        if (!__syncthreads_or(alive || !exhausted)) break;
+        while (__any_sync(0xffffffffu, jobs != 0)) {
+            if (jobs != 0) {
+                const int j = jobs & -jobs;
+                const bool any = j != kClosest;
+                int root = S0.top_root;
+                if constexpr (BATCH) root = __ldg(&P0.jobs[job].top_root);
+                Tracer T;
+                TraceCount cnt;
+                tracer_start_at(root, T, j == kEnv ? sh_o[0] : (j == kArea ? sh_o[1] : p.o),
+                                j == kEnv ? sh_d[0] : (j == kArea ? sh_d[1] : p.d), j == kArea ? sh_t : kTMax,
+                                any ? sh_prim : p.self_prim, any ? sh_inst : p.self_inst);
+                while (!tracer_run<false>(S0, T, stack, kEps, 1 << 30, flags, cnt, any)) {
+                }
+                if (any) {
+                    ++rays_s;
+                    if (T.hit_prim < 0) p.L = p.L + (j == kEnv ? sh_c[0] : sh_c[1]);
+                } else {
+                    ++rays_c;
+                    p.t = T.hit_prim >= 0 ? T.tmax : kTMax;
+                    p.prim = T.hit_prim;
+                    p.inst = T.hit_inst;
+                }
+                jobs ^= j;
+            }
+        }
     }
     for (int off = 16; off > 0; off >>= 1) {
         samples += __shfl_down_sync(0xffffffffu, samples, off);
         rays_c += __shfl_down_sync(0xffffffffu, rays_c, off);
         rays_s += __shfl_down_sync(0xffffffffu, rays_s, off);
+        sky_samples += __shfl_down_sync(0xffffffffu, sky_samples, off);
     }
     if (lane_id() == 0) {
         if (samples) atomicAdd(&st.ctr->samples, samples);
         if (rays_c) atomicAdd(&st.ctr->rays_closest, rays_c);
         if (rays_s) atomicAdd(&st.ctr->rays_shadow, rays_s);
+        if (sky_samples) atomicAdd(&st.ctr->sky_samples, sky_samples);
     }
 }
 
@@ -1807,7 +1928,7 @@ __global__ void k_step(WfState st, int cur, long long max_iters, cudaGraphCondit
     c->iters += 1;
     bool more = c->n_ext[cur ^ 1] > 0;
     if (more && tail_live > 0 && c->n_ext[cur ^ 1] <= tail_live && c->next_task >= fetch_end) {
-        c->tail = 1;  // the pool's tasks are all taken: k_tail finishes the few live slots
+        c->tail = 1;  // the pool's tasks are all taken: k_paths finishes the few live slots
         more = false;
     }
     if (more && c->iters >= max_iters) {
@@ -2071,6 +2192,34 @@ Grids pick_grids(int sm_count) {
     return g;
 }
 
+// k_paths over n_items tasks (TASKS) or live slots: one wave of blocks.
+// Fewer items than lanes spread over the warps, so that a warp diverges less.
+template <bool TASKS, bool BATCH, bool SHARED>
+void launch_paths_as(const WfScene& S, const WfParams& P, const WfState& st, const uint8_t* open, long long n_items,
+                     int sm_count, cudaStream_t s) {
+    auto kern = wf::k_paths<BATCH, TASKS, SHARED>;
+    int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, wf::kPathsBlock, 0);
+    const long long blocks = (long long)sm_count * std::max(occ, 1), warps = blocks * (wf::kPathsBlock / 32);
+    const unsigned lanes = (unsigned)std::min<long long>(32, std::max<long long>(1, (n_items + warps - 1) / warps));
+    const long long per_block = (long long)lanes * (wf::kPathsBlock / 32);
+    const unsigned grid = (unsigned)std::max<long long>(1, std::min(blocks, (n_items + per_block - 1) / per_block));
+    kern<<<grid, wf::kPathsBlock, 0, s>>>(S, P, st, open, lanes);
+}
+template <bool TASKS>
+void launch_paths(const WfScene& S, const WfParams& P, const WfState& st, const uint8_t* open, long long n_items,
+                  int sm_count, cudaStream_t s) {
+    const bool shared = S.max_stack <= wf::kSharedStack;
+    if (P.jobs) {
+        if (shared) launch_paths_as<TASKS, true, true>(S, P, st, open, n_items, sm_count, s);
+        else launch_paths_as<TASKS, true, false>(S, P, st, open, n_items, sm_count, s);
+    } else if (shared) {
+        launch_paths_as<TASKS, false, true>(S, P, st, open, n_items, sm_count, s);
+    } else {
+        launch_paths_as<TASKS, false, false>(S, P, st, open, n_items, sm_count, s);
+    }
+}
+
 // The pool's end of fetch ids (fetch_end on the device).
 long long host_fetch_end(const WfParams& P) {
     if (!P.geo_map) return P.n_tasks;
@@ -2166,7 +2315,7 @@ cudaError_t run_host_loop(const WfEnqueue& enqueue, const WfCounters* ctr, long 
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) break;
         if (probe.n_ext[0] == 0 && probe.n_ext[1] == 0) break;
-        if (probe.tail) break;  // k_tail finishes the live slots
+        if (probe.tail) break;  // k_paths finishes the live slots
         if ((probe.flags & TPT_FLAG_ITER_LIMIT) || launched > max_iters + 16) break;
     }
     return e;
@@ -2291,6 +2440,85 @@ cudaError_t reserve_pool(WfBuffers& B, WfParams& P, size_t part_tasks) {
 }
 }  // namespace
 
+namespace {
+// Whether a render of P.n_tasks tasks of up to P.task_spp samples runs in
+// k_paths alone.  Its divergent lanes trace 2 to 4 times slower than the
+// loop's kernels at full size, but the loop pays 0.7 to 1.3 ms for its graph
+// and some 25 launches, and once more per sample of a task.  Measured on one
+// B200, loop / direct, ms: 64x36 preview 0.70 / 0.09; 1-sample tasks, sphere
+// scene and mesh scene of 81,920 triangles: 36,864 tasks 0.81 / 0.16 and 1.46
+// / 0.38, 524,288 0.96 / 0.41 and 1.74 / 0.89, 2,097,152 1.48 / 1.23 and 2.35 /
+// 2.66, 4,194,304 2.11 / 2.23 and 2.94 / 4.57; 8-sample tasks: 1 Mi samples
+// 2.6 / 0.9 and 6.5 / 2.6, 4.7 M 3.7 / 2.8 and 7.8 / 6.6, 8.4 M 5.0 / 4.5 and
+// 9.0 / 10.3; batches of 64 scenes 2.1 M samples 7.5 / 5.8, 4.3 M 9.4 / 9.6.  So
+// the line lies at 1.2 M samples of 1-sample tasks and 3.9 M of 8-sample ones.
+// A caller that sets the drain's handover (TPT_TAIL_SLOTS) asks for the loop.
+bool direct_render(const WfParams& P) {
+    return P.tail_live < 0 && P.n_tasks * std::max(P.task_spp, 1) <= (P.task_spp + 2) * 393216LL;
+}
+
+// A render whose tasks all go to k_paths: no path state, no loop.  With camera
+// culling on, one thread per pixel classifies the film first (k_paths reads
+// the flags; nothing is compacted or read back).
+cudaError_t render_direct(const WfScene& S, const WfParams& P, WfBuffers& B, double* acc, double* acc_w, double* acc_sq,
+                          size_t part_tasks, cudaStream_t stream, int sm_count, WfCounters* hc, float* ms) {
+    cudaError_t e = wf_reserve(B, std::max<size_t>(B.slots, 1), std::max(B.part_tasks, part_tasks));
+    if (e == cudaErrorMemoryAllocation) {  // no room beside the slots of an earlier render
+        cudaGetLastError();
+        e = wf_reserve(B, 1, part_tasks);
+    }
+    if (e != cudaSuccess) return e;
+    WfState st = B.st;
+    st.acc = acc;
+    st.acc_w = acc_w;
+    st.acc_sq = acc_sq;
+    st.welford = nullptr;
+    st.ssq = nullptr;
+    if (!acc_sq) st.part_sq = nullptr;
+    Events total;
+    cudaEventRecord(total.e0, stream);
+    e = cudaMemsetAsync(st.ctr, 0, sizeof(WfCounters), stream);
+    long long launches = 1;
+    const uint8_t* open = nullptr;
+    const long long pixels = P.jobs ? P.total_pixels : (long long)P.n_pixels;
+    const bool pinhole = P.jobs || (P.max_bounces > 0 && S.cam.lens_radius == 0.0f && S.cam.focus_dist > 0.0f);
+    if (e == cudaSuccess && P.sky_cull && !P.adaptive && pinhole && pixels < (1ll << 31)) {
+        e = cull_reserve(B, (size_t)pixels);
+        const unsigned grid = (unsigned)((pixels + 255) / 256);
+        if (e == cudaSuccess) {
+            if (P.jobs) wf::k_cull_classify<true><<<grid, 256, 0, stream>>>(S, P, B.cull_flag[0], B.cull_flag[1]);
+            else wf::k_cull_classify<false><<<grid, 256, 0, stream>>>(S, P, B.cull_flag[0], B.cull_flag[1]);
+            open = B.cull_flag[1];
+            ++launches;
+        }
+    }
+    if (e == cudaSuccess) {
+        launch_paths<true>(S, P, st, open, P.n_tasks, sm_count, stream);
+        if (P.n_chunks > 1) {
+            if (P.jobs) wf::k_merge_batch<<<(unsigned)((pixels + 255) / 256), 256, 0, stream>>>(P, st);
+            else wf::k_merge<<<(P.n_pixels + 255) / 256, 256, 0, stream>>>(P, st);
+            ++launches;
+        }
+        e = cudaGetLastError();
+    }
+    cudaEventRecord(total.e1, stream);
+    WfCounters c{};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&c, st.ctr, sizeof(WfCounters), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return e;
+    }
+    c.samples += c.sky_samples;  // counted apart, as by k_sky_tasks
+    c.rays_closest += c.sky_samples;
+    c.pool_slots = P.n_slots;
+    c.launches = launches;
+    *hc = c;
+    if (ms) cudaEventElapsedTime(ms, total.e0, total.e1);
+    return e;
+}
+}  // namespace
+
 // A single render whose per-task sums would exceed P.max_part_tasks runs its
 // sample chunks in batches (chunks [c0, c1) of every pixel, then the next
 // batch), merging each onto the film in task order: device memory for the
@@ -2307,6 +2535,8 @@ cudaError_t wf_render(const WfScene& S, const WfParams& P_in, WfBuffers& B, doub
     size_t part_tasks = 0;
     if (P.n_chunks > 1)
         part_tasks = P.jobs ? (size_t)P.n_tasks : (size_t)std::min<long long>(P.n_tasks, batch_chunks * P.n_pixels);
+    const bool direct = !profile && use_graph_loop && batch_chunks >= P.n_chunks && direct_render(P);
+    if (direct) return render_direct(S, P, B, acc, acc_w, acc_sq, part_tasks, stream, sm_count, hc, ms);
     cudaError_t e = reserve_pool(B, P, part_tasks);
     if (e != cudaSuccess) return e;
     WfState st = B.st;
@@ -2358,7 +2588,7 @@ cudaError_t wf_render(const WfScene& S, const WfParams& P_in, WfBuffers& B, doub
             const long long pooled = P.jobs ? n_fetch : batch_chunk_count * n_may;
             if (pooled > 0 && pooled < Pb.n_slots) Pb.n_slots = (int)pooled;
         }
-        // the drain's handover to k_tail (1080p frame, 64 Mi slots: 2.838 -> 2.931 G paths/s at
+        // the drain's handover to k_paths (1080p frame, 64 Mi slots: 2.838 -> 2.931 G paths/s at
         // 262,144; 2.921 at 65,536, 2.930 at 1 Mi, 2.781 at 4 Mi)
         if (Pb.tail_live < 0) Pb.tail_live = std::min(262144, Pb.n_slots / 16);
         cudaMemsetAsync(st.ctr, 0, sizeof(WfCounters), stream);
@@ -2404,9 +2634,7 @@ cudaError_t wf_render(const WfScene& S, const WfParams& P_in, WfBuffers& B, doub
                 }, st.ctr, P.max_iters, stream, use_graph_loop);
                 if (e == cudaSuccess && Pb.tail_live > 0) {
                     // the slots the loop left (none when it drained the pool)
-                    const unsigned grid = (unsigned)((Pb.tail_live + 127) / 128);
-                    if (P.jobs) wf::k_tail<true><<<grid, 128, 0, stream>>>(S, Pb, st);
-                    else wf::k_tail<false><<<grid, 128, 0, stream>>>(S, Pb, st);
+                    launch_paths<false>(S, Pb, st, nullptr, Pb.tail_live, sm_count, stream);
                     ++launches;
                     e = cudaGetLastError();
                 }
@@ -2496,16 +2724,19 @@ cudaError_t wf_render_adaptive(const WfScene& S, const WfParams& P_in, WfBuffers
         Pb.task_first = 0;
         Pb.n_slots = (int)std::min<long long>(P0.n_slots, Pb.n_tasks);
         Pb.max_iters = (long long)tspp * (long long)(P0.max_bounces + 1) * ((Pb.n_tasks + Pb.n_slots - 1) / Pb.n_slots + 1) + 16;
-        if (Pb.tail_live < 0) Pb.tail_live = std::min(262144, Pb.n_slots / 16);  // each round's drain
         cudaMemsetAsync(st.ctr, 0, sizeof(WfCounters), stream);
-        wf::k_init<false><<<(Pb.n_slots + 255) / 256, 256, 0, stream>>>(S, Pb, st);
+        Pb.tail_live = P0.tail_live;
+        const bool direct = use_graph_loop && direct_render(Pb);
+        if (Pb.tail_live < 0) Pb.tail_live = std::min(262144, Pb.n_slots / 16);  // each round's drain
+        if (direct) launch_paths<true>(S, Pb, st, nullptr, Pb.n_tasks, sm_count, stream);
+        else wf::k_init<false><<<(Pb.n_slots + 255) / 256, 256, 0, stream>>>(S, Pb, st);
         e = cudaGetLastError();
-        if (e == cudaSuccess)
+        if (e == cudaSuccess && !direct)
             e = wf_run_loop([&](cudaStream_t s, cudaGraphConditionalHandle h, int use_cond) {
                 enqueue_iteration(S, Pb, st, g, s, h, use_cond);
             }, st.ctr, Pb.max_iters, stream, use_graph_loop);
-        if (e == cudaSuccess && Pb.tail_live > 0) {
-            wf::k_tail<false><<<(unsigned)((Pb.tail_live + 127) / 128), 128, 0, stream>>>(S, Pb, st);
+        if (e == cudaSuccess && !direct && Pb.tail_live > 0) {
+            launch_paths<false>(S, Pb, st, nullptr, Pb.tail_live, sm_count, stream);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemsetAsync(B.n_active, 0, sizeof(int), stream);
@@ -2549,37 +2780,20 @@ cudaError_t wf_render_adaptive(const WfScene& S, const WfParams& P_in, WfBuffers
 // Some callers cannot allocate device memory while they render: a process
 // that reserves the whole GPU for its own allocator at start-up, or one that
 // cannot afford the device-wide synchronisation cudaMalloc/cudaFree imply in
-// the middle of a frame loop.  wf_render_noalloc runs the same wavefront
-// kernels with their path state and queues carved out of one file-scope
-// device array instead of a cudaMalloc'd block, launches them directly (no
-// graph or event objects are created) and allocates nothing.
+// the middle of a frame loop.  wf_render_noalloc runs k_paths, which carries
+// its paths in registers, so all it needs in device memory is the counters,
+// a file-scope device variable; it launches it directly (no graph or event
+// objects are created) and allocates nothing.
 //
 // Limits: films of at most kNoAllocMaxSlots pixels.  Every call shares the
-// array: calls that overlap on the GPU (other streams or host threads) race
-// on it, and each call re-initialises the counters and path state it uses.
+// counters: calls that overlap on the GPU (other streams or host threads)
+// race on them, and each call clears them.
+static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(tpt::WfCounters)];
+
 namespace tpt {
 namespace {
 
 constexpr size_t kNoAllocMaxSlots = 16384;  // e.g. 128 x 128
-
-constexpr size_t na_align(size_t x) { return (x + 255) & ~(size_t)255; }
-// Same arrays as wf_reserve, for kNoAllocMaxSlots slots.
-constexpr size_t kNoAllocBytes =
-    na_align(2 * kNoAllocMaxSlots * 4) + 6 * na_align(kNoAllocMaxSlots * 16) + 3 * na_align(2 * kNoAllocMaxSlots * 16) +
-    na_align(kNoAllocMaxSlots * 16) + na_align(kNoAllocMaxSlots) + na_align(2 * kNoAllocMaxSlots * 4) +
-    na_align(kNoAllocMaxSlots * 4) + na_align(sizeof(WfCounters)) + na_align(kNoAllocMaxSlots * 32) +
-    2 * na_align(kNoAllocMaxSlots * 16) + na_align(5 * kNoAllocMaxSlots * 4) + na_align(64);
-
-}  // namespace
-}  // namespace tpt
-
-// 5,128,704 bytes (about 5.1 MB), held by every GPU that loads the library
-// until the process exits.
-static_assert(tpt::kNoAllocBytes == 5128704, "the documented size of the allocation-free scratch array");
-static __device__ __align__(256) unsigned char g_noalloc_scratch[tpt::kNoAllocBytes];
-
-namespace tpt {
-namespace {
 
 std::mutex g_noalloc_mu;
 void* g_noalloc_addr[256] = {};
@@ -2613,65 +2827,16 @@ cudaError_t wf_render_noalloc(const WfScene& S, const WfParams& P, double* acc, 
     void* base = nullptr;
     cudaError_t e = noalloc_scratch(&base);
     if (e != cudaSuccess) return e;
-    const size_t n = kNoAllocMaxSlots;
-    char* p = static_cast<char*>(base);
-    size_t off = 0;
-    auto take = [&](size_t bytes) { char* r = p + off; off += na_align(bytes); return (void*)r; };
     WfState st{};
-    st.q_ext[0] = (int*)take(2 * n * 4);
-    st.q_ext[1] = st.q_ext[0] + n;
-    st.path = (int4*)take(n * 16);
-    st.ray_o = (float4*)take(n * 16);
-    st.ray_d = (float4*)take(n * 16);
-    st.beta = (float4*)take(n * 16);
-    st.rad = (float4*)take(n * 16);
-    st.hit = (float4*)take(n * 16);
-    st.sh_o = (float4*)take(2 * n * 16);
-    st.sh_d = (float4*)take(2 * n * 16);
-    st.sh_c = (float4*)take(2 * n * 16);
-    st.welford = P.adaptive ? (double2*)take(n * 16) : (take(n * 16), nullptr);
-    st.act = (uint8_t*)take(n);
-    st.q_sh = (int*)take(2 * n * 4);
-    st.q_term = (int*)take(n * 4);
-    st.ctr = (WfCounters*)take(sizeof(WfCounters));
-    st.sacc = (double4*)take(n * 32);
-    st.surf_p = (float4*)take(n * 16);
-    st.surf_n = (float4*)take(n * 16);
-    st.q_mat = (int*)take(5 * n * 4);
-    st.cmp_counts = (int*)take(64);  // wf_compact_spans(16384) = 2 ints
-    st.job = nullptr;  // single-scene renders only
-    st.ssq = nullptr;
-    st.part = nullptr;
-    st.part_sq = nullptr;
+    st.ctr = static_cast<WfCounters*>(base);
     st.acc = acc;
     st.acc_w = acc_w;
-    st.acc_sq = nullptr;
-    const Grids g = pick_grids(sm_count);
-    // The counters must start at zero; k_init initialises every slot it uses.
     e = cudaMemsetAsync(st.ctr, 0, sizeof(WfCounters), stream);
     if (e != cudaSuccess) return e;
-    wf::k_init<false><<<(P.n_slots + 255) / 256, 256, 0, stream>>>(S, P, st);
+    launch_paths<true>(S, P, st, nullptr, P.n_tasks, sm_count, stream);
     e = cudaGetLastError();
-    long long iters = 0;
-    while (e == cudaSuccess) {
-        for (int k = 0; k < 8; ++k) {  // 8 x two iterations between host checks
-            for (int cur = 0; cur < 2; ++cur) {
-                launch_trace<false, false>(g.extend, stream, S, P, st, P.n_slots, P.trace_chunk, cur);
-                launch_shade(g, stream, S, P, st, cur);
-                launch_trace<true, false>(g.shadow, stream, S, P, st, P.n_slots, P.trace_chunk, cur);
-                launch_regen(g.regen, stream, S, P, st, cur);
-                if (P.ordered_queue) wf_launch_compact(stream, st, cur, P.n_slots);
-                wf::k_step<<<1, 1, 0, stream>>>(st, cur, P.max_iters, cudaGraphConditionalHandle{}, 0);
-            }
-        }
-        iters += 16;
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hc, st.ctr, sizeof(WfCounters), cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        if (e != cudaSuccess) break;
-        if (hc->n_ext[0] == 0 && hc->n_ext[1] == 0) break;
-        if ((hc->flags & TPT_FLAG_ITER_LIMIT) || iters > P.max_iters + 16) break;
-    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(hc, st.ctr, sizeof(WfCounters), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     return e;
 }
 

@@ -109,7 +109,7 @@ struct WfParams {
                                // from WfState::q_ext (use_ext_queue); 0: always sweep the act bytes
     int queue_div;             // TPT_QUEUE_DIV, default 8
     int tail_live;             // > 0: once no tasks are left and at most this many slots are live, the
-                               // bounce loop stops and k_tail runs each of them to the end (single,
+                               // bounce loop stops and k_paths runs each of them to the end (single,
                                // batch and adaptive-round renders; 0 = the loop drains the pool; -1 =
                                // the default, 262,144 but at most a sixteenth of the pool)
     int ordered_queue;         // 1: the extension queue is rebuilt in slot order after every iteration
@@ -157,9 +157,10 @@ struct WfCounters {
     int n_mat[5];              // surface-hit queue lengths per material kind
     int fetch_ext, fetch_sh;   // dynamic work-fetch cursors of the trace kernels
     int flags;                 // TPT_FLAG_*
-    int tail;                  // 1: the bounce loop handed its last live slots to k_tail
+    int tail;                  // 1: the bounce loop handed its last live slots to k_paths
     long long iters;
     long long next_task;       // task pool cursor
+    long long next_item;       // k_paths: tasks or live slots taken
     unsigned long long rays_closest, rays_shadow, samples;
     // profiling variant only: [0] closest hit, [1] occlusion
     unsigned long long cnt_nodes[2], cnt_tris[2], cnt_spheres[2], cnt_inst[2];
@@ -300,7 +301,7 @@ cudaError_t wf_run_loop(const WfEnqueue& enqueue, const WfCounters* ctr, long lo
                         bool use_graph_loop);
 
 // Allocation-free render (see the comment above wf_render_noalloc in
-// wavefront.cu): path state in a file-scope device array, direct launches,
+// wavefront.cu): one kernel, counters in a file-scope device variable,
 // films of at most wf_noalloc_max_slots() pixels.
 size_t wf_noalloc_max_slots();
 cudaError_t wf_render_noalloc(const WfScene& S, const WfParams& P, double* acc, double* acc_w, cudaStream_t stream,
