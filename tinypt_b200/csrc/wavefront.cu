@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(128) k_shade_pre(WfScene S, WfParams P, WfStat
 constexpr int kShadeBlock = 256;
 // A path between two closest-hit rays, in registers.
 struct PathRegs {
-    float3 o, d;              // the ray traced last; after bounce(): the next one
+    float3 o, d;              // the ray
     int self_prim, self_inst; // what it starts on
     float t;                  // what it met
     int prim, inst;
@@ -611,11 +611,14 @@ struct PathRegs {
 
 // One bounce of radiance() (src/integrator.rs:67-132): what the closest-hit
 // ray met, the NEE samples -- `emit(k, origin, tmax, direction, contribution)`
-// for each shadow ray, 0 = env, 1 = area light -- and the next direction.
-// Returns true when the path ends.  STAGED: every thread of the block calls
+// for each shadow ray, 0 = env, 1 = area light -- and the next ray --
+// `next(origin, direction, self primitive, self instance)`.  The callbacks let
+// k_shade store the rays at once instead of keeping them in registers (its
+// budget: 1080p frame +3% with them kept).  Returns true when the path ends.  STAGED: every thread of the block calls
 // it, `active` or not, and the block's warps meet between the stages.
-template <bool STAGED, class Emit>
-__device__ __forceinline__ bool bounce(const WfScene& S, const WfParams& P, PathRegs& p, bool active, Emit&& emit) {
+template <bool STAGED, class Emit, class Next>
+__device__ __forceinline__ bool bounce(const WfScene& S, const WfParams& P, PathRegs& p, bool active, Emit&& emit,
+                                       Next&& next) {
     auto stage = [] {
         if constexpr (STAGED) __syncthreads();
     };
@@ -791,10 +794,7 @@ __device__ __forceinline__ bool bounce(const WfScene& S, const WfParams& P, Path
             p.beta = p.beta * w;
             p.last_pdf = pdf;
             p.fl = delta ? (p.fl & ~F_LAST_ND) : (p.fl | F_LAST_ND);
-            p.o = no + nd * kEps;
-            p.d = nd;
-            p.self_prim = self_ok ? prim : -1;
-            p.self_inst = self_ok ? inst : -1;
+            next(no + nd * kEps, nd, self_ok ? prim : -1, self_ok ? inst : -1);
             p.m.y += 1;
             if (p.m.y >= P.max_bounces) done = true;  // bounce loop bound (:67)
         }
@@ -932,6 +932,9 @@ __global__ void __launch_bounds__(kShadeBlock, CTAS * 128 / kShadeBlock) k_shade
             sts(&st.sh_d[2 * slot + k], make_float4(wi.x, wi.y, wi.z, ifloat(prim)));
             sts(&st.sh_c[2 * slot + k], make_float4(contrib.x, contrib.y, contrib.z, ifloat(inst)));
             sh[k] = 1;
+        }, [&](float3 o, float3 d, int self_prim, int self_inst) {
+            sts(&st.ray_o[slot], make_float4(o.x, o.y, o.z, ifloat(self_prim)));
+            sts(&st.ray_d[slot], make_float4(d.x, d.y, d.z, ifloat(self_inst)));
         });
         if (active) p.fl |= (sh[0] ? F_PEND_ENV : 0) | (sh[1] ? F_PEND_AREA : 0);
         bool cont = active && !done, need_task = false, camera = false;
@@ -956,14 +959,12 @@ __global__ void __launch_bounds__(kShadeBlock, CTAS * 128 / kShadeBlock) k_shade
         }
         if (camera) {
             start_sample(S, P, tp, p);
+            sts(&st.ray_o[slot], make_float4(p.o.x, p.o.y, p.o.z, ifloat(-1)));
+            sts(&st.ray_d[slot], make_float4(p.d.x, p.d.y, p.d.z, ifloat(-1)));
             cont = true;
         }
         if (cont || term) {
-            if (cont) {
-                sts(&st.ray_o[slot], make_float4(p.o.x, p.o.y, p.o.z, ifloat(p.self_prim)));
-                sts(&st.ray_d[slot], make_float4(p.d.x, p.d.y, p.d.z, ifloat(p.self_inst)));
-                sts(&st.beta[slot], make_float4(p.beta.x, p.beta.y, p.beta.z, p.last_pdf));
-            }
+            if (cont) sts(&st.beta[slot], make_float4(p.beta.x, p.beta.y, p.beta.z, p.last_pdf));
             sts(&st.rad[slot], make_float4(p.L.x, p.L.y, p.L.z, p.time));
             p.m.z = p.fl;
             store_path(st, slot, p.m, p.rng);
@@ -1561,6 +1562,11 @@ __global__ void __launch_bounds__(kPathsBlock, 3) k_paths(WfScene S0, WfParams P
             if (k == 0) { sh_o[0] = so; sh_d[0] = wi; sh_c[0] = contrib; }
             else { sh_o[1] = so; sh_d[1] = wi; sh_c[1] = contrib; sh_t = tmax; }
             jobs |= k == 0 ? kEnv : kArea;
+        }, [&](float3 o, float3 d, int self_prim, int self_inst) {
+            p.o = o;
+            p.d = d;
+            p.self_prim = self_prim;
+            p.self_inst = self_inst;
         });
         if (shade) {
             if (done) ended = true;
