@@ -534,6 +534,7 @@ void batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, con
         J.cam = bs.cam;
         J.top_root = bs.top_root;
         J.env_kind = bs.env_kind; J.env_w = bs.env_w; J.env_h = bs.env_h; J.env_has_cdf = bs.env_has_cdf;
+        J.env_black = bs.env_black;
         J.env_tex = B.wf.env_tex ? B.wf.env_tex + bs.env_tex_off : nullptr;
         J.env_row = B.wf.env_row ? B.wf.env_row + bs.env_row_off : nullptr;
         J.env_col = B.wf.env_col ? B.wf.env_col + bs.env_col_off : nullptr;
@@ -572,6 +573,7 @@ void batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, con
         S.cam = bs.cam;
         S.top_root = bs.top_root;
         S.env_kind = bs.env_kind; S.env_w = bs.env_w; S.env_h = bs.env_h; S.env_has_cdf = bs.env_has_cdf;
+        S.env_black = bs.env_black;
         S.env_tex = B.wf.env_tex ? B.wf.env_tex + bs.env_tex_off : nullptr;
         S.env_row = B.wf.env_row ? B.wf.env_row + bs.env_row_off : nullptr;
         S.env_col = B.wf.env_col ? B.wf.env_col + bs.env_col_off : nullptr;
@@ -770,6 +772,7 @@ int tpt_scene_create(const tpt_scene_desc* desc, void** out_scene) {
         W.env_w = hs.env_w;
         W.env_h = hs.env_h;
         W.env_has_cdf = hs.env_total > 0.0;
+        W.env_black = P.env_black = env_is_black(hs);
         W.env_tex = h->upload(fi.env_texels);
         W.env_row = h->upload(fi.env_row_cdf);
         W.env_col = h->upload(fi.env_col_cdf);
@@ -923,6 +926,7 @@ int tpt_scene_set_materials(void* scene, const tpt_material* materials, const tp
         h.plain.n_lights = (int)pl.size();
         h.plain.light_total = h.hs.light_total;
         h.wf.lights64 = h.plain.lights;
+        h.wf.env_black = h.plain.env_black = env_is_black(h.hs);
         ck(cudaStreamSynchronize(h.stream), "material upload");
         return TPT_OK;
     });

@@ -537,7 +537,8 @@ __device__ __forceinline__ float3 sky(float3 rd) {
 // What a ray that leaves the scene sees (src/integrator.rs:71-83): the env
 // map, or without one the sky.
 __device__ __forceinline__ float3 background(const WfScene& S, float3 rd) {
-    return S.env_kind == TPT_ENV_MAP ? env_lookup(S, rd) : sky(rd);
+    if (S.env_kind != TPT_ENV_MAP) return sky(rd);
+    return S.env_black ? f3(0.0f, 0.0f, 0.0f) : env_lookup(S, rd);
 }
 static __device__ float env_pdf(const WfScene& S, float3 d) {
     if (!S.env_has_cdf) return 1.0f / (4.0f * kPi);

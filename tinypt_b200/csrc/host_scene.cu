@@ -305,6 +305,15 @@ void build_lights(HostScene& hs) {
     hs.light_total = total;
 }
 
+bool env_is_black(const HostScene& hs) {
+    if (hs.env_kind != TPT_ENV_MAP) return false;
+    for (const std::vector<tpt_material>* v : {&hs.mats, &hs.smats})
+        for (const tpt_material& m : *v)
+            if (!std::isfinite(m.rgb[0]) || !std::isfinite(m.rgb[1]) || !std::isfinite(m.rgb[2]) || !std::isfinite(m.param))
+                return false;
+    return std::all_of(hs.env_data.begin(), hs.env_data.end(), [](double x) { return x == 0.0; });
+}
+
 void set_materials(HostScene& hs, const tpt_material* mats, const tpt_material* sampling, size_t n) {
     if (n != hs.mats.size()) throw std::runtime_error("set_materials: material count differs from the scene's");
     if (!mats) throw std::runtime_error("set_materials: null materials");
@@ -917,6 +926,7 @@ void merge_scenes(const std::vector<const HostScene*>& scenes, BatchImage& out) 
         b.env_w = hs.env_w;
         b.env_h = hs.env_h;
         b.env_has_cdf = hs.env_total > 0.0;
+        b.env_black = env_is_black(hs);
         b.env_tex_off = F.env_texels.size();
         b.env_row_off = F.env_row_cdf.size();
         b.env_col_off = F.env_col_cdf.size();

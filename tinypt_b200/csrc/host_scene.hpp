@@ -92,6 +92,10 @@ void build_host_scene(const tpt_scene_desc& desc, HostScene& out, const MeshBvhB
 // are lights and their selection weights) with the emission of hs.mats.
 void build_lights(HostScene& hs);
 
+// True when the env map is black (every texel 0) and no material parameter is
+// infinite or NaN: then neither a miss nor an env sample adds anything.
+bool env_is_black(const HostScene& hs);
+
 // Replaces the materials (same count and kinds); sampling = nullptr means
 // sampling follows evaluation.  Rebuilds the light table.
 void set_materials(HostScene& hs, const tpt_material* mats, const tpt_material* sampling, size_t n);
@@ -148,7 +152,7 @@ void link_plain(const PlainImage& plain, const Fp32Image& fp, std::vector<int2>&
 struct BatchScene {
     int32_t top_root;
     CameraF32 cam;
-    int32_t env_kind, env_w, env_h, env_has_cdf;
+    int32_t env_kind, env_w, env_h, env_has_cdf, env_black;
     size_t env_tex_off, env_row_off, env_col_off;   // element offsets
     int32_t light_begin, n_lights;
     int32_t n_mats, mat_begin;

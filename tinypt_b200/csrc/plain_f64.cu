@@ -798,7 +798,9 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
         V bg = mk(0, 0, 0);
         double pe = 1.0 / (4.0 * kPi);
         __syncthreads();
-        if (has_env && shade && (!found || nee)) bg = env_at(S, dir, want_pdf, pe);
+        // (a black map adds 0 whatever the direction)
+        const bool dark = S.env_black && beta.x + beta.y + beta.z < kTMax;
+        if (has_env && !dark && shade && (!found || nee)) bg = env_at(S, dir, want_pdf, pe);
         __syncthreads();
         if (shade && !found) {  // miss
             if (!has_env) {
@@ -841,6 +843,7 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
                 const V wi = k == 0 ? dir : area_wi, li = k == 0 ? bg : le;
                 const double cs = k == 0 ? ce : ca, pl = k == 0 ? pe : lpdf;
                 ++n_shadow;
+                if (k == 0 && dark) continue;
                 V f;
                 double pb;
                 mat_eval(mat, wo, wi, nrm, f, pb);

@@ -23,7 +23,7 @@ struct PlainScene {
     const double* light_cdf;
     int n_lights;
     double light_total;
-    int env_kind, env_w, env_h;
+    int env_kind, env_w, env_h, env_black;  // env_black: env_is_black
     const double* env_data;
     const double* env_row_cdf;
     const double* env_col_cdf;

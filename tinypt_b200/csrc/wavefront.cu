@@ -52,6 +52,7 @@ __device__ __forceinline__ void apply_job(const WfJob& J, WfScene& S, WfParams& 
     S.cam = J.cam;
     S.top_root = J.top_root;
     S.env_kind = J.env_kind; S.env_w = J.env_w; S.env_h = J.env_h; S.env_has_cdf = J.env_has_cdf;
+    S.env_black = J.env_black;
     S.env_tex = J.env_tex; S.env_row = J.env_row; S.env_col = J.env_col;
     S.lights = J.lights; S.light_cdf = J.light_cdf; S.lights64 = J.lights64; S.n_lights = J.n_lights;
     P.width = J.width; P.height = J.height; P.spp = J.spp; P.max_bounces = J.max_bounces; P.rr_start = J.rr_start;
@@ -671,9 +672,19 @@ __device__ __forceinline__ bool bounce(const WfScene& S, const WfParams& P, Path
     float3 wi = rd, li = f3(0, 0, 0);
     float pe = 1.0f / (4.0f * kPi);
     bool want_pdf = (p.fl & F_LAST_ND) != 0;
-    if (nee && has_env) want_pdf = env_sample_to(S, p.rng, wi);
+    // a black map (XML scenes carry one) adds 0 whatever the direction: its
+    // samples only take their two draws
+    const bool dark = S.env_black && p.beta.x + p.beta.y + p.beta.z < INFINITY;
+    if (nee && has_env) {
+        if (dark) {
+            pcg_f32(p.rng);
+            pcg_f32(p.rng);
+        } else {
+            want_pdf = env_sample_to(S, p.rng, wi);
+        }
+    }
     stage();
-    if (has_env && (miss || nee)) {
+    if (has_env && !dark && (miss || nee)) {
         float pdf = pe;
         li = env_at(S, wi, &pdf);
         if (want_pdf) pe = pdf;
@@ -686,7 +697,7 @@ __device__ __forceinline__ bool bounce(const WfScene& S, const WfParams& P, Path
         p.L = p.L + clamp_lum(contrib, 50.0f);
         done = true;
     }
-    if (nee && has_env) {  // nee_environment (:148-172)
+    if (nee && has_env && !dark) {  // nee_environment (:148-172)
         const float c = fmaxf(dot(n, wi), 0.0f);
         if (c > 0.0f && pe > 0.0f) {
             float3 f;

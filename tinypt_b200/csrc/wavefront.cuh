@@ -45,6 +45,7 @@ struct WfScene {
     const float* light_cdf;
     int n_lights;
     int env_kind, env_w, env_h, env_has_cdf;
+    int env_black;             // env_is_black: the map adds nothing to any path
     const float4* env_tex;     // rgb + nearest-texel pdf_uv
     const float* env_row;      // h+1, normalised
     const float* env_col;      // h*(w+1), normalised per row
@@ -62,7 +63,7 @@ struct WfScene {
 struct WfJob {
     CameraF32 cam;
     int top_root;
-    int env_kind, env_w, env_h, env_has_cdf;
+    int env_kind, env_w, env_h, env_has_cdf, env_black;
     const float4* env_tex;
     const float* env_row;
     const float* env_col;
