@@ -74,6 +74,20 @@ __device__ __forceinline__ int find_job(const WfParams& P, long long task) {
 }
 __device__ __forceinline__ Film film_of(const WfState& st) { return Film{st.acc, st.acc_w, st.acc_sq}; }
 
+// The scene, parameters and film of a job (single renders: of the render).
+struct View {
+    WfScene S;
+    WfParams P;
+    Film F;
+    long long task_begin;
+};
+template <bool BATCH>
+__device__ __forceinline__ View view_of(const WfScene& S0, const WfParams& P0, const WfState& st, int job) {
+    View v{S0, P0, film_of(st), 0};
+    if constexpr (BATCH) apply_job(P0.jobs[job], v.S, v.P, v.F, v.task_begin);
+    return v;
+}
+
 // Where task lt (its index within its job) sits: task-space pixel j = lt %
 // n_pixels, sample chunk lt / n_pixels; the film pixel (through px_map in an
 // adaptive round), its first sample and its length.
@@ -924,13 +938,10 @@ __global__ void __launch_bounds__(kShadeBlock, CTAS * 128 / kShadeBlock) k_shade
             fetch(st.ray_o + next); fetch(st.ray_d + next); fetch(st.hit + next);
             fetch(st.beta + next); fetch(st.rad + next); fetch(st.path + next);
         }
-        WfScene S = S0;
-        WfParams P = P0;
-        Film F = film_of(st);
-        long long tbase = 0;
         PathRegs p{};
+        int job = 0;
         if (active) {
-            if constexpr (BATCH) apply_job(P0.jobs[st.job[slot]], S, P, F, tbase);
+            if constexpr (BATCH) job = st.job[slot];
             p = load_slot(st, slot);
             const float4 h4 = lds(&st.hit[slot]);
             p.t = h4.x;
@@ -939,7 +950,8 @@ __global__ void __launch_bounds__(kShadeBlock, CTAS * 128 / kShadeBlock) k_shade
         }
         int sh[2] = {0, 0};
         const int prim = p.prim, inst = p.inst;
-        const bool done = bounce<true>(S, P, p, active, [&](int k, float3 so, float tmax, float3 wi, float3 contrib) {
+        const View vb = view_of<BATCH>(S0, P0, st, job);  // (an idle thread: job 0's)
+        const bool done = bounce<true>(vb.S, vb.P, p, active, [&](int k, float3 so, float tmax, float3 wi, float3 contrib) {
             sts(&st.sh_o[2 * slot + k], make_float4(so.x, so.y, so.z, tmax));
             sts(&st.sh_d[2 * slot + k], make_float4(wi.x, wi.y, wi.z, ifloat(prim)));
             sts(&st.sh_c[2 * slot + k], make_float4(contrib.x, contrib.y, contrib.z, ifloat(inst)));
@@ -953,24 +965,26 @@ __global__ void __launch_bounds__(kShadeBlock, CTAS * 128 / kShadeBlock) k_shade
         const bool term = active && done && (sh[0] || sh[1]), finished = active && done && !term;
         TaskPos tp{};
         if (finished) {  // nothing pending: the sample ends here instead of in k_regen
-            tp = task_pos(P, (long long)p.m.w - tbase);
+            const View v = view_of<BATCH>(S0, P0, st, job);
+            tp = task_pos(v.P, (long long)p.m.w - v.task_begin);
             Sums sums = load_sums(st, slot, p.m.x == 0);
-            camera = finish_sums(P, st, p.m, p.L, need_task, F, tp, sums);
+            camera = finish_sums(v.P, st, p.m, p.L, need_task, v.F, tp, sums);
             if (camera) store_sums(st, slot, sums);
         }
         const long long task = next_task(P0, st, need_task);
         if (task >= 0) {
             if constexpr (BATCH) {
-                const int j = find_job(P0, task);
-                st.job[slot] = j;
-                apply_job(P0.jobs[j], S, P, F, tbase);
+                job = find_job(P0, task);
+                st.job[slot] = job;
             }
-            tp = task_pos(P, task - tbase);
+            const View v = view_of<BATCH>(S0, P0, st, job);
+            tp = task_pos(v.P, task - v.task_begin);
             p.m = make_int4(0, 0, 0, (int)task);
             camera = true;
         }
         if (camera) {
-            start_sample(S, P, tp, p);
+            const View v = view_of<BATCH>(S0, P0, st, job);
+            start_sample(v.S, v.P, tp, p);
             sts(&st.ray_o[slot], make_float4(p.o.x, p.o.y, p.o.z, ifloat(-1)));
             sts(&st.ray_d[slot], make_float4(p.d.x, p.d.y, p.d.z, ifloat(-1)));
             cont = true;
@@ -1557,20 +1571,16 @@ __global__ void __launch_bounds__(kPathsBlock, 3) k_paths(WfScene S0, WfParams P
     int job = 0, jobs = 0;
     long long visits = 0;
     bool alive = false, ended = false, sky_task = false, exhausted = lane_id() >= lanes;
+    // taken anew at each use, so that no job's fields wait in registers
+    auto view = [&](int j) { return view_of<BATCH>(S0, P0, st, j); };
     for (;;) {
-        WfScene S = S0;
-        WfParams P = P0;
-        Film F = film_of(st);
-        long long tbase = 0;
-        // (A lane without a task takes its last job's view, or job 0's: with
-        // the overlay under a condition nvcc 12.9 left P.width at P0's 0.)
-        if constexpr (BATCH) apply_job(P0.jobs[job], S, P, F, tbase);
         const bool shade = alive && !ended;
         if (shade) {
             sh_prim = p.prim;
             sh_inst = p.inst;
         }
-        const bool done = bounce<true>(S, P, p, shade, [&](int k, float3 so, float tmax, float3 wi, float3 contrib) {
+        const View v = view(job);  // (a lane without a task: its last job's, or job 0's)
+        const bool done = bounce<true>(v.S, v.P, p, shade, [&](int k, float3 so, float tmax, float3 wi, float3 contrib) {
             if (k == 0) { sh_o[0] = so; sh_d[0] = wi; sh_c[0] = contrib; }
             else { sh_o[1] = so; sh_d[1] = wi; sh_c[1] = contrib; sh_t = tmax; }
             jobs |= k == 0 ? kEnv : kArea;
@@ -1592,9 +1602,10 @@ __global__ void __launch_bounds__(kPathsBlock, 3) k_paths(WfScene S0, WfParams P
         bool camera = false;
         TaskPos tp{};
         if (alive && ended && jobs == 0) {  // the sample is complete
-            tp = task_pos(P, (long long)p.m.w - tbase);
+            const View v = view(job);
+            tp = task_pos(v.P, (long long)p.m.w - v.task_begin);
             bool task_done = false;
-            camera = finish_sums(P, st, p.m, p.L, task_done, F, tp, sums);
+            camera = finish_sums(v.P, st, p.m, p.L, task_done, v.F, tp, sums);
             if (sky_task) ++sky_samples;
             else ++samples;
             alive = !task_done;
@@ -1618,10 +1629,10 @@ __global__ void __launch_bounds__(kPathsBlock, 3) k_paths(WfScene S0, WfParams P
                         long long pixel0 = 0;
                         if constexpr (BATCH) {
                             job = find_job(P0, task);
-                            apply_job(P0.jobs[job], S, P, F, tbase);
                             pixel0 = P0.jobs[job].pixel_begin;
                         }
-                        tp = task_pos(P, task - tbase);
+                        const View v = view(job);
+                        tp = task_pos(v.P, task - v.task_begin);
                         p.m = make_int4(0, 0, 0, (int)task);
                         sums = zero_sums();
                         sky_task = open && open[pixel0 + tp.pixel];
@@ -1638,7 +1649,8 @@ __global__ void __launch_bounds__(kPathsBlock, 3) k_paths(WfScene S0, WfParams P
             }
         }
         if (camera) {
-            start_sample(S, P, tp, p);
+            const View v = view(job);
+            start_sample(v.S, v.P, tp, p);
             p.t = kTMax;
             p.prim = p.inst = -1;
             ended = false;
