@@ -341,7 +341,7 @@ typedef struct tpt_tuning {
     int32_t task_spp;           /* samples per pool task (default 8)          */
     int32_t trace_chunk;        /* leaf visits between lane refills (def. 16) */
     int32_t shade_ctas;         /* resident blocks per SM the shading kernel is
-                                   compiled for: 4 or 8 (default 4)          */
+                                   compiled for: 4 or 8 (default 8)          */
 } tpt_tuning;
 
 /* Builds every scene's BVHs and uploads them merged (one handle). */

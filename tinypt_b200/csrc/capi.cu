@@ -463,14 +463,14 @@ struct Schedule {
     long long pool;
     int task_spp;
     int trace_chunk;
-    int shade_ctas;  // 4 or 8
+    int shade_ctas;  // 4 or 8 (8 by default: batch of 10 scenes 28.2 ms, 29.6 at 4)
 };
 Schedule schedule_of(const tpt_tuning* t) {
     Schedule sc;
     sc.pool = (t && t->pool_slots > 0) ? t->pool_slots : env_int("TPT_POOL", kDefaultPool);
     sc.task_spp = (t && t->task_spp > 0) ? t->task_spp : env_int("TPT_TASK_SPP", kDefaultTaskSpp);
     sc.trace_chunk = (t && t->trace_chunk > 0) ? std::min(std::max(t->trace_chunk, 1), 64) : trace_chunk_setting();
-    const int ctas = (t && t->shade_ctas > 0) ? t->shade_ctas : env_int("TPT_SHADE_CTAS", 4);
+    const int ctas = (t && t->shade_ctas > 0) ? t->shade_ctas : env_int("TPT_SHADE_CTAS", 8);
     sc.shade_ctas = ctas == 8 ? 8 : 4;
     if (sc.pool < 1) sc.pool = 1;
     if (sc.task_spp < 1) sc.task_spp = 1;
