@@ -776,6 +776,15 @@ int tpt_scene_create(const tpt_scene_desc* desc, void** out_scene) {
         W.env_tex = h->upload(fi.env_texels);
         W.env_row = h->upload(fi.env_row_cdf);
         W.env_col = h->upload(fi.env_col_cdf);
+        if (W.env_has_cdf) {
+            const size_t w = (size_t)hs.env_w, rows = (size_t)hs.env_h;
+            std::vector<uint16_t> row_guide, col_guide;
+            W.env_row_k = guide_table(fi.env_row_cdf, 1, rows + 1, row_guide);
+            W.env_col_k = guide_table(fi.env_col_cdf, rows, w + 1, col_guide);
+            W.env_row_guide = h->upload(row_guide);
+            W.env_col_guide = h->upload(col_guide);
+            ck(cudaStreamSynchronize(h->stream), "env guide upload");
+        }
         const CameraF64& c = hs.cam;
         W.cam.o = make_float3((float)c.o[0], (float)c.o[1], (float)c.o[2]);
         W.cam.u = make_float3((float)c.u[0], (float)c.u[1], (float)c.u[2]);

@@ -138,6 +138,12 @@ struct Fp32Image {       // FP32 layout for the wavefront kernels
 };
 void flatten_fp32(const HostScene& hs, Fp32Image& img);
 
+// Starting brackets for searches of `rows` non-decreasing CDFs of n entries
+// each: for k = the power of two from n, at most 1024, buckets of [0, 1], the
+// largest lo in [0, n - 2] with cdf[lo] <= j / k (0 if none), j = 0 .. k.
+// Returns k, or 0 (no table) where an entry would not fit 16 bits.
+int guide_table(const std::vector<float>& cdf, size_t rows, size_t n, std::vector<uint16_t>& guide);
+
 // What the plain f64 kernel needs to walk the FP32 image's trees: per
 // triangle in their leaf order, its index in plain.tris and the node of
 // plain.nodes whose leaf range holds it; and the padding of the top-level

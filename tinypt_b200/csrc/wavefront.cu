@@ -53,6 +53,7 @@ __device__ __forceinline__ void apply_job(const WfJob& J, WfScene& S, WfParams& 
     S.top_root = J.top_root;
     S.env_kind = J.env_kind; S.env_w = J.env_w; S.env_h = J.env_h; S.env_has_cdf = J.env_has_cdf;
     S.env_black = J.env_black;
+    S.env_row_guide = S.env_col_guide = nullptr;  // (a batch's maps are searched whole)
     S.env_tex = J.env_tex; S.env_row = J.env_row; S.env_col = J.env_col;
     S.lights = J.lights; S.light_cdf = J.light_cdf; S.lights64 = J.lights64; S.n_lights = J.n_lights;
     P.width = J.width; P.height = J.height; P.spp = J.spp; P.max_bounces = J.max_bounces; P.rr_start = J.rr_start;
