@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <memory>
 #include <stdexcept>
@@ -779,10 +780,19 @@ int tpt_scene_create(const tpt_scene_desc* desc, void** out_scene) {
         if (W.env_has_cdf) {
             const size_t w = (size_t)hs.env_w, rows = (size_t)hs.env_h;
             std::vector<uint16_t> row_guide, col_guide;
-            W.env_row_k = guide_table(fi.env_row_cdf, 1, rows + 1, row_guide);
-            W.env_col_k = guide_table(fi.env_col_cdf, rows, w + 1, col_guide);
+            auto unit = [](size_t) { return 1.0f; };
+            W.env_row_k = guide_table(fi.env_row_cdf, 1, rows + 1, unit, row_guide);
+            W.env_col_k = guide_table(fi.env_col_cdf, rows, w + 1, unit, col_guide);
             W.env_row_guide = h->upload(row_guide);
             W.env_col_guide = h->upload(col_guide);
+            // the f64 form's CDFs are not normalised: the kernel's row sums
+            std::vector<uint16_t> row_guide64, col_guide64;
+            const std::vector<double>& rc = pi.env_row_cdf;
+            P.env_row_k = guide_table(rc, 1, rows + 1, [&](size_t) { return hs.env_total; }, row_guide64);
+            P.env_col_k = guide_table(pi.env_col_cdf, rows, w + 1,
+                                      [&](size_t y) { return std::fmax(rc[y + 1] - rc[y], 0.0); }, col_guide64);
+            P.env_row_guide = h->upload(row_guide64);
+            P.env_col_guide = h->upload(col_guide64);
             ck(cudaStreamSynchronize(h->stream), "env guide upload");
         }
         const CameraF64& c = hs.cam;

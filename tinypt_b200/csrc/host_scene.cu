@@ -778,22 +778,6 @@ void flatten_fp32(const HostScene& hs, Fp32Image& img) {
     }
 }
 
-int guide_table(const std::vector<float>& cdf, size_t rows, size_t n, std::vector<uint16_t>& guide) {
-    if (n < 2 || n > 65535) return 0;
-    size_t k = 1;
-    while (k < n && k < 1024) k *= 2;
-    guide.resize(rows * (k + 1));
-    for (size_t r = 0; r < rows; ++r) {
-        const float* c = &cdf[r * n];
-        size_t lo = 0;
-        for (size_t j = 0; j <= k; ++j) {
-            while (lo + 1 <= n - 2 && c[lo + 1] <= (float)j / (float)k) ++lo;
-            guide[r * (k + 1) + j] = (uint16_t)lo;
-        }
-    }
-    return (int)k;
-}
-
 void link_plain(const PlainImage& plain, const Fp32Image& fp, std::vector<int2>& links, float& top_pad) {
     const size_t n = plain.tris.size();
     links.resize(n);

@@ -596,8 +596,18 @@ __device__ __forceinline__ V env_at(const PlainScene& S, V dir, bool want_pdf, d
     }
     return c0 * (1.0 - fy) + c1 * fy;
 }
-__device__ size_t cdf_search(const double* cdf, size_t n, double x) {      // env.rs:185-197, world.rs:324-336
+// env.rs:185-197, world.rs:324-336.  guide, when given, holds the answers at
+// the edges of k equal buckets of the variate u that x is a multiple of: the
+// answer for x lies between those of u's bucket.
+__device__ size_t cdf_search(const double* cdf, size_t n, double x, const uint16_t* guide = nullptr, int k = 0,
+                             double u = 0.0) {
     size_t lo = 0, hi = n == 0 ? 0 : n - 1;
+    if (guide) {
+        const int b = (int)(u * (double)k);  // u in [0, 1), k a power of two: exact
+        lo = guide[b];
+        const size_t above = (size_t)guide[b + 1] + 1;
+        if (above < hi) hi = above;
+    }
 #pragma unroll 1
     while (lo + 1 < hi) {
         size_t mid = (lo + hi) / 2;
@@ -610,13 +620,14 @@ __device__ size_t cdf_search(const double* cdf, size_t n, double x) {      // en
 __device__ bool env_sample_dir(const PlainScene& S, uint64_t& rng, V& dir) {
     const size_t W = (size_t)S.env_w, H = (size_t)S.env_h;
     if (S.env_total > 0.0) {
-        double r0 = pcg_f64(rng) * S.env_total;
-        size_t y = cdf_search(S.env_row_cdf, H + 1, r0);
+        const double u0 = pcg_f64(rng), r0 = u0 * S.env_total;
+        size_t y = cdf_search(S.env_row_cdf, H + 1, r0, S.env_row_guide, S.env_row_k, u0);
         if (y > H - 1) y = H - 1;
         double row_sum = fmax(S.env_row_cdf[y + 1] - S.env_row_cdf[y], 0.0);
         if (row_sum > 0.0) {
-            double r1 = pcg_f64(rng) * row_sum;
-            size_t x = cdf_search(S.env_col_cdf + y * (W + 1), W + 1, r1);
+            const double u1 = pcg_f64(rng), r1 = u1 * row_sum;
+            const uint16_t* guide = S.env_col_guide ? S.env_col_guide + y * (size_t)(S.env_col_k + 1) : nullptr;
+            size_t x = cdf_search(S.env_col_cdf + y * (W + 1), W + 1, r1, guide, S.env_col_k, u1);
             if (x > W - 1) x = W - 1;
             double u = ((double)x + pcg_f64(rng)) / (double)W;
             double v = ((double)y + pcg_f64(rng)) / (double)H;

@@ -28,6 +28,10 @@ struct PlainScene {
     const double* env_row_cdf;
     const double* env_col_cdf;
     double env_total;
+    // brackets of the two searches by the variate (guide_table; null: none)
+    const uint16_t* env_row_guide;
+    const uint16_t* env_col_guide;  // env_col_k + 1 per row
+    int env_row_k, env_col_k;
     CameraF64 cam;
     // The FP32 forms' trees (WfScene's arrays) and, per triangle in their
     // leaf order, its place in `tris` (x) and its leaf in `nodes` (y).
