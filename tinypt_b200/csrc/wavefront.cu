@@ -2722,7 +2722,10 @@ cudaError_t wf_render_adaptive(const WfScene& S, const WfParams& P_in, WfBuffers
     // round 0 takes the first min_spp samples (whole tasks): no pixel can stop before them
     const int min_spp = std::min(std::max(P0.adaptive_min_spp, 1), std::max(P0.spp, 1));
     const int first_len = std::min(P0.spp, (min_spp + tspp - 1) / tspp * tspp);
-    const size_t cap = std::max(round_bytes / 16, (size_t)n_film * (size_t)first_len);
+    // never more than the render's samples: round_bytes follows the free memory,
+    // and a buffer sized by it was allocated anew whenever that grew
+    const size_t cap = std::min(std::max(round_bytes / 16, (size_t)n_film * (size_t)first_len),
+                                (size_t)n_film * (size_t)std::max(P0.spp, first_len));
     cudaError_t e = round_reserve(B, (size_t)n_film, cap);
     if (e == cudaSuccess) e = reserve_pool(B, P0, 0);
     if (e != cudaSuccess) return e;
