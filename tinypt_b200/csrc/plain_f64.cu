@@ -13,6 +13,7 @@
 // (world_trace), and only the primitives that are left run the reference's
 // f64 arithmetic.
 #include "plain_f64.cuh"
+#include "texel.hpp"
 
 #include <algorithm>
 
@@ -46,8 +47,6 @@ __device__ __forceinline__ V clamp_lum(V c, double m) {             // math.rs:4
 }
 __device__ __forceinline__ V reflect(V v, V n) { return v - (2.0 * dot(v, n)) * n; }  // math.rs:193
 __device__ __forceinline__ double clampd(double x, double a, double b) { return fmin(fmax(x, a), b); }
-// Rust `f as usize` (saturating; NaN -> 0) for the small ranges used here.
-__device__ __forceinline__ size_t as_usize(double f) { return f > 0.0 ? (size_t)f : 0; }
 
 struct Ray { V o, d; double time; };
 struct Hit { double t; V p, n; int mat; };
@@ -563,10 +562,10 @@ __device__ __forceinline__ V env_at(const PlainScene& S, V dir, bool want_pdf, d
     const int W = S.env_w, H = S.env_h;
     double x = u * (double)W;
     double y = v * ((double)H - 1.0);
-    int x0 = (int)floor(x);           // 0 <= u <= 1 (a NaN converts to 0), so x0 % W needs one step
+    int x0 = texel_index(x, W);       // 0 <= u <= 1 or NaN, so x0 % W needs one step
     if (x0 >= W) x0 -= W;
     const int x1 = x0 + 1 < W ? x0 + 1 : 0;
-    const int y0 = (int)floor(clampd(y, 0.0, (double)(H - 1)));
+    const int y0 = texel_index(y, H - 1);
     const int y1 = y0 + 1 < H - 1 ? y0 + 1 : H - 1;
     double fx = x - floor(x), fy = y - floor(y);
     const double* D = S.env_data;
@@ -578,10 +577,7 @@ __device__ __forceinline__ V env_at(const PlainScene& S, V dir, bool want_pdf, d
     if (want_pdf) {
         pdf = 1.0 / (4.0 * kPi);
         if (S.env_total > 0.0) {
-            double fxw = floor(u * (double)W), fyh = floor(v * (double)H);
-            fxw = fxw < 0.0 ? 0.0 : (fxw > (double)(W - 1) ? (double)(W - 1) : fxw);
-            fyh = fyh < 0.0 ? 0.0 : (fyh > (double)(H - 1) ? (double)(H - 1) : fyh);
-            const int px = (int)fxw, py = (int)fyh;
+            const int px = texel_index(u * (double)W, W - 1), py = texel_index(v * (double)H, H - 1);
             double th0 = kPi * (double)py / (double)H, th1 = kPi * (double)(py + 1) / (double)H;
             double st = fmax(sin(theta), 1e-6);
             double rw = fmax(cos(th0) - cos(th1), 0.0);
