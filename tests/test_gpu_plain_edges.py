@@ -1,0 +1,60 @@
+"""The plain f64 form where numbers leave their usual range: rays that are not
+numbers, infinite lights, directions far from unit length, films of 2^30
+pixels.  The oracle runs the reference's loops; pixels are NaN where its are
+and equal its to 1e-9 otherwise, but for the samples whose path a last bit of
+CUDA's sine or cosine sends another way (at most 0.2%, the bar of the other
+plain f64 tests)."""
+import math
+
+import numpy as np
+import pytest
+
+from tinypt_b200 import _abi, scenes
+from tinypt_b200.render import DeviceScene
+from tinypt_b200.scene import Camera, Instance, Material, Mesh, Scene, Sphere, Transform, World
+from tests.parity_util import cfg, gpu_film
+
+pytestmark = pytest.mark.gpu
+
+PLAIN = _abi.TPT_MODE_PLAIN_F64
+W, H = 48, 32
+INF, NAN = float("inf"), float("nan")
+
+
+def _same_as_oracle(oracle_mod, scene, spp=4, depth=6, w=W, h=H):
+    c = cfg(w, h, spp, depth, PLAIN, seed=3)
+    with oracle_mod.OracleScene(scene) as o:
+        want, want_w, _, _ = o.render(c, want_sq=True)
+    with DeviceScene(scene) as ds:
+        (acc, acc_w, _), st = gpu_film(ds, c)
+    assert np.array_equal(acc_w, want_w) and st.device_flags == 0
+    same = (np.isnan(acc) & np.isnan(want)) | (acc == want) | (np.abs(acc - want) <= 1e-9 * np.maximum(np.abs(want), 1e-12))
+    assert (~same.all(axis=1)).mean() <= 1.0 - 0.998 ** spp
+    return want
+
+
+def _spheres(light, aspect):
+    """A light as the light-th of five spheres, one of them of a glass that
+    refracts into a NaN."""
+    mats = [Material.dielectric(INF, (0.1, 0.1, 0.1)), Material.lambert((0.7, 0.5, 0.3)),
+            Material.metal((0.8, 0.8, 0.8)), Material.diffuse_light((1.0, 2.0, 3.0))]
+    s = Scene(Camera.look_at((0.0, 0.6, 4.0), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 45.0, aspect), World(), mats, None)
+    others = [Sphere((-0.8, 0.0, 0.0), 0.5, 0), Sphere((0.8, 0.0, 0.0), 0.5, 1), Sphere((0.0, -100.5, 0.0), 100.0, 2),
+              Sphere((0.1, 0.0, -1.0), 0.4, 1)]
+    others.insert(light, Sphere((0.0, 0.9, 0.0), 0.3, 3))
+    s.world.spheres.extend(others)
+    return s
+
+
+@pytest.mark.parametrize("light", [0, 2, 4])
+@pytest.mark.parametrize("aspect", [W / H, NAN])
+def test_rays_that_are_not_numbers(gpu, oracle_mod, light, aspect):
+    """Every test of the reference's loops lets a NaN pass, so such a ray meets
+    the last sphere; mesh hits at a NaN distance do not count."""
+    s = _spheres(light, aspect)
+    v, f = scenes.displaced_icosphere(1, 0.08, 3, 5)
+    s.world.meshes.append(Mesh.from_arrays(v * 0.3, f, 1))
+    s.world.instances.append(Instance(0, Transform.translate((0.3, 0.3, 1.0)), None))
+    want = _same_as_oracle(oracle_mod, s)
+    if math.isnan(aspect):
+        assert (want.max() > 0.0) == (light == 4)

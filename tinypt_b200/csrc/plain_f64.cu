@@ -233,6 +233,29 @@ __device__ __forceinline__ bool mesh_done(const PlainScene& S, const Ray& r, V o
     return true;
 }
 
+// World::hit by the reference's own loops, for a ray that is not a number or
+// beyond the range of the FP32 box tests.  Every comparison of the reference's
+// tests lets a NaN pass, so such a ray meets the last sphere; which one that is
+// only the order of its loop says.
+__device__ __noinline__ Best world_loops(const PlainScene& S, V ro, V rd, double time, double tmax, int* flags) {
+    const Ray r{ro, rd, time};
+    Best best{tmax, 0.0, -1, -1};
+    for (int i = 0; i < S.n_instances; ++i) {
+        const InstanceF64& I = S.instances[i];
+        const MeshF64 m = S.meshes[I.mesh_id];
+        if (m.n_nodes == 0) continue;
+        const V o = mat_vec(I.a_inv, r.o - ld(I.t)), d = norm(mat_vec(I.a_inv, r.d));
+        double th;
+        const int tri = bvh_hit(S.nodes + m.node_offset, S.tris + m.tri_offset, flags, o, d, r.time, kEps, 1e30, &th);
+        mesh_done(S, r, o, d, i, tri < 0 ? -1 : tri + m.tri_offset, th, best);
+    }
+    for (int i = 0; i < S.n_spheres; ++i) {
+        double t;
+        if (sphere_test(ld(S.spheres[i].c), S.spheres[i].r, r, kEps, best.t, t)) best = Best{t, 0.0, -1, i};
+    }
+    return best;
+}
+
 constexpr int kLeaveMesh = ~0;  // stack entry: back to world space (no leaf of a tree has the code 0 / 0)
 
 // World::hit over the top-level tree (spheres and instances) and the mesh
@@ -255,6 +278,10 @@ constexpr int kLeaveMesh = ~0;  // stack entry: back to world space (no leaf of 
 //    hit).  Then the mesh is walked again by bvh_hit.
 __device__ __forceinline__ bool world_trace(const PlainScene& S, const Ray& r, double tmax, bool any, Best& best,
                                             int* stack, int* flags) {
+    if (!(fabs(r.o.x + r.o.y + r.o.z + r.d.x + r.d.y + r.d.z) < 1e30)) {
+        best = world_loops(S, r.o, r.d, r.time, tmax, flags);
+        return best.prim >= 0;
+    }
     best = Best{tmax, 0.0, -1, -1};
     Ray32 q = ray32(r.o, r.d, S.top_pad);
     float far = __double2float_ru(tmax);
