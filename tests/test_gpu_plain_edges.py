@@ -1,7 +1,6 @@
 """The plain f64 form where numbers leave their usual range: rays that are not
-numbers, infinite lights, directions far from unit length, films of 2^30
-pixels.  The oracle runs the reference's loops; pixels are NaN where its are
-and equal its to 1e-9 otherwise, but for the samples whose path a last bit of
+numbers, directions far from unit length.  The oracle runs the reference's
+loops; pixels are NaN where its are and equal its to 1e-9 otherwise, but for the samples whose path a last bit of
 CUDA's sine or cosine sends another way (at most 0.2%, the bar of the other
 plain f64 tests)."""
 import math
@@ -58,3 +57,28 @@ def test_rays_that_are_not_numbers(gpu, oracle_mod, light, aspect):
     want = _same_as_oracle(oracle_mod, s)
     if math.isnan(aspect):
         assert (want.max() > 0.0) == (light == 4)
+
+
+def test_directions_of_another_length(gpu, oracle_mod):
+    """A mirror ball of radius 1e-11 at 1000 reflects into directions whose
+    length is off by a per cent (its normals are).  A hit of a mesh counts at
+    dot(p - o, d), a sphere's at its root: a glowing square just
+    outside a large sphere may be the closer one from inside."""
+    at = np.array([1000.0, 0.0, 0.0])
+    u, a = np.array([0.0, 0.0, 1.0]), np.array([1.0, 0.0, 0.0])
+    b = np.cross(u, a)
+    mats = [Material.metal((0.9, 0.9, 0.9)), Material.lambert((0.9, 0.1, 0.1)), Material.diffuse_light((0.1, 0.1, 0.9))]
+    r, d = 1e-11, 2e-4
+    s = Scene(Camera.look_at(tuple(at + d * u), tuple(at), (1.0, 0.0, 0.0), math.degrees(0.5 * r / d), W / H),
+              World(), mats, None)
+    s.world.spheres += [Sphere(tuple(at), r, 0), Sphere(tuple(at - 490.0 * u), 500.0, 1)]
+    centre, half = at + 10.1 * u, 5.0
+    k = 8  # squares a side, so that the mesh has a tree
+    p = np.array([centre + half * ((2 * i / k - 1.0) * a + (2 * j / k - 1.0) * b) for j in range(k + 1) for i in range(k + 1)])
+    q = np.array([j * (k + 1) + i for j in range(k) for i in range(k)])
+    f = np.concatenate([np.stack([q, q + 1, q + k + 2], 1), np.stack([q, q + k + 2, q + k + 1], 1)])
+    s.world.meshes.append(Mesh.from_arrays(p, f, 2))
+    s.world.instances.append(Instance(0, Transform.identity(), None))
+    want = _same_as_oracle(oracle_mod, s, spp=8, depth=3)
+    lit = want[:, 2] > 0.5 * want[:, 2].max()
+    assert 0.1 < lit.mean() < 0.9

@@ -233,10 +233,12 @@ __device__ __forceinline__ bool mesh_done(const PlainScene& S, const Ray& r, V o
     return true;
 }
 
-// World::hit by the reference's own loops, for a ray that is not a number or
-// beyond the range of the FP32 box tests.  Every comparison of the reference's
-// tests lets a NaN pass, so such a ray meets the last sphere; which one that is
-// only the order of its loop says.
+// World::hit by the reference's own loops, for a ray that is not a number,
+// beyond the range of the FP32 box tests or whose direction is not of unit
+// length.  Every comparison of the reference's tests lets a NaN pass, so such a
+// ray meets the last sphere; which one that is only the order of its loop says.
+// And instances count at dot(p - o, d), spheres at their root: only for a unit
+// direction does a box that starts past the one hold no closer other.
 __device__ __noinline__ Best world_loops(const PlainScene& S, V ro, V rd, double time, double tmax, int* flags) {
     const Ray r{ro, rd, time};
     Best best{tmax, 0.0, -1, -1};
@@ -278,7 +280,7 @@ constexpr int kLeaveMesh = ~0;  // stack entry: back to world space (no leaf of 
 //    hit).  Then the mesh is walked again by bvh_hit.
 __device__ __forceinline__ bool world_trace(const PlainScene& S, const Ray& r, double tmax, bool any, Best& best,
                                             int* stack, int* flags) {
-    if (!(fabs(r.o.x + r.o.y + r.o.z + r.d.x + r.d.y + r.d.z) < 1e30)) {
+    if (!(fabs(dot(r.d, r.d) - 1.0) < 1e-7 && fabs(r.o.x + r.o.y + r.o.z) < 1e30)) {
         best = world_loops(S, r.o, r.d, r.time, tmax, flags);
         return best.prim >= 0;
     }
@@ -334,8 +336,9 @@ __device__ __forceinline__ bool world_trace(const PlainScene& S, const Ray& r, d
                 redo = S.meshes[I.mesh_id].deep != 0;
                 q = ray32(o, d, 0.0f);
                 // hits past the closest one so far are not needed; one world
-                // unit is |A^-1 d| units here
-                const double reach = best.t * len(du) * (1.0 + 1e-6);
+                // unit is |A^-1 d| units here (|d| is 1), up to the rounding
+                // of the two transforms
+                const double reach = (best.t * (1.0 + 1e-6) + S.top_pad) * len(du);
                 far = reach < 1e30 ? __double2float_ru(reach) : 1e30f;
                 if (sp < kStack) stack[sp++] = kLeaveMesh;
                 else raise_flag(flags, TPT_FLAG_STACK_OVERFLOW);
