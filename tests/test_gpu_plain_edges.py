@@ -1,5 +1,5 @@
 """The plain f64 form where numbers leave their usual range: rays that are not
-numbers, directions far from unit length.  The oracle runs the reference's
+numbers, directions far from unit length, path weights that overflow.  The oracle runs the reference's
 loops; pixels are NaN where its are and equal its to 1e-9 otherwise, but for the samples whose path a last bit of
 CUDA's sine or cosine sends another way (at most 0.2%, the bar of the other
 plain f64 tests)."""
@@ -10,12 +10,12 @@ import pytest
 
 from tinypt_b200 import _abi, scenes
 from tinypt_b200.render import DeviceScene
-from tinypt_b200.scene import Camera, Instance, Material, Mesh, Scene, Sphere, Transform, World
+from tinypt_b200.scene import Camera, EnvMap, Instance, Material, Mesh, Scene, Sphere, Transform, World
 from tests.parity_util import cfg, gpu_film
 
 pytestmark = pytest.mark.gpu
 
-PLAIN = _abi.TPT_MODE_PLAIN_F64
+WF, PLAIN = _abi.TPT_MODE_WAVEFRONT_FP32, _abi.TPT_MODE_PLAIN_F64
 W, H = 48, 32
 INF, NAN = float("inf"), float("nan")
 
@@ -82,3 +82,24 @@ def test_directions_of_another_length(gpu, oracle_mod):
     want = _same_as_oracle(oracle_mod, s, spp=8, depth=3)
     lit = want[:, 2] > 0.5 * want[:, 2].max()
     assert 0.1 < lit.mean() < 0.9
+
+
+@pytest.mark.parametrize("mode", [WF, PLAIN])
+@pytest.mark.parametrize("albedos", [(-1e200, -1e200), (1e29, 1e300)])
+def test_black_map_with_overflowing_albedo(gpu, mode, albedos):
+    """A path weight that overflows times black is a NaN on the general path
+    (an unused infinite material selects it), so it is one on the shortcut."""
+    c = cfg(W, H, 4, 2, mode, seed=4)
+    films = []
+    for general in (False, True):
+        s = scenes.build_scene(W, H)
+        s.env = EnvMap.from_pixels(3, 2, np.zeros((2, 3, 3)))
+        s.mats = [Material.lambert((albedos[k % 2], albedos[k % 2], 0.5)) for k in range(len(s.mats))]
+        if general:
+            s.mats = s.mats + [Material.lambert((INF, 0.0, 0.0))]
+        with DeviceScene(s) as ds:
+            films.append(gpu_film(ds, c)[0])
+    if mode == PLAIN:
+        assert np.isnan(films[1][0]).any()
+    for a, b in zip(*films):
+        assert np.array_equal(a, b, equal_nan=True)

@@ -307,10 +307,11 @@ void build_lights(HostScene& hs) {
 
 bool env_is_black(const HostScene& hs) {
     if (hs.env_kind != TPT_ENV_MAP) return false;
+    // (at most 1e100: no product with a path weight below 1e30 overflows)
+    auto plain = [](double x) { return std::fabs(x) <= 1e100; };
     for (const std::vector<tpt_material>* v : {&hs.mats, &hs.smats})
         for (const tpt_material& m : *v)
-            if (!std::isfinite(m.rgb[0]) || !std::isfinite(m.rgb[1]) || !std::isfinite(m.rgb[2]) || !std::isfinite(m.param))
-                return false;
+            if (!plain(m.rgb[0]) || !plain(m.rgb[1]) || !plain(m.rgb[2]) || !plain(m.param)) return false;
     return std::all_of(hs.env_data.begin(), hs.env_data.end(), [](double x) { return x == 0.0; });
 }
 

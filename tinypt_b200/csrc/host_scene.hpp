@@ -93,7 +93,7 @@ void build_host_scene(const tpt_scene_desc& desc, HostScene& out, const MeshBvhB
 void build_lights(HostScene& hs);
 
 // True when the env map is black (every texel 0) and no material parameter is
-// infinite or NaN: then neither a miss nor an env sample adds anything.
+// NaN or beyond 1e100: then neither a miss nor an env sample adds anything.
 bool env_is_black(const HostScene& hs);
 
 // Replaces the materials (same count and kinds); sampling = nullptr means

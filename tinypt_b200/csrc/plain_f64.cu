@@ -835,8 +835,8 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
         V bg = mk(0, 0, 0);
         double pe = 1.0 / (4.0 * kPi);
         __syncthreads();
-        // (a black map adds 0 whatever the direction)
-        const bool dark = S.env_black && beta.x + beta.y + beta.z < kTMax;
+        // (a black map adds 0 whatever the direction, unless the weight overflows)
+        const bool dark = S.env_black && fabs(beta.x) + fabs(beta.y) + fabs(beta.z) < kTMax;
         if (has_env && !dark && shade && (!found || nee)) bg = env_at(S, dir, want_pdf, pe);
         __syncthreads();
         if (shade && !found) {  // miss
