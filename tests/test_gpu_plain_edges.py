@@ -1,7 +1,8 @@
 """The plain f64 form where numbers leave their usual range: rays that are not
-numbers, directions far from unit length, path weights that overflow.  The oracle runs the reference's
-loops; pixels are NaN where its are and equal its to 1e-9 otherwise, but for the samples whose path a last bit of
-CUDA's sine or cosine sends another way (at most 0.2%, the bar of the other
+numbers, directions far from unit length, path weights that overflow, films of
+2^30 pixels.  The oracle runs the reference's loops; pixels are NaN where its
+are and equal its to 1e-9 otherwise, but for the samples whose path a last bit
+of CUDA's sine or cosine sends another way (at most 0.2%, the bar of the other
 plain f64 tests)."""
 import math
 
@@ -103,3 +104,19 @@ def test_black_map_with_overflowing_albedo(gpu, mode, albedos):
         assert np.isnan(films[1][0]).any()
     for a, b in zip(*films):
         assert np.array_equal(a, b, equal_nan=True)
+
+
+def test_film_of_2_30_pixels_in_one_row(gpu):
+    """In whole 8x4 tiles such a film has 2^32 pixels."""
+    import torch
+
+    n = 1 << 30
+    acc = torch.full((3 * n,), -1.0, dtype=torch.float64, device="cuda")
+    acc_w = torch.zeros(n, dtype=torch.float64, device="cuda")
+    with DeviceScene(scenes.sphere_scene(8, 8)) as ds:
+        st = ds.render_device(cfg(n, 1, 1, 0, PLAIN), acc.data_ptr(), acc_w.data_ptr())
+    torch.cuda.synchronize()
+    whole = bool((acc_w == 1.0).all()) and bool((acc == 0.0).all())  # (not in the assert, which would list the film)
+    del acc, acc_w
+    torch.cuda.empty_cache()
+    assert whole and st.paths == n

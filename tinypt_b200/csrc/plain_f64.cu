@@ -784,7 +784,9 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
     const int max_spp = P.spp > 1 ? P.spp : 1;
     const int min_spp = min(P.adaptive_min_spp > 1 ? P.adaptive_min_spp : 1, max_spp);
     // pixels are handed out by 8 x 4 tiles, a warp's worth each
-    const unsigned tiles_x = (unsigned)(P.width + 7) / 8u, n_ids = tiles_x * ((unsigned)(P.n_rows + 3) / 4u) * 32u;
+    // (a film of 2^30 pixels in one row has 2^32 in whole tiles)
+    const unsigned tiles_x = (unsigned)(P.width + 7) / 8u;
+    const unsigned long long n_ids = (unsigned long long)tiles_x * ((unsigned)(P.n_rows + 3) / 4u) * 32u;
     int stack[kStack];
     unsigned long long n_samples = 0, n_closest = 0, n_shadow = 0;
     // the pixel
@@ -936,14 +938,14 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
         const bool want = x < 0 && !exhausted;
         const unsigned wm = __ballot_sync(0xffffffffu, want);
         if (wm) {
-            unsigned base = 0;
+            unsigned long long base = 0;
             const int leader = __ffs(wm) - 1;
-            if ((int)lane == leader) base = (unsigned)atomicAdd(&counters[3], (unsigned long long)__popc(wm));
+            if ((int)lane == leader) base = atomicAdd(&counters[3], (unsigned long long)__popc(wm));
             base = __shfl_sync(0xffffffffu, base, leader);
             if (want) {
-                const unsigned id = base + __popc(wm & ((1u << lane) - 1u));
-                const unsigned tile = id >> 5, ty = tile / tiles_x;
-                const int px = (int)((tile - ty * tiles_x) * 8u + (id & 7u)), py = (int)(ty * 4u + ((id >> 3) & 3u));
+                const unsigned long long id = base + __popc(wm & ((1u << lane) - 1u));
+                const unsigned tile = (unsigned)(id >> 5), in = (unsigned)id & 31u, ty = tile / tiles_x;
+                const int px = (int)((tile - ty * tiles_x) * 8u + (in & 7u)), py = (int)(ty * 4u + (in >> 3));
                 exhausted = id >= n_ids;
                 if (!exhausted && px < P.width && py < P.n_rows) {
                     x = px;
