@@ -113,6 +113,7 @@ def test_film_of_2_30_pixels_in_one_row(gpu):
     n = 1 << 30
     acc = torch.full((3 * n,), -1.0, dtype=torch.float64, device="cuda")
     acc_w = torch.zeros(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()  # the fills run on another stream than the render
     with DeviceScene(scenes.sphere_scene(8, 8)) as ds:
         st = ds.render_device(cfg(n, 1, 1, 0, PLAIN), acc.data_ptr(), acc_w.data_ptr())
     torch.cuda.synchronize()
