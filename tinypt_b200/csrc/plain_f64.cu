@@ -176,12 +176,14 @@ __device__ V mat_vec(const double* a, V p) {
 // in world units.  The second part, and `pad` (world units), widen the box:
 // the near planes' offset is lowered and the far planes' raised by that
 // much; the first is covered by kSlack on the far distance.
-constexpr float kSlack = 1.0f + 1e-6f;
+constexpr float kSlack = 1.0f + 3e-6f;
 struct Ray32 {
     float3 idir, near_off, far_off;
 };
-__device__ __forceinline__ float safe_rcp(float d) {
-    return 1.0f / (fabsf(d) > 1e-20f ? d : copysignf(1e-20f, d));
+__device__ __forceinline__ float safe_rcp(float d) {  // within an ulp
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(fabsf(d) > 1e-20f ? d : copysignf(1e-20f, d)));
+    return r;
 }
 __device__ __forceinline__ void set_axis(double o, double d, float pad, float& idir, float& lo, float& hi) {
     const float of = (float)o;
@@ -233,12 +235,19 @@ __device__ __forceinline__ bool mesh_done(const PlainScene& S, const Ray& r, V o
     return true;
 }
 
-// World::hit by the reference's own loops, for a ray that is not a number,
-// beyond the range of the FP32 box tests or whose direction is not of unit
-// length.  Every comparison of the reference's tests lets a NaN pass, so such a
-// ray meets the last sphere; which one that is only the order of its loop says.
-// And instances count at dot(p - o, d), spheres at their root: only for a unit
-// direction does a box that starts past the one hold no closer other.
+// A ray that is not a number, beyond the range of the FP32 box tests or not of
+// unit length.  (Shadow rays are none of these: a contribution is zero or
+// stopped by its cosine where the hit they start from is not a number.)
+__device__ __forceinline__ bool unusual(const Ray& r) {
+    const float ox = (float)r.o.x, oy = (float)r.o.y, oz = (float)r.o.z;
+    const float dx = (float)r.d.x, dy = (float)r.d.y, dz = (float)r.d.z;
+    return !(fabsf(dx * dx + dy * dy + dz * dz - 1.0f) < 1e-6f && fabsf(ox + oy + oz) < 1e30f);
+}
+// World::hit by the reference's own loops, for unusual rays.  Every comparison
+// of the reference's tests lets a NaN pass, so such a ray meets the last
+// sphere; which one that is only the order of its loop says.  And instances
+// count at dot(p - o, d), spheres at their root: only for a unit direction does
+// a box that starts past the one hold no closer other.
 __device__ __noinline__ Best world_loops(const PlainScene& S, V ro, V rd, double time, double tmax, int* flags) {
     const Ray r{ro, rd, time};
     Best best{tmax, 0.0, -1, -1};
@@ -278,9 +287,9 @@ constexpr int kLeaveMesh = ~0;  // stack entry: back to world space (no leaf of 
 //    triangles of one mesh hit at the same distance, or a leaf box entered
 //    no earlier than the hit (the box might have been culled by an earlier
 //    hit).  Then the mesh is walked again by bvh_hit.
-__device__ __forceinline__ bool world_trace(const PlainScene& S, const Ray& r, double tmax, bool any, Best& best,
-                                            int* stack, int* flags) {
-    if (!(fabs(dot(r.d, r.d) - 1.0) < 1e-7 && fabs(r.o.x + r.o.y + r.o.z) < 1e30)) {
+__device__ __forceinline__ bool world_trace(const PlainScene& S, const Ray& r, double tmax, bool any, bool by_loops,
+                                            Best& best, int* stack, int* flags) {
+    if (by_loops) {
         best = world_loops(S, r.o, r.d, r.time, tmax, flags);
         return best.prim >= 0;
     }
@@ -336,9 +345,9 @@ __device__ __forceinline__ bool world_trace(const PlainScene& S, const Ray& r, d
                 redo = S.meshes[I.mesh_id].deep != 0;
                 q = ray32(o, d, 0.0f);
                 // hits past the closest one so far are not needed; one world
-                // unit is |A^-1 d| units here (|d| is 1), up to the rounding
+                // unit is |A^-1 d| units here (|d|^2 is within 1e-6 of 1), up to the rounding
                 // of the two transforms
-                const double reach = (best.t * (1.0 + 1e-6) + S.top_pad) * len(du);
+                const double reach = (best.t * (1.0 + 3e-6) + S.top_pad) * len(du);
                 far = reach < 1e30 ? __double2float_ru(reach) : 1e30f;
                 if (sp < kStack) stack[sp++] = kLeaveMesh;
                 else raise_flag(flags, TPT_FLAG_STACK_OVERFLOW);
@@ -800,7 +809,7 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
     V L = mk(0, 0, 0), beta = mk(1, 1, 1);
     double last_pdf = 0.0;
     int bounce = 0, jobs = 0;
-    bool last_nd = false, ended = false, found = false;
+    bool last_nd = false, ended = false, found = false, odd = false;
     Best best{};
     // shadow rays: direction, contribution when nothing is in the way
     V sh_p = mk(0, 0, 0), env_wi = mk(0, 0, 0), env_c = mk(0, 0, 0), area_wi = mk(0, 0, 0), area_c = mk(0, 0, 0);
@@ -904,6 +913,7 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
                 ray = s.ray;
                 if (++bounce >= P.max_bounces) ended = true;
                 else jobs |= kJobClosest;
+                odd = unusual(ray);
             }
         }
         __syncthreads();
@@ -972,6 +982,7 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
             bounce = 0;
             ended = P.max_bounces <= 0;
             if (!ended) jobs = kJobClosest;
+            odd = unusual(ray);
         }
         if (!__syncthreads_or(x >= 0 || !exhausted)) break;
         while (__any_sync(0xffffffffu, jobs != 0)) {
@@ -985,7 +996,7 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
                     if (job == kJobArea) tmax = area_t;
                 }
                 Best b;
-                const bool h = world_trace(S, r, tmax, job != kJobClosest, b, stack, flags);
+                const bool h = world_trace(S, r, tmax, job != kJobClosest, job == kJobClosest && odd, b, stack, flags);
                 if (job == kJobClosest) {
                     best = b;
                     found = h;
