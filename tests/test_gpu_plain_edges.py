@@ -106,16 +106,31 @@ def test_black_map_with_overflowing_albedo(gpu, mode, albedos):
         assert np.array_equal(a, b, equal_nan=True)
 
 
-def test_film_of_2_30_pixels_in_one_row(gpu):
-    """In whole 8x4 tiles such a film has 2^32 pixels."""
+@pytest.mark.parametrize("w, h", [(1, 70), (5, 4), (7, 33), (8, 5), (9, 33), (33, 12), (200, 5)])
+def test_pixels_do_not_depend_on_the_tiles(gpu, w, h):
+    """A film's pixels are handed out by 8 x 4 or, below 8 columns, 1 x 32; a shard
+    of its rows with fewer than 4 by 32 x 1.  The shards make up the film, bit for
+    bit."""
+    step = (h + 2) // 3
+    with DeviceScene(scenes.build_scene(w, h)) as ds:
+        whole = ds.render(cfg(w, h, 4, 4, PLAIN)).acc.reshape(h, w, 3)
+        for k in range(step):
+            part = ds.render(cfg(w, h, 4, 4, PLAIN, row_begin=k, row_step=step)).acc.reshape(-1, w, 3)
+            assert 1 <= len(part) <= 3 and np.array_equal(part, whole[k::step])
+    assert whole.min() >= 0.0 and np.count_nonzero(whole.max(axis=2)) > 0
+
+
+@pytest.mark.parametrize("w, h", [(1 << 30, 1), (1, 1 << 30), (9, (1 << 30) // 9)])
+def test_films_of_2_30_pixels(gpu, w, h):
+    """In 8x4 tiles the first has 2^32 pixels, the second 2^33."""
     import torch
 
-    n = 1 << 30
+    n = w * h
     acc = torch.full((3 * n,), -1.0, dtype=torch.float64, device="cuda")
     acc_w = torch.zeros(n, dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()  # the fills run on another stream than the render
     with DeviceScene(scenes.sphere_scene(8, 8)) as ds:
-        st = ds.render_device(cfg(n, 1, 1, 0, PLAIN), acc.data_ptr(), acc_w.data_ptr())
+        st = ds.render_device(cfg(w, h, 1, 0, PLAIN), acc.data_ptr(), acc_w.data_ptr())
     torch.cuda.synchronize()
     whole = bool((acc_w == 1.0).all()) and bool((acc == 0.0).all())  # (not in the assert, which would list the film)
     del acc, acc_w

@@ -758,6 +758,21 @@ __device__ Ray camera_ray(const CameraF64& c, double sx, double sy, uint64_t& rn
     return Ray{origin, dir, time};
 }
 
+// Pixels are handed out by tiles of 32, a warp's worth each: 8 x 4, and where
+// the film is thinner than that 32 x 1 or 1 x 32.  A film of 2^30 pixels, the
+// largest, then has fewer than 3.1e9 ids, so that 32 bits hold them and what the
+// last lanes take in vain (64-bit ids cost 2 to 3% of a small scene's render).
+struct Tiles {
+    int log_w;
+    unsigned across, n_ids;
+};
+__host__ __device__ __forceinline__ Tiles tiles_of(const PlainParams& P) {
+    const int log_w = P.n_rows < 4 ? 5 : (P.width < 8 ? 0 : 3);
+    const unsigned w = 1u << log_w, h = 32u >> log_w;
+    const unsigned across = ((unsigned)P.width + w - 1u) / w;
+    return Tiles{log_w, across, across * (((unsigned)P.n_rows + h - 1u) / h) * 32u};
+}
+
 // What a path waits for before its next bounce.
 constexpr int kJobEnv = 1, kJobArea = 2, kJobClosest = 4;
 
@@ -792,10 +807,7 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
     const double inv_w = 1.0 / (double)P.width, inv_h = 1.0 / (double)P.height;
     const int max_spp = P.spp > 1 ? P.spp : 1;
     const int min_spp = min(P.adaptive_min_spp > 1 ? P.adaptive_min_spp : 1, max_spp);
-    // pixels are handed out by 8 x 4 tiles, a warp's worth each
-    // (a film of 2^30 pixels in one row has 2^32 in whole tiles)
-    const unsigned tiles_x = (unsigned)(P.width + 7) / 8u;
-    const unsigned long long n_ids = (unsigned long long)tiles_x * ((unsigned)(P.n_rows + 3) / 4u) * 32u;
+    const Tiles T = tiles_of(P);
     int stack[kStack];
     unsigned long long n_samples = 0, n_closest = 0, n_shadow = 0;
     // the pixel
@@ -948,15 +960,16 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
         const bool want = x < 0 && !exhausted;
         const unsigned wm = __ballot_sync(0xffffffffu, want);
         if (wm) {
-            unsigned long long base = 0;
+            unsigned base = 0;
             const int leader = __ffs(wm) - 1;
-            if ((int)lane == leader) base = atomicAdd(&counters[3], (unsigned long long)__popc(wm));
+            if ((int)lane == leader) base = (unsigned)atomicAdd(&counters[3], (unsigned long long)__popc(wm));
             base = __shfl_sync(0xffffffffu, base, leader);
             if (want) {
-                const unsigned long long id = base + __popc(wm & ((1u << lane) - 1u));
-                const unsigned tile = (unsigned)(id >> 5), in = (unsigned)id & 31u, ty = tile / tiles_x;
-                const int px = (int)((tile - ty * tiles_x) * 8u + (in & 7u)), py = (int)(ty * 4u + (in >> 3));
-                exhausted = id >= n_ids;
+                const unsigned id = base + __popc(wm & ((1u << lane) - 1u));
+                const unsigned tile = id >> 5, in = id & 31u, ty = tile / T.across;
+                const int px = (int)(((tile - ty * T.across) << T.log_w) + (in & ((1u << T.log_w) - 1u)));
+                const int py = (int)((ty << (5 - T.log_w)) + (in >> T.log_w));
+                exhausted = id >= T.n_ids;
                 if (!exhausted && px < P.width && py < P.n_rows) {
                     x = px;
                     row = py;
@@ -1035,7 +1048,7 @@ cudaError_t launch_plain(const PlainScene& S, const PlainParams& P, double* acc,
     // over the warps: a warp of a few lanes diverges less, and it is each
     // pixel's own chain of bounces that the render waits for (48x30 x 64 spp:
     // 7.5 ms in full warps, 4.6 spread).
-    const long long pixels = (long long)((P.width + 7) / 8) * ((P.n_rows + 3) / 4) * 32;  // in whole 8 x 4 tiles
+    const long long pixels = plain::tiles_of(P).n_ids;  // in whole tiles
     const long long warps = (long long)sm_count * 8;
     const unsigned lanes = (unsigned)std::min<long long>(32, std::max<long long>(1, (pixels + warps - 1) / warps));
     const long long per_block = (long long)lanes * (block / 32);
