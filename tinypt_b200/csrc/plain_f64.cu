@@ -294,6 +294,7 @@ __device__ __forceinline__ bool world_trace(const PlainScene& S, const Ray& r, d
         return best.prim >= 0;
     }
     best = Best{tmax, 0.0, -1, -1};
+    if (S.top_root == TPT_REF_NONE) return false;
     Ray32 q = ray32(r.o, r.d, S.top_pad);
     float far = __double2float_ru(tmax);
     V o = r.o, d = r.d;  // the ray in the entered mesh's space
@@ -730,6 +731,10 @@ __device__ bool sample_light(const PlainScene& S, uint64_t& rng, double time, V 
 }
 
 // ---- src/integrator.rs -----------------------------------------------------
+__device__ __forceinline__ V sky(V d) {  // :25-28
+    double t = 0.5 * (d.y + 1.0);
+    return (1.0 - t) * mk(0.9, 0.95, 1.0) + t * mk(0.6, 0.75, 1.0);
+}
 __device__ __forceinline__ double mis(double a, double b) {
     double a2 = a * a, b2 = b * b;
     return (a2 + b2 > 0.0) ? a2 / (a2 + b2) : 0.0;
@@ -773,6 +778,70 @@ __host__ __device__ __forceinline__ Tiles tiles_of(const PlainParams& P) {
     return Tiles{log_w, across, across * (((unsigned)P.n_rows + h - 1u) / h) * 32u};
 }
 
+// A pixel's sums (src/render.rs:158-191).
+struct Sums {
+    V c, c2;
+    double mean, m2;
+    int n;
+};
+// Adds a sample; true when it was the pixel's last.
+__device__ __forceinline__ bool add_sample(const PlainParams& P, Sums& s, V L) {
+    s.c = s.c + L;
+    s.c2 = s.c2 + had(L, L);
+    s.n += 1;
+    bool stop = s.n >= P.spp;
+    if (P.adaptive) {  // render.rs:160-176
+        const int min_spp = min(P.adaptive_min_spp > 1 ? P.adaptive_min_spp : 1, P.spp > 1 ? P.spp : 1);
+        double l = lum(L);
+        double delta = l - s.mean;
+        s.mean += delta / (double)s.n;
+        double delta2 = l - s.mean;
+        s.m2 += delta * delta2;
+        if (s.n >= min_spp) {
+            double var = s.n > 1 ? s.m2 / (double)(s.n - 1) : __longlong_as_double(0x7ff0000000000000ll);
+            double den = fmax(fabs(s.mean), 1e-4);
+            if (sqrt(var) / den < P.adaptive_threshold) stop = true;
+        }
+    }
+    return stop;
+}
+__device__ __forceinline__ void store_pixel(const PlainParams& P, int x, int row, const Sums& s, double* acc, double* acc_w,
+                                            double* acc_sq) {
+    const size_t gi = (size_t)row * (size_t)P.width + (size_t)x;
+    acc[3 * gi] = s.c.x; acc[3 * gi + 1] = s.c.y; acc[3 * gi + 2] = s.c.z;
+    acc_w[gi] = (double)s.n;
+    if (acc_sq) { acc_sq[3 * gi] = s.c2.x; acc_sq[3 * gi + 1] = s.c2.y; acc_sq[3 * gi + 2] = s.c2.z; }
+}
+__device__ __forceinline__ Ray sample_ray(const PlainScene& S, const PlainParams& P, int x, int row, double inv_w,
+                                          double inv_h, uint64_t& rng) {  // src/render.rs:151-158
+    const int y = P.row_begin + row * P.row_step;
+    double jx = pcg_f64(rng);
+    double jy = pcg_f64(rng);
+    double sx = ((double)x + jx) * inv_w * 2.0 - 1.0;
+    double sy = 1.0 - ((double)y + jy) * inv_h * 2.0;
+    return camera_ray(S.cam, sx, sy, rng);
+}
+// Pixel `id` of the film in the order of its tiles; false past the film's edge.
+__device__ __forceinline__ bool tile_pixel(const Tiles& T, const PlainParams& P, unsigned id, int& x, int& row) {
+    const unsigned tile = id >> 5, in = id & 31u, ty = tile / T.across;
+    x = (int)(((tile - ty * T.across) << T.log_w) + (in & ((1u << T.log_w) - 1u)));
+    row = (int)((ty << (5 - T.log_w)) + (in >> T.log_w));
+    return x < P.width && row < P.n_rows;
+}
+__device__ __forceinline__ void count_rays(unsigned long long* counters, unsigned long long n_samples,
+                                           unsigned long long n_closest, unsigned long long n_shadow) {
+    for (int off = 16; off > 0; off >>= 1) {
+        n_samples += __shfl_down_sync(0xffffffffu, n_samples, off);
+        n_closest += __shfl_down_sync(0xffffffffu, n_closest, off);
+        n_shadow += __shfl_down_sync(0xffffffffu, n_shadow, off);
+    }
+    if ((threadIdx.x & 31u) == 0) {
+        atomicAdd(&counters[0], n_samples);
+        atomicAdd(&counters[1], n_closest);
+        atomicAdd(&counters[2], n_shadow);
+    }
+}
+
 // What a path waits for before its next bounce.
 constexpr int kJobEnv = 1, kJobArea = 2, kJobClosest = 4;
 
@@ -795,9 +864,10 @@ constexpr int kJobEnv = 1, kJobArea = 2, kJobClosest = 4;
 // over the reference's tree and linear loops 43.7 / 115; this kernel without
 // barriers 21.0 / 17.3; with them 8.5 / 16.2 in blocks of 256, one per SM,
 // and 11.8 / 13.8 in blocks of 128, two per SM.  At 128 registers (512 lanes
-// per SM) 10.6 / 18.4.  `lanes` lanes of each warp take pixels.
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_constant__ PlainScene S,
+// per SM) 10.6 / 18.4.  `lanes` lanes of each warp take pixels.  SHORT: samples
+// end in the round of their last shadow rays.
+template <int BLOCK, int CTAS, bool SHORT>
+__global__ void __launch_bounds__(BLOCK, CTAS) k_paths(const __grid_constant__ PlainScene S,
                                                      const __grid_constant__ PlainParams P, double* __restrict__ acc,
                                                      double* __restrict__ acc_w, double* __restrict__ acc_sq,
                                                      unsigned long long* __restrict__ counters, int* flags,
@@ -805,16 +875,13 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
     const unsigned lane = threadIdx.x & 31u;
     const bool has_env = S.env_kind == TPT_ENV_MAP;
     const double inv_w = 1.0 / (double)P.width, inv_h = 1.0 / (double)P.height;
-    const int max_spp = P.spp > 1 ? P.spp : 1;
-    const int min_spp = min(P.adaptive_min_spp > 1 ? P.adaptive_min_spp : 1, max_spp);
     const Tiles T = tiles_of(P);
     int stack[kStack];
     unsigned long long n_samples = 0, n_closest = 0, n_shadow = 0;
     // the pixel
-    int x = -1, row = 0, n = 0;
+    int x = -1, row = 0;
     uint64_t rng = 0;
-    V c = mk(0, 0, 0), c2 = mk(0, 0, 0);
-    double mean = 0.0, m2 = 0.0;
+    Sums sums{};
     bool exhausted = lane >= lanes;
     // the path
     Ray ray{};
@@ -826,6 +893,74 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
     // shadow rays: direction, contribution when nothing is in the way
     V sh_p = mk(0, 0, 0), env_wi = mk(0, 0, 0), env_c = mk(0, 0, 0), area_wi = mk(0, 0, 0), area_c = mk(0, 0, 0);
     double area_t = 0.0;
+    // where a path has ended, its sample ends and the next one starts
+    auto next_sample = [&] {
+        bool start = false;
+        if (x >= 0 && ended && jobs == 0) {  // the sample is complete (src/render.rs:158-191)
+            const bool stop = add_sample(P, sums, L);
+            if (stop) {
+                store_pixel(P, x, row, sums, acc, acc_w, acc_sq);
+                n_samples += (unsigned long long)sums.n;
+                x = -1;
+            }
+            start = !stop;
+        }
+        const bool want = x < 0 && !exhausted;
+        const unsigned wm = __ballot_sync(0xffffffffu, want);
+        if (wm) {
+            unsigned base = 0;
+            const int leader = __ffs(wm) - 1;
+            if ((int)lane == leader) base = (unsigned)atomicAdd(&counters[3], (unsigned long long)__popc(wm));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (want) {
+                const unsigned id = base + __popc(wm & ((1u << lane) - 1u));
+                exhausted = id >= T.n_ids;
+                int px, py;
+                if (!exhausted && tile_pixel(T, P, id, px, py)) {
+                    x = px;
+                    row = py;
+                    sums = Sums{};
+                    rng = pixel_seed((uint32_t)x, (uint32_t)(P.row_begin + row * P.row_step), P.seed);
+                    start = true;
+                }
+            }
+        }
+        if (start) {
+            ray = sample_ray(S, P, x, row, inv_w, inv_h, rng);
+            L = mk(0, 0, 0);
+            beta = mk(1, 1, 1);
+            last_pdf = 0.0;
+            last_nd = false;
+            bounce = 0;
+            ended = P.max_bounces <= 0;
+            if (!ended) jobs = kJobClosest;
+            odd = unusual(ray);
+        }
+    };
+    auto trace = [&](int due) {
+        while (__any_sync(0xffffffffu, (jobs & due) != 0)) {
+            if ((jobs & due) != 0) {
+                const int job = jobs & -jobs;
+                Ray r = ray;
+                double tmax = kTMax;
+                if (job != kJobClosest) {
+                    const V wi = job == kJobEnv ? env_wi : area_wi;
+                    r = Ray{sh_p + kEps * wi, wi, ray.time};
+                    if (job == kJobArea) tmax = area_t;
+                }
+                Best b;
+                const bool h = world_trace(S, r, tmax, job != kJobClosest, job == kJobClosest && odd, b, stack, flags);
+                if (job == kJobClosest) {
+                    best = b;
+                    found = h;
+                    ++n_closest;
+                } else if (!h) {
+                    L = L + (job == kJobEnv ? env_c : area_c);
+                }
+                jobs ^= job;
+            }
+        }
+    };
     for (;;) {
         __syncthreads();
         const bool shade = x >= 0 && !ended;
@@ -863,10 +998,7 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
         if (has_env && !dark && shade && (!found || nee)) bg = env_at(S, dir, want_pdf, pe);
         __syncthreads();
         if (shade && !found) {  // miss
-            if (!has_env) {
-                double t = 0.5 * (ray.d.y + 1.0);  // sky (:25-28)
-                bg = (1.0 - t) * mk(0.9, 0.95, 1.0) + t * mk(0.6, 0.75, 1.0);
-            }
+            if (!has_env) bg = sky(ray.d);
             V contrib = had(beta, bg);
             if (has_env && last_nd) contrib = contrib * mis(last_pdf, pe);
             L = L + clamp_lum(contrib, 50.0);
@@ -929,132 +1061,143 @@ __global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_paths(const __grid_const
             }
         }
         __syncthreads();
-        bool start = false;
-        if (x >= 0 && ended && jobs == 0) {  // the sample is complete (src/render.rs:158-191)
-            c = c + L;
-            c2 = c2 + had(L, L);
-            n += 1;
-            bool stop = n >= P.spp;
-            if (P.adaptive) {  // render.rs:160-176
-                double l = lum(L);
-                double delta = l - mean;
-                mean += delta / (double)n;
-                double delta2 = l - mean;
-                m2 += delta * delta2;
-                if (n >= min_spp) {
-                    double var = n > 1 ? m2 / (double)(n - 1) : __longlong_as_double(0x7ff0000000000000ll);
-                    double den = fmax(fabs(mean), 1e-4);
-                    if (sqrt(var) / den < P.adaptive_threshold) stop = true;
-                }
-            }
-            if (stop) {
-                const size_t gi = (size_t)row * (size_t)P.width + (size_t)x;
-                acc[3 * gi] = c.x; acc[3 * gi + 1] = c.y; acc[3 * gi + 2] = c.z;
-                acc_w[gi] = (double)n;
-                if (acc_sq) { acc_sq[3 * gi] = c2.x; acc_sq[3 * gi + 1] = c2.y; acc_sq[3 * gi + 2] = c2.z; }
-                n_samples += (unsigned long long)n;
-                x = -1;
-            }
-            start = !stop;
+        if constexpr (SHORT) {
+            trace(kJobEnv | kJobArea);
+            __syncthreads();
         }
-        const bool want = x < 0 && !exhausted;
-        const unsigned wm = __ballot_sync(0xffffffffu, want);
-        if (wm) {
-            unsigned base = 0;
-            const int leader = __ffs(wm) - 1;
-            if ((int)lane == leader) base = (unsigned)atomicAdd(&counters[3], (unsigned long long)__popc(wm));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (want) {
-                const unsigned id = base + __popc(wm & ((1u << lane) - 1u));
-                const unsigned tile = id >> 5, in = id & 31u, ty = tile / T.across;
-                const int px = (int)(((tile - ty * T.across) << T.log_w) + (in & ((1u << T.log_w) - 1u)));
-                const int py = (int)((ty << (5 - T.log_w)) + (in >> T.log_w));
-                exhausted = id >= T.n_ids;
-                if (!exhausted && px < P.width && py < P.n_rows) {
-                    x = px;
-                    row = py;
-                    n = 0;
-                    c = c2 = mk(0, 0, 0);
-                    mean = m2 = 0.0;
-                    rng = pixel_seed((uint32_t)x, (uint32_t)(P.row_begin + row * P.row_step), P.seed);
-                    start = true;
-                }
-            }
-        }
-        if (start) {  // src/render.rs:151-158
-            const int y = P.row_begin + row * P.row_step;
-            double jx = pcg_f64(rng);
-            double jy = pcg_f64(rng);
-            double sx = ((double)x + jx) * inv_w * 2.0 - 1.0;
-            double sy = 1.0 - ((double)y + jy) * inv_h * 2.0;
-            ray = camera_ray(S.cam, sx, sy, rng);
-            L = mk(0, 0, 0);
-            beta = mk(1, 1, 1);
-            last_pdf = 0.0;
-            last_nd = false;
-            bounce = 0;
-            ended = P.max_bounces <= 0;
-            if (!ended) jobs = kJobClosest;
-            odd = unusual(ray);
-        }
+        next_sample();
         if (!__syncthreads_or(x >= 0 || !exhausted)) break;
-        while (__any_sync(0xffffffffu, jobs != 0)) {
-            if (jobs != 0) {
-                const int job = jobs & -jobs;
-                Ray r = ray;
-                double tmax = kTMax;
-                if (job != kJobClosest) {
-                    const V wi = job == kJobEnv ? env_wi : area_wi;
-                    r = Ray{sh_p + kEps * wi, wi, ray.time};
-                    if (job == kJobArea) tmax = area_t;
-                }
-                Best b;
-                const bool h = world_trace(S, r, tmax, job != kJobClosest, job == kJobClosest && odd, b, stack, flags);
-                if (job == kJobClosest) {
-                    best = b;
-                    found = h;
-                    ++n_closest;
-                } else if (!h) {
-                    L = L + (job == kJobEnv ? env_c : area_c);
-                }
-                jobs ^= job;
+        trace(kJobEnv | kJobArea | kJobClosest);
+    }
+    count_rays(counters, n_samples, n_closest, n_shadow);
+}
+
+// Paths that are all alike and all short (launch_plain): a lane per pixel runs
+// them sample after sample.  Where nothing diverges k_paths' rounds only add to
+// the latency of a sample's chain: empty scene 960x540 x 16 spp 0.55 ms in
+// k_paths, 0.27 here, built-in scene at one bounce 1280x720 x 4 spp 1.15 and 0.51.
+__global__ void __launch_bounds__(128, 3) k_first_hits(const __grid_constant__ PlainScene S,
+                                                       const __grid_constant__ PlainParams P, double* __restrict__ acc,
+                                                       double* __restrict__ acc_w, double* __restrict__ acc_sq,
+                                                       unsigned long long* __restrict__ counters, int* flags) {
+    const Tiles T = tiles_of(P);
+    const unsigned id = blockIdx.x * 128u + threadIdx.x;
+    const bool has_env = S.env_kind == TPT_ENV_MAP;
+    const double inv_w = 1.0 / (double)P.width, inv_h = 1.0 / (double)P.height;
+    int x = 0, row = 0;
+    unsigned long long n_samples = 0, n_closest = 0, n_shadow = 0;
+    int stack[kStack];
+    if (id < T.n_ids && tile_pixel(T, P, id, x, row)) {
+        uint64_t rng = pixel_seed((uint32_t)x, (uint32_t)(P.row_begin + row * P.row_step), P.seed);
+        Sums sums{};
+        V L;
+        do {
+            const Ray ray = sample_ray(S, P, x, row, inv_w, inv_h, rng);
+            L = mk(0, 0, 0);
+            if (P.max_bounces <= 0) continue;
+            ++n_closest;
+            Best best;
+            if (!world_trace(S, ray, kTMax, false, unusual(ray), best, stack, flags)) {
+                double unused;
+                L = L + clamp_lum(has_env ? env_at(S, ray.d, false, unused) : sky(ray.d), 50.0);
+                continue;
             }
-        }
+            V beta = mk(1, 1, 1);
+            if (P.rr_start <= 0) {
+                const double p = 0.95;  // of the largest channel, 1
+                if (pcg_f64(rng) > p) continue;
+                beta = beta / p;
+            }
+            const Hit hit = hit_of(S, ray, best);
+            const MaterialF64& mat = S.mats[hit.mat];
+            if (mat.kind == TPT_MAT_DIFFUSE_LIGHT) {
+                L = L + clamp_lum(had(beta, ld(mat.c)), 50.0);
+                continue;
+            }
+            if (mat.kind != TPT_MAT_METAL && mat.kind != TPT_MAT_DIELECTRIC) {
+                const V nrm = dot(hit.n, ray.d) < 0.0 ? hit.n : -hit.n, wo = norm(-ray.d);
+                // nee_environment (:148-172), then nee_area_light (:178-213)
+#pragma unroll 1
+                for (int k = has_env ? 0 : 1; k < 2; ++k) {
+                    V wi, li;
+                    double pl, tmax = kTMax;
+                    if (k == 0) {
+                        const bool by_cdf = env_sample_dir(S, rng, wi);
+                        pl = 1.0 / (4.0 * kPi);
+                        li = env_at(S, wi, by_cdf, pl);
+                    } else {
+                        V lp, ln;
+                        if (!sample_light(S, rng, ray.time, hit.p, lp, ln, li, pl)) continue;
+                        const V tl = lp - hit.p;
+                        const double dist = sqrt(dot(tl, tl));
+                        if (!(dist > 1e-6)) continue;
+                        wi = tl / dist;
+                        tmax = fmax(dist - kEps, kEps);
+                    }
+                    const double cs = fmax(dot(nrm, wi), 0.0);
+                    if (!(cs > 0.0) || (k == 0 && !(pl > 0.0))) continue;
+                    ++n_shadow;
+                    V f;
+                    double pb;
+                    mat_eval(mat, wo, wi, nrm, f, pb);
+                    const V contrib = had(had(beta, f), li) * (cs * mis(pl, pb) / pl);
+                    if (contrib.x == 0.0 && contrib.y == 0.0 && contrib.z == 0.0) continue;
+                    if (!world_trace(S, Ray{hit.p + kEps * wi, wi, ray.time}, tmax, true, false, best, stack, flags))
+                        L = L + contrib;
+                }
+            }
+            Bsdf unused;
+            mat_sample(mat, ray, hit, rng, unused);  // its draws
+        } while (!add_sample(P, sums, L));
+        store_pixel(P, x, row, sums, acc, acc_w, acc_sq);
+        n_samples = (unsigned long long)sums.n;
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        n_samples += __shfl_down_sync(0xffffffffu, n_samples, off);
-        n_closest += __shfl_down_sync(0xffffffffu, n_closest, off);
-        n_shadow += __shfl_down_sync(0xffffffffu, n_shadow, off);
-    }
-    if (lane == 0) {
-        atomicAdd(&counters[0], n_samples);
-        atomicAdd(&counters[1], n_closest);
-        atomicAdd(&counters[2], n_shadow);
-    }
+    count_rays(counters, n_samples, n_closest, n_shadow);
 }
 
 }  // namespace plain
 
 cudaError_t launch_plain(const PlainScene& S, const PlainParams& P, double* acc, double* acc_w, double* acc_sq,
                          unsigned long long* counters, int* flags, int sm_count, cudaStream_t stream) {
+    const plain::Tiles tiles = plain::tiles_of(P);
+    // One bounce among spheres under the sky, or nothing to hit at all.  With
+    // triangles or an env map k_paths is faster (512x512 x 8 spp at one bounce, ms,
+    // in k_paths / here: sphere scene 0.60 / 0.87, 5,120 triangles 1.55 / 8.1, 24
+    // spheres with a map 0.42 / 0.67, without 0.26 / 0.16).
+    if (P.max_bounces <= 0 || S.top_root == TPT_REF_NONE ||
+        (P.max_bounces == 1 && S.n_tris == 0 && S.env_kind != TPT_ENV_MAP)) {
+        const unsigned grid = (tiles.n_ids + 127u) / 128u;
+        plain::k_first_hits<<<grid, 128, 0, stream>>>(S, P, acc, acc_w, acc_sq, counters, flags);
+        return cudaGetLastError();
+    }
     // Short walks: one block of 256 per SM, whose warps share the most fetched
     // lines.  Past about a thousand triangles the warps' walks differ so much
     // in length that waiting for the slowest of 8 costs more than fetching for
     // 4, and two blocks of 128 are better (480x270 x 32 spp with 200 spheres
     // and 1,280 / 20,480 / 327,680 triangles, ms: 9.6 / 11.9 / 15.9 in blocks
     // of 256, 9.2 / 10.7 / 14.0 in blocks of 128; sphere scene 8.5 / 11.7).
-    const int block = S.n_tris < 1024 ? 256 : 128;
-    // 256 lanes per SM hold a pixel each.  A film of fewer pixels spreads them
+    // One bounce: a sample's shadow rays are its last, so it ends in their round
+    // and the next one's camera ray joins it (512x512 x 8 spp, ms: sphere scene
+    // 0.93 -> 0.65, 5,120 triangles 1.7 -> 1.56; with paths of several bounces the
+    // extra barrier costs 2 to 8%), and 384 lanes per SM hide more of the short
+    // chains' latency than 256 (0.65 -> 0.60).
+    const bool brief = P.max_bounces <= 1;
+    const int block = brief ? 192 : (S.n_tris < 1024 ? 256 : 128), ctas = brief ? 2 : 256 / block;
+    // 256 (384) lanes per SM hold a pixel each.  A film of fewer pixels spreads them
     // over the warps: a warp of a few lanes diverges less, and it is each
     // pixel's own chain of bounces that the render waits for (48x30 x 64 spp:
     // 7.5 ms in full warps, 4.6 spread).
-    const long long pixels = plain::tiles_of(P).n_ids;  // in whole tiles
-    const long long warps = (long long)sm_count * 8;
+    const long long pixels = tiles.n_ids;  // in whole tiles
+    const long long warps = (long long)sm_count * ctas * (block / 32);
     const unsigned lanes = (unsigned)std::min<long long>(32, std::max<long long>(1, (pixels + warps - 1) / warps));
     const long long per_block = (long long)lanes * (block / 32);
     const unsigned grid = (unsigned)std::min<long long>((pixels + per_block - 1) / per_block, warps * 32 / block);
-    if (block == 256) plain::k_paths<256><<<grid, 256, 0, stream>>>(S, P, acc, acc_w, acc_sq, counters, flags, lanes);
-    else plain::k_paths<128><<<grid, 128, 0, stream>>>(S, P, acc, acc_w, acc_sq, counters, flags, lanes);
+    auto launch = [&](auto kernel) {
+        kernel<<<grid, block, 0, stream>>>(S, P, acc, acc_w, acc_sq, counters, flags, lanes);
+    };
+    if (brief) launch(plain::k_paths<192, 2, true>);
+    else if (block == 256) launch(plain::k_paths<256, 1, false>);
+    else launch(plain::k_paths<128, 2, false>);
     return cudaGetLastError();
 }
 
