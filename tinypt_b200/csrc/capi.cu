@@ -502,7 +502,10 @@ void add_stats(tpt_stats& s, const WfCounters& hc, float ms) {
 // shared loop).
 constexpr long long kBatchAlonePaths = 16ll << 20;
 
-void batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, const Schedule& sc, int spp_div,
+// spp_div > 1: a trial of the autotuner, at that part of each job's spp.
+// Returns whether the jobs that share a render went through the bounce loop,
+// which is what the schedule's pool, refill and shading fields are about.
+bool batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, const Schedule& sc, int spp_div,
                   tpt_stats* stats) {
     if (n_jobs <= 0) throw TptError(TPT_ERR_INVALID, "no jobs");
     DeviceGuard device_guard(B.device);
@@ -511,8 +514,8 @@ void batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, con
     std::vector<WfJob> hj;
     hj.reserve((size_t)n_jobs);
     std::vector<int64_t> alone;
-    long long tasks = 0, pixels = 0;
-    int max_chunks = 1, max_task = 1, max_bounces = 0;
+    long long tasks = 0, pixels = 0, full_tasks = 0;
+    int max_chunks = 1, max_task = 1, max_bounces = 0, full_task = 1;
     for (int64_t k = 0; k < n_jobs; ++k) {
         const tpt_batch_job& j = jobs[k];
         tpt_render_config c = j.config;
@@ -528,6 +531,9 @@ void batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, con
             alone.push_back(k);
             continue;
         }
+        const int whole = std::min(sc.task_spp, c.spp);
+        full_tasks += (long long)c.width * film_rows(c) * ((c.spp + whole - 1) / whole);
+        full_task = std::max(full_task, whole);
         if (spp_div > 1) c.spp = std::max(1, c.spp / spp_div);
         const BatchScene& bs = B.scenes[(size_t)j.scene];
         hj.emplace_back();
@@ -599,7 +605,7 @@ void batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, con
             std::snprintf(buf, sizeof buf, "kernel raised device flags 0x%x", s.device_flags);
             throw TptError(TPT_ERR_DEVICE, buf);
         }
-        return;
+        return false;
     }
     if (tasks >= (1ll << 31)) throw TptError(TPT_ERR_UNSUPPORTED, "batch has more than 2^31 tasks");
     if (B.d_jobs_n < hj.size()) {
@@ -630,6 +636,9 @@ void batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, con
     p.queue_div = queue_div_setting();
     p.ordered_queue = env_int("TPT_QUEUE_ORDER", 1) != 0;
     p.shade_ctas = sc.shade_ctas;
+    // (decided at the jobs' own spp, so that a trial runs what the render will)
+    const bool one_kernel = p.tail_live < 0 && wf_one_kernel(full_tasks, full_task);
+    p.one_kernel = one_kernel ? 1 : -1;
     p.jobs = B.d_jobs;
     p.n_jobs = (int)hj.size();
     p.total_pixels = pixels;
@@ -646,6 +655,7 @@ void batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, con
         std::snprintf(buf, sizeof buf, "kernel raised device flags 0x%x", s.device_flags);
         throw TptError(TPT_ERR_DEVICE, buf);
     }
+    return !one_kernel;
 }
 
 }  // namespace
@@ -1172,13 +1182,16 @@ int tpt_batch_autotune(void* batch, const tpt_batch_job* jobs, int64_t n_jobs, t
         // were slower at the full spp); coordinate descent over the pool size,
         // the task length, the refill chunk, then the shading kernel's blocks
         // per SM.  Each coordinate skips the value it starts from: that
-        // schedule is the one best_ms was measured on.
+        // schedule is the one best_ms was measured on.  The pool, the refill
+        // chunk and the shading blocks are the bounce loop's: where the jobs
+        // run in one kernel, trials of them differ by noise and none is taken.
         const int div = 2;
         Schedule cur = schedule_of(nullptr);
         int trials = 0;
+        bool looped = false;
         auto trial = [&](const Schedule& sc) {
             tpt_stats st{};
-            batch_render(B, jobs, n_jobs, sc, div, &st);
+            looped = batch_render(B, jobs, n_jobs, sc, div, &st);
             if (trial_ms && trials < n_trials) trial_ms[trials] = st.render_ms;
             ++trials;
             return (double)st.render_ms;
@@ -1192,7 +1205,7 @@ int tpt_batch_autotune(void* batch, const tpt_batch_job* jobs, int64_t n_jobs, t
             Schedule sc = cur;
             sc.pool = pool;
             const double ms = trial(sc);
-            if (ms < best_ms) { best_ms = ms; cur = sc; }
+            if (looped && ms < best_ms) { best_ms = ms; cur = sc; }
         }
         const int tasks_spp[] = {4, 8, 16, 32};
         const int task0 = cur.task_spp;
@@ -1210,13 +1223,13 @@ int tpt_batch_autotune(void* batch, const tpt_batch_job* jobs, int64_t n_jobs, t
             Schedule sc = cur;
             sc.trace_chunk = ch;
             const double ms = trial(sc);
-            if (ms < best_ms) { best_ms = ms; cur = sc; }
+            if (looped && ms < best_ms) { best_ms = ms; cur = sc; }
         }
         {
             Schedule sc = cur;
             sc.shade_ctas = cur.shade_ctas == 8 ? 4 : 8;
             const double ms = trial(sc);
-            if (ms < best_ms) { best_ms = ms; cur = sc; }
+            if (looped && ms < best_ms) { best_ms = ms; cur = sc; }
         }
         best->pool_slots = (int32_t)cur.pool;
         best->task_spp = cur.task_spp;

@@ -2482,9 +2482,8 @@ cudaError_t reserve_pool(WfBuffers& B, WfParams& P, size_t part_tasks) {
 }
 }  // namespace
 
-namespace {
-// Whether a render of P.n_tasks tasks of up to P.task_spp samples runs in
-// k_paths alone.  Its divergent lanes trace 2 to 4 times slower than the
+// Whether a render of n_tasks tasks of up to task_spp samples runs in k_paths
+// alone.  Its divergent lanes trace 2 to 4 times slower than the
 // loop's kernels at full size, but the loop pays 0.7 to 1.3 ms for its graph
 // and some 25 launches, and once more per sample of a task.  Measured on one
 // B200, loop / direct, ms: 64x36 preview 0.70 / 0.09; 1-sample tasks, sphere
@@ -2495,8 +2494,14 @@ namespace {
 // 9.0 / 10.3; batches of 64 scenes 2.1 M samples 7.5 / 5.8, 4.3 M 9.4 / 9.6.  So
 // the line lies at 1.2 M samples of 1-sample tasks and 3.9 M of 8-sample ones.
 // A caller that sets the drain's handover (TPT_TAIL_SLOTS) asks for the loop.
+bool wf_one_kernel(long long n_tasks, int task_spp) {
+    return n_tasks * std::max(task_spp, 1) <= (task_spp + 2) * 393216LL;
+}
+
+namespace {
 bool direct_render(const WfParams& P) {
-    return P.tail_live < 0 && P.n_tasks * std::max(P.task_spp, 1) <= (P.task_spp + 2) * 393216LL;
+    if (P.tail_live >= 0) return false;
+    return P.one_kernel ? P.one_kernel > 0 : wf_one_kernel(P.n_tasks, P.task_spp);
 }
 
 // A render whose tasks all go to k_paths: no path state, no loop.  With camera

@@ -117,6 +117,8 @@ struct WfParams {
                                // bounce loop stops and k_paths runs each of them to the end (single,
                                // batch and adaptive-round renders; 0 = the loop drains the pool; -1 =
                                // the default, 262,144 but at most a sixteenth of the pool)
+    int one_kernel;            // 1 / -1: the render runs in k_paths / the bounce loop; 0: by its size
+                               // (wf_one_kernel)
     int ordered_queue;         // 1: the extension queue is rebuilt in slot order after every iteration
                                // (wf_launch_compact) and the kernels always take it
     // batch renders: the jobs (device memory); the other per-render fields
@@ -304,6 +306,10 @@ cudaError_t wf_cull_pixels(const WfScene& S, const WfParams& P, WfBuffers& B, cu
 size_t wf_compact_spans(size_t n_slots);
 cudaError_t wf_run_loop(const WfEnqueue& enqueue, const WfCounters* ctr, long long max_iters, cudaStream_t stream,
                         bool use_graph_loop);
+
+// Whether a render of n_tasks tasks of up to task_spp samples runs in one kernel
+// (k_paths) instead of the bounce loop, the drain's handover not being set.
+bool wf_one_kernel(long long n_tasks, int task_spp);
 
 // Allocation-free render (see the comment above wf_render_noalloc in
 // wavefront.cu): one kernel, counters in a file-scope device variable,
