@@ -13,6 +13,8 @@ translation unit gets the floating-point flags its numerics need:
   FMAs out): automatic contraction varied with each kernel instantiation's
   register budget, and batch films, single films and the adjoint must
   follow the same paths bit for bit;
+* ``env_guide.cu``: plain IEEE arithmetic, as the searches whose brackets it
+  makes;
 * ``host_scene.cu`` / ``capi.cu`` / ``image_io.cpp`` / ``scene_io.cpp`` /
   ``fp32_tree.cpp``: host
   code with ``-ffp-contract=off`` so the f64 scene quantities (camera basis,
@@ -42,6 +44,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=o
 UNITS = {
     "host_scene.cu": [],
     "capi.cu": [],
+    "env_guide.cu": [],
     "plain_f64.cu": ["-fmad=false"],
     "bvh_build.cu": ["-fmad=false"],
     "wavefront.cu": ["-fmad=false", "-ftz=true", "-prec-div=false", "-prec-sqrt=false"],

@@ -17,6 +17,7 @@
 #include "adjoint.cuh"
 #include "bvh_build.cuh"
 #include "checkpoint.hpp"
+#include "env_guide.cuh"
 #include "host_scene.hpp"
 #include "image_io.hpp"
 #include "plain_f64.cuh"
@@ -95,13 +96,18 @@ struct SceneHandle {
     }
 
     template <class T>
+    T* alloc(size_t n) {
+        void* p = nullptr;
+        ck(cudaMalloc(&p, n * sizeof(T)), "cudaMalloc(scene)");
+        allocs.push_back(p);
+        return static_cast<T*>(p);
+    }
+    template <class T>
     T* upload(const std::vector<T>& v) {
         if (v.empty()) return nullptr;
-        void* p = nullptr;
-        ck(cudaMalloc(&p, v.size() * sizeof(T)), "cudaMalloc(scene)");
-        allocs.push_back(p);
+        T* p = alloc<T>(v.size());
         ck(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, stream), "upload scene");
-        return static_cast<T*>(p);
+        return p;
     }
     ~SceneHandle() {
         if (stream) cudaStreamSynchronize(stream);
@@ -788,22 +794,26 @@ int tpt_scene_create(const tpt_scene_desc* desc, void** out_scene) {
         W.env_row = h->upload(fi.env_row_cdf);
         W.env_col = h->upload(fi.env_col_cdf);
         if (W.env_has_cdf) {
-            const size_t w = (size_t)hs.env_w, rows = (size_t)hs.env_h;
-            std::vector<uint16_t> row_guide, col_guide;
-            auto unit = [](size_t) { return 1.0f; };
-            W.env_row_k = guide_table(fi.env_row_cdf, 1, rows + 1, unit, row_guide);
-            W.env_col_k = guide_table(fi.env_col_cdf, rows, w + 1, unit, col_guide);
-            W.env_row_guide = h->upload(row_guide);
-            W.env_col_guide = h->upload(col_guide);
+            const size_t w1 = (size_t)hs.env_w + 1, rows = (size_t)hs.env_h;
+            auto table = [&](size_t n_rows, size_t n, int& k) -> uint16_t* {
+                k = guide_buckets(n);
+                return k ? h->alloc<uint16_t>(n_rows * (size_t)(k + 1)) : nullptr;
+            };
+            cudaError_t e = cudaSuccess;
+            auto make = [&](uint16_t* t, auto... args) {
+                if (t && e == cudaSuccess) e = make_guide(args..., t, h->stream);
+            };
+            uint16_t* t = nullptr;
+            make(t = table(1, rows + 1, W.env_row_k), W.env_row, 1, rows + 1);
+            W.env_row_guide = t;
+            make(t = table(rows, w1, W.env_col_k), W.env_col, rows, w1);
+            W.env_col_guide = t;
             // the f64 form's CDFs are not normalised: the kernel's row sums
-            std::vector<uint16_t> row_guide64, col_guide64;
-            const std::vector<double>& rc = pi.env_row_cdf;
-            P.env_row_k = guide_table(rc, 1, rows + 1, [&](size_t) { return hs.env_total; }, row_guide64);
-            P.env_col_k = guide_table(pi.env_col_cdf, rows, w + 1,
-                                      [&](size_t y) { return std::fmax(rc[y + 1] - rc[y], 0.0); }, col_guide64);
-            P.env_row_guide = h->upload(row_guide64);
-            P.env_col_guide = h->upload(col_guide64);
-            ck(cudaStreamSynchronize(h->stream), "env guide upload");
+            make(t = table(1, rows + 1, P.env_row_k), P.env_row_cdf, 1, rows + 1, (const double*)nullptr, hs.env_total);
+            P.env_row_guide = t;
+            make(t = table(rows, w1, P.env_col_k), P.env_col_cdf, rows, w1, P.env_row_cdf, 0.0);
+            P.env_col_guide = t;
+            ck(e, "env guide");
         }
         const CameraF64& c = hs.cam;
         W.cam.o = make_float3((float)c.o[0], (float)c.o[1], (float)c.o[2]);

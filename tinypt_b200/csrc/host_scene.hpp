@@ -138,29 +138,6 @@ struct Fp32Image {       // FP32 layout for the wavefront kernels
 };
 void flatten_fp32(const HostScene& hs, Fp32Image& img);
 
-// Starting brackets for searches of `rows` non-decreasing CDFs of n entries
-// each, for x = u * scale(row), u in [0, 1): for k = the power of two from n, at
-// most 1024, buckets of u, the largest lo in [0, n - 2] with cdf[lo] <= (j / k)
-// * scale (0 if none), j = 0 .. k.  Returns k, or 0 (no table) where an entry
-// would not fit 16 bits.
-template <class T, class Scale>
-int guide_table(const std::vector<T>& cdf, size_t rows, size_t n, Scale&& scale, std::vector<uint16_t>& guide) {
-    if (n < 2 || n > 65535) return 0;
-    size_t k = 1;
-    while (k < n && k < 1024) k *= 2;
-    guide.resize(rows * (k + 1));
-    for (size_t r = 0; r < rows; ++r) {
-        const T* c = &cdf[r * n];
-        const T s = scale(r);
-        size_t lo = 0;
-        for (size_t j = 0; j <= k; ++j) {
-            while (lo + 1 <= n - 2 && c[lo + 1] <= (T)j / (T)k * s) ++lo;
-            guide[r * (k + 1) + j] = (uint16_t)lo;
-        }
-    }
-    return (int)k;
-}
-
 // What the plain f64 kernel needs to walk the FP32 image's trees: per
 // triangle in their leaf order, its index in plain.tris and the node of
 // plain.nodes whose leaf range holds it; and the padding of the top-level

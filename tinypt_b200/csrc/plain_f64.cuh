@@ -28,7 +28,7 @@ struct PlainScene {
     const double* env_row_cdf;
     const double* env_col_cdf;
     double env_total;
-    // brackets of the two searches by the variate (guide_table; null: none)
+    // brackets of the two searches by the variate (make_guide; null: none)
     const uint16_t* env_row_guide;
     const uint16_t* env_col_guide;  // env_col_k + 1 per row
     int env_row_k, env_col_k;

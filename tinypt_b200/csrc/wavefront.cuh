@@ -49,7 +49,7 @@ struct WfScene {
     const float4* env_tex;     // rgb + nearest-texel pdf_uv
     const float* env_row;      // h+1, normalised
     const float* env_col;      // h*(w+1), normalised per row
-    // cdf_search's starting brackets (null: none), see guide_table
+    // cdf_search's starting brackets (null: none), see make_guide
     const uint16_t* env_row_guide;
     const uint16_t* env_col_guide;  // env_col_k + 1 per row
     int env_row_k, env_col_k;
