@@ -85,6 +85,41 @@ def test_directions_of_another_length(gpu, oracle_mod):
     assert 0.1 < lit.mean() < 0.9
 
 
+def _out_of_range(kind):
+    v, f = scenes.displaced_icosphere(2, 0.08, 3, 5)
+    v = np.array(v)
+    at = int(np.argmax(v[:, 2]))  # the vertex nearest the camera
+    if kind == "infinite vertex":
+        v[at] = [0.1, INF, 0.2]
+    elif kind == "nan vertex":
+        v[at] = [NAN, NAN, NAN]
+    elif kind == "nan in a vertex":
+        v[at, 1] = NAN
+    elif kind == "vertex at 1e200":
+        v[at] = [0.1, 0.2, -1e200]
+    mats = [Material.lambert(c) for c in ((0.8, 0.3, 0.2), (0.2, 0.3, 0.8), (0.3, 0.8, 0.3))]
+    s = Scene(Camera.look_at((0.0, 0.6, 4.0), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 45.0, W / H), World(), mats, None)
+    xf = {"flat transform": Transform.scale((1.0, 0.0, 1.0)), "nan transform": Transform.translate((NAN, 0.0, 0.0)),
+          "infinite transform": Transform.translate((0.0, INF, 0.0))}
+    s.world.meshes.append(Mesh.from_arrays(v, f, 0))
+    s.world.instances.append(Instance(0, Transform.translate((0.1, 0.0, 0.0)), None))
+    if kind in xf:
+        s.world.instances.append(Instance(0, xf[kind], 1))
+    s.world.spheres += [Sphere((1.2, 0.0, 0.0), 0.5, 1), Sphere((-1.4, 0.0, 0.0), 0.5, 2)]
+    ball = {"nan sphere": ((NAN, 0.0, 0.0), 0.5), "infinite sphere": ((0.0, INF, 0.0), 0.5), "nan radius": ((0.0, -1.0, 0.0), NAN),
+            "infinite radius": ((0.0, -1.0, 0.0), INF), "negative radius": ((0.0, 1.0, 0.0), -0.4)}
+    if kind in ball:
+        s.world.spheres.insert(1, Sphere(*ball[kind], 2))
+    return s
+
+
+@pytest.mark.parametrize("kind", [
+    "usual", "infinite vertex", "nan vertex", "nan in a vertex", "vertex at 1e200", "flat transform", "nan transform",
+    "infinite transform", "nan sphere", "infinite sphere", "nan radius", "infinite radius", "negative radius"])
+def test_geometry_out_of_range(gpu, oracle_mod, kind):
+    _same_as_oracle(oracle_mod, _out_of_range(kind))
+
+
 @pytest.mark.parametrize("mode", [WF, PLAIN])
 @pytest.mark.parametrize("albedos", [(-1e200, -1e200), (1e29, 1e300)])
 def test_black_map_with_overflowing_albedo(gpu, mode, albedos):

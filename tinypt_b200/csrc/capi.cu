@@ -755,8 +755,11 @@ int tpt_scene_create(const tpt_scene_desc* desc, void** out_scene) {
         PlainScene& P = h->plain;
         std::vector<int2> links;
         float top_pad = 0.0f;
-        std::future<void> linked = std::async(std::launch::async | std::launch::deferred,
-                                              [&] { link_plain(pi, fi, links, top_pad); });
+        bool by_loops = false;
+        std::future<void> linked = std::async(std::launch::async | std::launch::deferred, [&] {
+            link_plain(pi, fi, links, top_pad);
+            by_loops = geometry_out_of_range(hs);
+        });
         P.nodes = h->upload(pi.nodes);
         P.tris = h->upload(pi.tris);
         P.meshes = h->upload(pi.meshes);
@@ -841,6 +844,7 @@ int tpt_scene_create(const tpt_scene_desc* desc, void** out_scene) {
         P.top_root = W.top_root;
         linked.get();
         P.top_pad = top_pad;
+        P.by_loops = by_loops;
         P.links = h->upload(links);
         P.n_tris = (int)links.size();
         ck(cudaStreamSynchronize(h->stream), "scene upload");

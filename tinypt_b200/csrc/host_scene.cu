@@ -779,6 +779,17 @@ void flatten_fp32(const HostScene& hs, Fp32Image& img) {
     }
 }
 
+bool geometry_out_of_range(const HostScene& hs) {
+    auto bad = [](double x) { return !(std::fabs(x) <= 1e30); };
+    for (const HostScene::Mesh& m : hs.meshes)
+        if (std::any_of(m.pos.begin(), m.pos.end(), bad)) return true;
+    for (const tpt_sphere& s : hs.spheres)
+        if (std::any_of(s.center, s.center + 3, bad) || bad(s.radius)) return true;
+    for (const InstanceF64& x : hs.instances)
+        if (std::any_of(x.a, x.a + 9, bad) || std::any_of(x.t, x.t + 3, bad)) return true;
+    return false;
+}
+
 void link_plain(const PlainImage& plain, const Fp32Image& fp, std::vector<int2>& links, float& top_pad) {
     const size_t n = plain.tris.size();
     links.resize(n);

@@ -144,6 +144,10 @@ void flatten_fp32(const HostScene& hs, Fp32Image& img);
 // boxes, 2^-20 of the largest coordinate in them.
 void link_plain(const PlainImage& plain, const Fp32Image& fp, std::vector<int2>& links, float& top_pad);
 
+// True when a vertex, sphere or transform is not a number or beyond 1e30: what
+// the reference's tests then say depends on the order it asks in.
+bool geometry_out_of_range(const HostScene& hs);
+
 // Several scenes in one set of device arrays for batch renders: the FP32
 // images and the f64 light/instance/sphere tables of each scene appended,
 // every index rebased (BVH node and leaf references, material ids, mesh

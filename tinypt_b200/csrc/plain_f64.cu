@@ -243,11 +243,12 @@ __device__ __forceinline__ bool unusual(const Ray& r) {
     const float dx = (float)r.d.x, dy = (float)r.d.y, dz = (float)r.d.z;
     return !(fabsf(dx * dx + dy * dy + dz * dz - 1.0f) < 1e-6f && fabsf(ox + oy + oz) < 1e30f);
 }
-// World::hit by the reference's own loops, for unusual rays.  Every comparison
-// of the reference's tests lets a NaN pass, so such a ray meets the last
-// sphere; which one that is only the order of its loop says.  And instances
-// count at dot(p - o, d), spheres at their root: only for a unit direction does
-// a box that starts past the one hold no closer other.
+// World::hit by the reference's own loops, for unusual rays and for scenes with
+// geometry out of range.  Every comparison of the reference's tests lets a NaN
+// pass, so a NaN ray meets the last sphere and a NaN triangle stops the rays that
+// come to its leaf; which ones these are only the order of its loops says.  And
+// instances count at dot(p - o, d), spheres at their root: only for a unit
+// direction does a box that starts past the one hold no closer other.
 __device__ __noinline__ Best world_loops(const PlainScene& S, V ro, V rd, double time, double tmax, int* flags) {
     const Ray r{ro, rd, time};
     Best best{tmax, 0.0, -1, -1};
@@ -949,7 +950,7 @@ __global__ void __launch_bounds__(BLOCK, CTAS) k_paths(const __grid_constant__ P
                     if (job == kJobArea) tmax = area_t;
                 }
                 Best b;
-                const bool h = world_trace(S, r, tmax, job != kJobClosest, job == kJobClosest && odd, b, stack, flags);
+                const bool h = world_trace(S, r, tmax, job != kJobClosest, S.by_loops || (job == kJobClosest && odd), b, stack, flags);
                 if (job == kJobClosest) {
                     best = b;
                     found = h;
@@ -1097,7 +1098,7 @@ __global__ void __launch_bounds__(128, 3) k_first_hits(const __grid_constant__ P
             if (P.max_bounces <= 0) continue;
             ++n_closest;
             Best best;
-            if (!world_trace(S, ray, kTMax, false, unusual(ray), best, stack, flags)) {
+            if (!world_trace(S, ray, kTMax, false, S.by_loops || unusual(ray), best, stack, flags)) {
                 double unused;
                 L = L + clamp_lum(has_env ? env_at(S, ray.d, false, unused) : sky(ray.d), 50.0);
                 continue;
@@ -1142,7 +1143,7 @@ __global__ void __launch_bounds__(128, 3) k_first_hits(const __grid_constant__ P
                     mat_eval(mat, wo, wi, nrm, f, pb);
                     const V contrib = had(had(beta, f), li) * (cs * mis(pl, pb) / pl);
                     if (contrib.x == 0.0 && contrib.y == 0.0 && contrib.z == 0.0) continue;
-                    if (!world_trace(S, Ray{hit.p + kEps * wi, wi, ray.time}, tmax, true, false, best, stack, flags))
+                    if (!world_trace(S, Ray{hit.p + kEps * wi, wi, ray.time}, tmax, true, S.by_loops != 0, best, stack, flags))
                         L = L + contrib;
                 }
             }

@@ -41,6 +41,7 @@ struct PlainScene {
     const int2* links;
     int n_tris;
     int top_root;
+    int by_loops;              // geometry_out_of_range: every ray takes the reference's loops
     float top_pad;             // widens the top-level boxes: far above the f64 error of a sphere test
 };
 
