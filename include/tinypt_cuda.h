@@ -163,7 +163,9 @@ typedef struct tpt_stats {
     double   render_ms;         /* device time of the render (CUDA events)     */
     uint64_t paths;             /* camera samples finished (sum of acc_w)      */
     uint64_t rays_closest;      /* closest-hit traces: camera + extension      */
-    uint64_t rays_shadow;       /* occlusion traces (NEE shadow rays)          */
+    uint64_t rays_shadow;       /* NEE shadow rays.  FP32: those traced; f64: those
+                                   the reference traces -- where the light adds
+                                   exactly zero this library does not walk     */
     uint64_t iterations;        /* wavefront iterations (0 for PLAIN_F64 and for
                                    small renders, which run in one kernel)   */
     int32_t  device_flags;      /* TPT_FLAG_* raised by kernels                */
@@ -340,8 +342,9 @@ typedef struct tpt_tuning {
     int32_t pool_slots;         /* paths in flight (default 64 Mi)            */
     int32_t task_spp;           /* samples per pool task (default 8)          */
     int32_t trace_chunk;        /* leaf visits between lane refills (def. 16) */
-    int32_t shade_ctas;         /* resident blocks per SM the shading kernel is
-                                   compiled for: 4 or 8 (default 8)          */
+    int32_t shade_ctas;         /* register budget of the shading kernel, in blocks
+                                   of 128 threads resident per SM: 4 or 8 (2 or
+                                   4 of its blocks of 256; default 8)        */
 } tpt_tuning;
 
 /* Builds every scene's BVHs and uploads them merged (one handle). */

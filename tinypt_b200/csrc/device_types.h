@@ -63,7 +63,7 @@ __host__ __device__ inline int32_t make_leaf_ref(uint32_t start, uint32_t count)
 }
 
 // Interior node of the flattened BVH2: the boxes of both children, so one
-// 64-byte visit (four 16-byte loads) decides the traversal order.
+// 64-byte visit (two 32-byte loads) decides the traversal order.
 //   lx = (c0.min.x, c0.max.x, c0.min.y, c0.max.y)
 //   rx = (c1.min.x, c1.max.x, c1.min.y, c1.max.y)
 //   zz = (c0.min.z, c0.max.z, c1.min.z, c1.max.z)

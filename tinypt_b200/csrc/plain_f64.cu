@@ -199,8 +199,11 @@ __device__ __forceinline__ Ray32 ray32(V o, V d, float pad) {
     set_axis(o.z, d.z, pad, r.idir.z, r.near_off.z, r.far_off.z);
     return r;
 }
-// Entry distance of the widened box; *hit = false only when no f64 test in
-// the box can succeed below tmax (a NaN keeps the box).
+// Entry distance of the widened box; *hit = false only when no point of the
+// box lies on the ray below tmax (a NaN keeps the box).  That no f64 test in the
+// box succeeds then rests on the hits lying in their boxes: a triangle's by its
+// box's 1e-9 and the widening here, which a ray within about 1e-9 of the
+// triangle's plane (det near its bound of 1e-10) may pass by at an edge.
 __device__ __forceinline__ float box32(const Ray32& r, float x0, float x1, float y0, float y1, float z0, float z1,
                                        float tmax, bool* hit) {
     const bool sx = r.idir.x < 0.0f, sy = r.idir.y < 0.0f, sz = r.idir.z < 0.0f;

@@ -19,8 +19,10 @@
 //
 // Slots are visited in slot order (an active byte per slot); shadow records
 // and pending completions go through queues filled with warp-aggregated
-// atomics.  The iterations run inside one CUDA graph whose WHILE
-// conditional node is re-armed on the device until no slot is active.
+// atomics.  The first iterations are launched from the host; a loop that goes on
+// runs in one CUDA graph whose WHILE conditional node is re-armed on the device
+// until no slot is active.  Small renders have no loop: k_paths runs their paths
+// whole.
 #include "fp32_device.cuh"
 
 #include <algorithm>
@@ -2483,16 +2485,22 @@ cudaError_t reserve_pool(WfBuffers& B, WfParams& P, size_t part_tasks) {
 }  // namespace
 
 // Whether a render of n_tasks tasks of up to task_spp samples runs in k_paths
-// alone.  Its divergent lanes trace 2 to 4 times slower than the
-// loop's kernels at full size, but the loop pays 0.7 to 1.3 ms for its graph
-// and some 25 launches, and once more per sample of a task.  Measured on one
-// B200, loop / direct, ms: 64x36 preview 0.70 / 0.09; 1-sample tasks, sphere
-// scene and mesh scene of 81,920 triangles: 36,864 tasks 0.81 / 0.16 and 1.46
-// / 0.38, 524,288 0.96 / 0.41 and 1.74 / 0.89, 2,097,152 1.48 / 1.23 and 2.35 /
-// 2.66, 4,194,304 2.11 / 2.23 and 2.94 / 4.57; 8-sample tasks: 1 Mi samples
-// 2.6 / 0.9 and 6.5 / 2.6, 4.7 M 3.7 / 2.8 and 7.8 / 6.6, 8.4 M 5.0 / 4.5 and
-// 9.0 / 10.3; batches of 64 scenes 2.1 M samples 7.5 / 5.8, 4.3 M 9.4 / 9.6.  So
-// the line lies at 1.2 M samples of 1-sample tasks and 3.9 M of 8-sample ones.
+// alone.  Its divergent lanes trace 2 to 4 times slower than the loop's kernels
+// at full size, but the loop's some 25 launches and waits cost 0.3 to 1 ms, and
+// once more per sample of a task.  So the line is one of tasks: some 390,000,
+// three times as many of one sample, which pay the loop once.  Measured on one
+// B200, loop / direct, ms, sphere scene; mesh scene of 81,920 triangles; Cornell box
+// with glass:
+//   1-sample tasks    36,864   0.44 / 0.14   0.98 / 0.32   1.19 / 0.34
+//                  1,179,648   0.84 / 0.60   1.86 / 1.41   2.55 / 2.85  (last direct)
+//                  2,097,152   1.09 / 0.97   2.12 / 2.18   3.45 / 4.80
+//   8-sample         131,072   2.89 / 0.82   6.33 / 2.23   7.49 / 3.15
+//                    491,520   3.84 / 2.23   7.51 / 5.70   10.4 / 9.69  (last direct)
+//                  1,048,576   5.05 / 3.98   9.01 / 9.67   15.5 / 19.5
+//   64-sample        360,000   19.8 / 10.0   48.3 / 27.7   64.4 / 53.1
+//   256-sample       262,144   70.5 / 28.7    180 / 88.5    226 / 156
+// Batches of 64 small scenes, 8-sample tasks, two sets: 2.0 M samples 8.6 / 5.4 and
+// 8.7 / 6.4, 3.7 M 10.7 / 8.7 and 10.4 / 8.7, 6.5 M 13.4 / 13.4.
 // A caller that sets the drain's handover (TPT_TAIL_SLOTS) asks for the loop.
 bool wf_one_kernel(long long n_tasks, int task_spp) {
     return n_tasks * std::max(task_spp, 1) <= (task_spp + 2) * 393216LL;
