@@ -359,11 +359,12 @@ void tpt_batch_destroy(void* batch);
 int tpt_batch_render_device(void* batch, const tpt_batch_job* jobs, int64_t n_jobs,
                             const tpt_tuning* tuning, tpt_stats* stats);
 
-/* Autotuner: times short renders of the same jobs at reduced spp over a
- * set of schedules (pool size, then task length, then refill chunk, each
- * chosen with the others fixed, then the shading variant; 13 trials at
+/* Autotuner: times renders of the same jobs, large batches at reduced spp,
+ * over a set of schedules (pool size, then task length, then refill chunk,
+ * each chosen with the others fixed, then the shading variant; 13 trials at
  * most, a warm-up included) and writes the fastest to *best (jobs that
- * render alone take their own schedule in every trial);
+ * render alone take their own schedule in every trial; pool, chunk and
+ * shading variant keep their defaults where the jobs run in one kernel);
  * trial_ms (nullable, n_trials entries) receives each trial's time.
  * Returns the number of trials run, or a negative error code. */
 int tpt_batch_autotune(void* batch, const tpt_batch_job* jobs, int64_t n_jobs,

@@ -521,8 +521,8 @@ bool batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, con
     std::vector<WfJob> hj;
     hj.reserve((size_t)n_jobs);
     std::vector<int64_t> alone;
-    long long tasks = 0, pixels = 0, full_tasks = 0;
-    int max_chunks = 1, max_task = 1, max_bounces = 0, full_task = 1;
+    long long tasks = 0, pixels = 0;
+    int max_chunks = 1, max_task = 1, max_bounces = 0;
     for (int64_t k = 0; k < n_jobs; ++k) {
         const tpt_batch_job& j = jobs[k];
         tpt_render_config c = j.config;
@@ -538,9 +538,6 @@ bool batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, con
             alone.push_back(k);
             continue;
         }
-        const int whole = std::min(sc.task_spp, c.spp);
-        full_tasks += (long long)c.width * film_rows(c) * ((c.spp + whole - 1) / whole);
-        full_task = std::max(full_task, whole);
         if (spp_div > 1) c.spp = std::max(1, c.spp / spp_div);
         const BatchScene& bs = B.scenes[(size_t)j.scene];
         hj.emplace_back();
@@ -643,9 +640,7 @@ bool batch_render(BatchHandle& B, const tpt_batch_job* jobs, int64_t n_jobs, con
     p.queue_div = queue_div_setting();
     p.ordered_queue = env_int("TPT_QUEUE_ORDER", 1) != 0;
     p.shade_ctas = sc.shade_ctas;
-    // (decided at the jobs' own spp, so that a trial runs what the render will)
-    const bool one_kernel = p.tail_live < 0 && wf_one_kernel(full_tasks, full_task);
-    p.one_kernel = one_kernel ? 1 : -1;
+    const bool one_kernel = p.tail_live < 0 && wf_one_kernel(p.n_tasks, p.task_spp);
     p.jobs = B.d_jobs;
     p.n_jobs = (int)hj.size();
     p.total_pixels = pixels;
@@ -749,14 +744,15 @@ int tpt_scene_create(const tpt_scene_desc* desc, void** out_scene) {
         Fp32Image fi;
         flatten_fp32(hs, fi);
         if (fi.max_stack > 64) throw TptError(TPT_ERR_UNSUPPORTED, "BVH deeper than the 64-entry traversal stack");
-        // The f64 form's links, beside the uploads (1.31 M triangles: 45 ms of a
-        // second on their own).  Declared after what it reads and writes: an
-        // exception waits for it first.
+        // The f64 form's links, beside the uploads where they take longer than a
+        // thread does to start (1.31 M triangles: 45 ms of a second on their own).
+        // Declared after what it reads and writes: an exception waits for it first.
         PlainScene& P = h->plain;
         std::vector<int2> links;
         float top_pad = 0.0f;
         bool by_loops = false;
-        std::future<void> linked = std::async(std::launch::async | std::launch::deferred, [&] {
+        const std::launch beside = std::launch::async | std::launch::deferred;
+        std::future<void> linked = std::async(pi.tris.size() > 8192 ? beside : std::launch::deferred, [&] {
             link_plain(pi, fi, links, top_pad);
             by_loops = geometry_out_of_range(hs);
         });
@@ -1197,17 +1193,24 @@ int tpt_batch_autotune(void* batch, const tpt_batch_job* jobs, int64_t n_jobs, t
     return guarded([&] {
         if (!batch || !jobs || !best) throw TptError(TPT_ERR_INVALID, "null argument");
         BatchHandle& B = *static_cast<BatchHandle*>(batch);
-        long long total_tasks = 0;
-        for (int64_t k = 0; k < n_jobs; ++k)
-            total_tasks += (long long)jobs[k].config.width * jobs[k].config.height;
-        // Trials at half of each job's spp (a quarter picked schedules that
-        // were slower at the full spp); coordinate descent over the pool size,
-        // the task length, the refill chunk, then the shading kernel's blocks
-        // per SM.  Each coordinate skips the value it starts from: that
-        // schedule is the one best_ms was measured on.  The pool, the refill
-        // chunk and the shading blocks are the bounce loop's: where the jobs
-        // run in one kernel, trials of them differ by noise and none is taken.
-        const int div = 2;
+        long long total_tasks = 0, half_samples = 0;
+        for (int64_t k = 0; k < n_jobs; ++k) {
+            const tpt_render_config& c = jobs[k].config;
+            total_tasks += (long long)c.width * c.height;
+            half_samples += (long long)c.width * film_rows(c) * (c.spp / 2);
+        }
+        // Trials at half of each job's spp (a quarter picked schedules that were
+        // slower at the full spp), but whole ones where half the batch might run
+        // in one kernel and the batch not: 64 small scenes of 2.1 M samples take
+        // 3.2 ms at half their spp in 8-sample tasks and 4.7 in 4-sample ones,
+        // which the loop runs, but 5.5 and 4.9 whole.  Coordinate descent over
+        // the pool size, the task length, the refill chunk, then the shading
+        // kernel's register budget.  Each coordinate skips the value it starts
+        // from: that schedule is the one best_ms was measured on.  The pool, the
+        // refill chunk and the budget are the bounce loop's: where the jobs run
+        // in one kernel, trials of them differ by noise and none is taken.
+        const int tasks_spp[] = {4, 8, 16, 32};
+        const int div = wf_one_kernel(half_samples / tasks_spp[3], tasks_spp[3]) ? 1 : 2;
         Schedule cur = schedule_of(nullptr);
         int trials = 0;
         bool looped = false;
@@ -1229,7 +1232,6 @@ int tpt_batch_autotune(void* batch, const tpt_batch_job* jobs, int64_t n_jobs, t
             const double ms = trial(sc);
             if (looped && ms < best_ms) { best_ms = ms; cur = sc; }
         }
-        const int tasks_spp[] = {4, 8, 16, 32};
         const int task0 = cur.task_spp;
         for (int ts : tasks_spp) {
             if (ts == task0) continue;

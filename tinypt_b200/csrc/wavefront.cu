@@ -2507,10 +2507,7 @@ bool wf_one_kernel(long long n_tasks, int task_spp) {
 }
 
 namespace {
-bool direct_render(const WfParams& P) {
-    if (P.tail_live >= 0) return false;
-    return P.one_kernel ? P.one_kernel > 0 : wf_one_kernel(P.n_tasks, P.task_spp);
-}
+bool direct_render(const WfParams& P) { return P.tail_live < 0 && wf_one_kernel(P.n_tasks, P.task_spp); }
 
 // A render whose tasks all go to k_paths: no path state, no loop.  With camera
 // culling on, one thread per pixel classifies the film first (k_paths reads

@@ -117,8 +117,6 @@ struct WfParams {
                                // bounce loop stops and k_paths runs each of them to the end (single,
                                // batch and adaptive-round renders; 0 = the loop drains the pool; -1 =
                                // the default, 262,144 but at most a sixteenth of the pool)
-    int one_kernel;            // 1 / -1: the render runs in k_paths / the bounce loop; 0: by its size
-                               // (wf_one_kernel)
     int ordered_queue;         // 1: the extension queue is rebuilt in slot order after every iteration
                                // (wf_launch_compact) and the kernels always take it
     // batch renders: the jobs (device memory); the other per-render fields
