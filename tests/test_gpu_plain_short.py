@@ -1,17 +1,17 @@
-"""The plain f64 form's kernels for short paths: renders of at most one bounce
-and scenes without primitives.
+"""The plain f64 form's kernels beside the general one.
 
-Spheres under the sky run in a kernel of their own; a triangle that no ray
+Scenes of spheres alone run in a kernel of their own; a triangle that no ray
 meets sends the same render to the general kernel, whose film must be the same
-bit for bit.  One bounce among triangles or under an env map ends its samples
-earlier in the general kernel; those films are compared with the oracle."""
+bit for bit.  One bounce among triangles ends its samples earlier in the
+general kernel; those films are compared with the oracle."""
 import numpy as np
 import pytest
 
 from tinypt_b200 import _abi, scenes
 from tinypt_b200.render import DeviceScene
-from tinypt_b200.scene import Camera, Instance, Mesh, RenderConfig, Scene, Transform, World
+from tinypt_b200.scene import Camera, EnvMap, Instance, Material, Mesh, RenderConfig, Scene, Sphere, Transform, World
 from tests.parity_util import small_mesh_env_scene
+from tests.test_gpu_plain_walk import coincident_spheres
 
 pytestmark = pytest.mark.gpu
 
@@ -22,10 +22,21 @@ def _empty(w, h, env=None):
     return Scene(Camera.look_at((0.0, 0.0, 1.5), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 45.0, w / h), World(), [], env)
 
 
+def _spheres(w, h, n, env):
+    """n spheres of every material, one of them a light."""
+    rng = np.random.default_rng(n)
+    s = _empty(w, h, env)
+    s.mats = [Material.lambert((0.7, 0.5, 0.3)), Material.metal((0.8, 0.8, 0.8)), Material.dielectric(1.5, (0.1, 0.2, 0.3)),
+              Material.ggx((0.8, 0.6, 0.4), 0.2), Material.subsurface((0.8, 0.7, 0.6), 0.05), Material.diffuse_light((8.0, 7.0, 5.0))]
+    for k in range(n):
+        s.world.spheres.append(Sphere(tuple(rng.uniform((-2.0, -1.5, -4.0), (2.0, 1.5, -0.5))), float(rng.uniform(0.05, 0.5)), k % 6))
+    return s
+
+
 def _out_of_sight(s):
     """A triangle of 1e-30 that no ray comes near."""
     p = np.array([[0.0, 0.0, 0.0], [1e-30, 0.0, 0.0], [0.0, 1e-30, 0.0]])
-    s.mats = list(s.mats) or [scenes.Material.lambert((0.5, 0.5, 0.5))]
+    s.mats = list(s.mats) or [Material.lambert((0.5, 0.5, 0.5))]
     s.world.meshes.append(Mesh.from_arrays(p, np.array([[0, 1, 2]]), 0))
     s.world.instances.append(Instance(len(s.world.meshes) - 1, Transform.translate((0.0, 1e6, 0.0)), None))
     return s
@@ -54,6 +65,13 @@ def _cfg(w, h, spp, depth, rr=3, **kw):
     (lambda: scenes.build_scene(48, 32), _cfg(48, 32, 64, 1, adaptive_enabled=True, adaptive_min_spp=4, adaptive_threshold=0.3)),
     (lambda: scenes.build_scene(1, 1), _cfg(1, 1, 7, 1)),
     (lambda: scenes.build_scene(301, 203), _cfg(301, 203, 2, 1)),
+    (lambda: scenes.build_scene(61, 37), _cfg(61, 37, 5, 8)),
+    (lambda: scenes.build_scene(61, 37), _cfg(61, 37, 5, 20, rr=0)),
+    (lambda: _spheres(61, 37, 1, scenes.sky_env(16, 8)), _cfg(61, 37, 5, 8)),
+    (lambda: _spheres(61, 37, 60, scenes.sky_env(17, 9)), _cfg(61, 37, 5, 8, rr=1)),
+    (lambda: _spheres(61, 37, 255, None), _cfg(61, 37, 5, 8)),
+    (lambda: _spheres(61, 37, 60, EnvMap.constant((0.0, 0.0, 0.0))), _cfg(61, 37, 5, 8)),
+    (lambda: coincident_spheres(47, 31), _cfg(47, 31, 4, 6)),
     (lambda: _empty(61, 37), _cfg(61, 37, 5, 8)),
     (lambda: _empty(61, 37, scenes.sky_env(16, 8)), _cfg(61, 37, 5, 8)),
     (lambda: _empty(5, 3, scenes.sky_env(16, 8)), _cfg(5, 3, 5, 1)),

@@ -271,6 +271,19 @@ __device__ __noinline__ Best world_loops(const PlainScene& S, V ro, V rd, double
     return best;
 }
 
+// World::hit in a scene of spheres alone: the reference's loop over them.
+__device__ __forceinline__ bool spheres_hit(const PlainScene& S, const Ray& r, double tmax, bool any, Best& best) {
+    best = Best{tmax, 0.0, -1, -1};
+#pragma unroll 1
+    for (int i = 0; i < S.n_spheres; ++i) {
+        double t;
+        if (!sphere_test(ld(S.spheres[i].c), S.spheres[i].r, r, kEps, best.t, t)) continue;
+        best = Best{t, 0.0, -1, i};
+        if (any) return true;
+    }
+    return best.prim >= 0;
+}
+
 constexpr int kLeaveMesh = ~0;  // stack entry: back to world space (no leaf of a tree has the code 0 / 0)
 
 // World::hit over the top-level tree (spheres and instances) and the mesh
@@ -1076,11 +1089,13 @@ __global__ void __launch_bounds__(BLOCK, CTAS) k_paths(const __grid_constant__ P
     count_rays(counters, n_samples, n_closest, n_shadow);
 }
 
-// Paths that are all alike and all short (launch_plain): a lane per pixel runs
-// them sample after sample.  Where nothing diverges k_paths' rounds only add to
-// the latency of a sample's chain: empty scene 960x540 x 16 spp 0.55 ms in
-// k_paths, 0.27 here, built-in scene at one bounce 1280x720 x 4 spp 1.15 and 0.51.
-__global__ void __launch_bounds__(128, 3) k_first_hits(const __grid_constant__ PlainScene S,
+// Scenes of spheres alone (launch_plain): a lane per pixel runs its samples, and
+// each sample's path, to the end.  Bound by f64 latency at 12 warps per SM.  The
+// loop over the spheres is the same for every lane and the code without trees
+// short, so that k_paths' steps only add to each sample's chain: built-in scene
+// 1280x720 x 4 spp 2.75 ms in k_paths, 2.27 here, at one bounce 1.15 and 0.49, empty
+// scene 960x540 x 16 spp 0.55 and 0.24.
+__global__ void __launch_bounds__(128, 3) k_pixels(const __grid_constant__ PlainScene S,
                                                        const __grid_constant__ PlainParams P, double* __restrict__ acc,
                                                        double* __restrict__ acc_w, double* __restrict__ acc_sq,
                                                        unsigned long long* __restrict__ counters, int* flags) {
@@ -1090,68 +1105,76 @@ __global__ void __launch_bounds__(128, 3) k_first_hits(const __grid_constant__ P
     const double inv_w = 1.0 / (double)P.width, inv_h = 1.0 / (double)P.height;
     int x = 0, row = 0;
     unsigned long long n_samples = 0, n_closest = 0, n_shadow = 0;
-    int stack[kStack];
     if (id < T.n_ids && tile_pixel(T, P, id, x, row)) {
         uint64_t rng = pixel_seed((uint32_t)x, (uint32_t)(P.row_begin + row * P.row_step), P.seed);
         Sums sums{};
         V L;
         do {
-            const Ray ray = sample_ray(S, P, x, row, inv_w, inv_h, rng);
-            L = mk(0, 0, 0);
-            if (P.max_bounces <= 0) continue;
-            ++n_closest;
-            Best best;
-            if (!world_trace(S, ray, kTMax, false, S.by_loops || unusual(ray), best, stack, flags)) {
-                double unused;
-                L = L + clamp_lum(has_env ? env_at(S, ray.d, false, unused) : sky(ray.d), 50.0);
-                continue;
-            }
+            Ray ray = sample_ray(S, P, x, row, inv_w, inv_h, rng);
             V beta = mk(1, 1, 1);
-            if (P.rr_start <= 0) {
-                const double p = 0.95;  // of the largest channel, 1
-                if (pcg_f64(rng) > p) continue;
-                beta = beta / p;
-            }
-            const Hit hit = hit_of(S, ray, best);
-            const MaterialF64& mat = S.mats[hit.mat];
-            if (mat.kind == TPT_MAT_DIFFUSE_LIGHT) {
-                L = L + clamp_lum(had(beta, ld(mat.c)), 50.0);
-                continue;
-            }
-            if (mat.kind != TPT_MAT_METAL && mat.kind != TPT_MAT_DIELECTRIC) {
-                const V nrm = dot(hit.n, ray.d) < 0.0 ? hit.n : -hit.n, wo = norm(-ray.d);
-                // nee_environment (:148-172), then nee_area_light (:178-213)
+            double last_pdf = 0.0;
+            bool last_nd = false;
+            L = mk(0, 0, 0);
 #pragma unroll 1
-                for (int k = has_env ? 0 : 1; k < 2; ++k) {
-                    V wi, li;
-                    double pl, tmax = kTMax;
-                    if (k == 0) {
-                        const bool by_cdf = env_sample_dir(S, rng, wi);
-                        pl = 1.0 / (4.0 * kPi);
-                        li = env_at(S, wi, by_cdf, pl);
-                    } else {
-                        V lp, ln;
-                        if (!sample_light(S, rng, ray.time, hit.p, lp, ln, li, pl)) continue;
-                        const V tl = lp - hit.p;
-                        const double dist = sqrt(dot(tl, tl));
-                        if (!(dist > 1e-6)) continue;
-                        wi = tl / dist;
-                        tmax = fmax(dist - kEps, kEps);
-                    }
-                    const double cs = fmax(dot(nrm, wi), 0.0);
-                    if (!(cs > 0.0) || (k == 0 && !(pl > 0.0))) continue;
-                    ++n_shadow;
-                    V f;
-                    double pb;
-                    mat_eval(mat, wo, wi, nrm, f, pb);
-                    const V contrib = had(had(beta, f), li) * (cs * mis(pl, pb) / pl);
-                    if (contrib.x == 0.0 && contrib.y == 0.0 && contrib.z == 0.0) continue;
-                    if (!world_trace(S, Ray{hit.p + kEps * wi, wi, ray.time}, tmax, true, S.by_loops != 0, best, stack, flags))
-                        L = L + contrib;
+            for (int bounce = 0; bounce < P.max_bounces; ++bounce) {
+                ++n_closest;
+                Best best;
+                if (!spheres_hit(S, ray, kTMax, false, best)) {
+                    double pe = 1.0 / (4.0 * kPi);
+                    V contrib = had(beta, has_env ? env_at(S, ray.d, last_nd, pe) : sky(ray.d));
+                    if (has_env && last_nd) contrib = contrib * mis(last_pdf, pe);
+                    L = L + clamp_lum(contrib, 50.0);
+                    break;
                 }
+                if (bounce >= P.rr_start) {
+                    const double p = fmax(fmin(fmax(fmax(beta.x, beta.y), beta.z), 0.95), 0.05);
+                    if (pcg_f64(rng) > p) break;
+                    beta = beta / p;
+                }
+                const Hit hit = hit_of(S, ray, best);
+                const MaterialF64& mat = S.mats[hit.mat];
+                if (mat.kind == TPT_MAT_DIFFUSE_LIGHT) {
+                    L = L + clamp_lum(had(beta, ld(mat.c)), 50.0);
+                    break;
+                }
+                if (mat.kind != TPT_MAT_METAL && mat.kind != TPT_MAT_DIELECTRIC) {
+                    const V nrm = dot(hit.n, ray.d) < 0.0 ? hit.n : -hit.n, wo = norm(-ray.d);
+                    // nee_environment (:148-172), then nee_area_light (:178-213)
+#pragma unroll 1
+                    for (int k = has_env ? 0 : 1; k < 2; ++k) {
+                        V wi, li;
+                        double pl, tmax = kTMax;
+                        if (k == 0) {
+                            const bool by_cdf = env_sample_dir(S, rng, wi);
+                            pl = 1.0 / (4.0 * kPi);
+                            li = env_at(S, wi, by_cdf, pl);
+                        } else {
+                            V lp, ln;
+                            if (!sample_light(S, rng, ray.time, hit.p, lp, ln, li, pl)) continue;
+                            const V tl = lp - hit.p;
+                            const double dist = sqrt(dot(tl, tl));
+                            if (!(dist > 1e-6)) continue;
+                            wi = tl / dist;
+                            tmax = fmax(dist - kEps, kEps);
+                        }
+                        const double cs = fmax(dot(nrm, wi), 0.0);
+                        if (!(cs > 0.0) || (k == 0 && !(pl > 0.0))) continue;
+                        ++n_shadow;
+                        V f;
+                        double pb;
+                        mat_eval(mat, wo, wi, nrm, f, pb);
+                        const V contrib = had(had(beta, f), li) * (cs * mis(pl, pb) / pl);
+                        if (contrib.x == 0.0 && contrib.y == 0.0 && contrib.z == 0.0) continue;
+                        if (!spheres_hit(S, Ray{hit.p + kEps * wi, wi, ray.time}, tmax, true, best)) L = L + contrib;
+                    }
+                }
+                Bsdf s;
+                if (!mat_sample(mat, ray, hit, rng, s)) break;
+                last_pdf = s.pdf;
+                last_nd = !s.delta;
+                beta = had(beta, s.w);
+                ray = s.ray;
             }
-            Bsdf unused;
-            mat_sample(mat, ray, hit, rng, unused);  // its draws
         } while (!add_sample(P, sums, L));
         store_pixel(P, x, row, sums, acc, acc_w, acc_sq);
         n_samples = (unsigned long long)sums.n;
@@ -1164,14 +1187,17 @@ __global__ void __launch_bounds__(128, 3) k_first_hits(const __grid_constant__ P
 cudaError_t launch_plain(const PlainScene& S, const PlainParams& P, double* acc, double* acc_w, double* acc_sq,
                          unsigned long long* counters, int* flags, int sm_count, cudaStream_t stream) {
     const plain::Tiles tiles = plain::tiles_of(P);
-    // One bounce among spheres under the sky, or nothing to hit at all.  With
-    // triangles or an env map k_paths is faster (512x512 x 8 spp at one bounce, ms,
-    // in k_paths / here: sphere scene 0.60 / 0.87, 5,120 triangles 1.55 / 8.1, 24
-    // spheres with a map 0.42 / 0.67, without 0.26 / 0.16).
-    if (P.max_bounces <= 0 || S.top_root == TPT_REF_NONE ||
-        (P.max_bounces == 1 && S.n_tris == 0 && S.env_kind != TPT_ENV_MAP)) {
+    // Spheres alone, few enough for the reference's loop over them, or nothing to
+    // hit: a lane per pixel on its own.  Over 284 random calls of that kind (films
+    // to 1280x720, 1 to 600 spheres, with and without maps and lights) it is 1.29
+    // times as fast as k_paths; past some hundred spheres small films lose (200
+    // spheres 16x16 x 17 spp 1.9 ms in k_paths, 2.5 here), large ones gain (1280x720 x
+    // 2 spp 53 and 17), and 600 lose.  A single triangle brings the meshes' trees in,
+    // where lanes on their own fall behind (512x512 x 8 spp at one bounce, ms, in k_paths
+    // / lane by lane: 2 triangles 0.60 / 0.87, 5,120 triangles 1.55 / 8.1).
+    if (P.max_bounces <= 0 || (S.n_tris == 0 && S.n_spheres <= 256)) {
         const unsigned grid = (tiles.n_ids + 127u) / 128u;
-        plain::k_first_hits<<<grid, 128, 0, stream>>>(S, P, acc, acc_w, acc_sq, counters, flags);
+        plain::k_pixels<<<grid, 128, 0, stream>>>(S, P, acc, acc_w, acc_sq, counters, flags);
         return cudaGetLastError();
     }
     // Short walks: one block of 256 per SM, whose warps share the most fetched
