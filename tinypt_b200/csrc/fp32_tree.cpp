@@ -1,8 +1,9 @@
-// Mesh trees of the FP32 forms (wavefront, adjoint, batch).
+// Mesh trees that rays walk in all forms (wavefront, adjoint, batch, plain f64).
 //
-// The plain f64 form walks the reference's tree (src/bvh.rs:51-242: splits
-// on the axis of largest centroid extent only, 8 bins, every leaf of at most
-// 4 triangles), because its results must match the reference's bit for bit.
+// The reference's tree (src/bvh.rs:51-242) splits on the axis of largest
+// centroid extent only, over 8 bins, into leaves of at most 4 triangles; the plain
+// f64 form, whose results must match the reference's bit for bit, keeps it for
+// its leaf boxes and for hits that depend on its order, and walks this one.
 // The FP32 forms match the reference in distribution only, so they may walk
 // any tree over the same triangles; the closest hit does not depend on the
 // tree.  This one is a binned surface-area-heuristic tree over all three
